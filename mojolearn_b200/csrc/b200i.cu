@@ -18,6 +18,7 @@
 #include "gemm_tile.cuh"
 #include "gemm_skinny.cuh"
 #include "gemm_packed.cuh"
+#include "gemm_tall.cuh"
 #include "gemm_skinny_reg.cuh"
 #include "lowbit.cuh"
 
@@ -90,7 +91,7 @@ int64_t check_wait_status(char *err, int64_t err_cap, const char *who) {
 }
 
 // ---- plans -----------------------------------------------------------------------------
-enum { PLAN_AUTO = -1, PLAN_FLAT = 0, PLAN_T128 = 1, PLAN_T64 = 2, PLAN_DECODE = 3, PLAN_T32 = 4, PLAN_T128X64 = 5, PLAN_SKINNY = 6, PLAN_PACKED = 7 };
+enum { PLAN_AUTO = -1, PLAN_FLAT = 0, PLAN_T128 = 1, PLAN_T64 = 2, PLAN_DECODE = 3, PLAN_T32 = 4, PLAN_T128X64 = 5, PLAN_SKINNY = 6, PLAN_PACKED = 7, PLAN_TALL = 8 };
 
 // Up to this many rows the weight-streaming decode plan wins; above, the skinny plan. Low-bit weights
 // switch earlier: at three and four rows the decode kernel's serial chains cost more than the register
@@ -244,6 +245,15 @@ size_t packed_need(long long m, long long n, long long k, int groups) {
     return round256(groups > 1 ? (size_t)groups * m * n * 4 : 0) + pk_workspace_bytes(m, n, k);
 }
 
+// A^T B of few cells over many rows: every leaf of every 32 x 32 tile as a warp of its own (gemm_tall.cuh).
+constexpr long long TALL_MIN_LEAVES = 16;
+inline bool tall_fits(long long m, long long n, long long k, int op, int wkind) {
+    return op == OP_TN && wkind == W_F32 && m <= TALL_MAX_EXTENT && n <= TALL_MAX_EXTENT && leaf_count(k) >= 2;
+}
+inline bool tall_candidate(long long m, long long n, long long k) {
+    return m <= TALL_MAX_EXTENT && n <= TALL_MAX_EXTENT && leaf_count(k) >= TALL_MIN_LEAVES;
+}
+
 // The packed plan's leaf split: with at least two CTAs per slot of the device the tiles alone keep every SM busy
 // (a CTA left alone on an SM in the last wave runs at nearly twice the speed, so a partial wave costs little)
 // and a split would only add group nodes; below that, the tile plan's split stands.
@@ -391,6 +401,9 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         if (dec && m <= prefer_m && !(skinny && epilogue_pairs(g.epi))) plan = Plan{PLAN_DECODE, g.leaves, 1}; // (a gated store needs the skinny plan)
         else if (skinny) plan = choose_skinny(m, n, k, sm_count(dev), wkind != W_F32);
         else if (dec) plan = Plan{PLAN_DECODE, g.leaves, 1};
+        if (tall_fits(m, n, k, op, wkind) && tall_candidate(m, n, k) && !leave_nodes && !epilogue_pairs(g.epi) && ws && aligned(ws, 4) &&
+            (size_t)ws_bytes >= tall_workspace_bytes(m, n, k))
+            plan = Plan{PLAN_TALL, 1, g.leaves};
     } else {
         plan.kind = plan_kind;
         int s = group_leaves > 0 ? (int)group_leaves : g.leaves;
@@ -401,7 +414,12 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         plan.group_leaves = s;
         plan.groups = (g.leaves + s - 1) / s;
         if (plan.groups > 1 && (s & (s - 1))) return fail(err, err_cap, "identical gemm: a leaf group must be a power of two");
-        if (plan.groups > MAX_GROUPS) return fail(err, err_cap, "identical gemm: more than %d leaf groups", MAX_GROUPS);
+        if (plan.kind == PLAN_TALL) {
+            if (!tall_fits(m, n, k, op, wkind))
+                return fail(err, err_cap, "identical gemm: the tall plan needs op TN, float32 operands, m and n up to %d and at least two leaves", TALL_MAX_EXTENT);
+            plan.group_leaves = 1;
+            plan.groups = g.leaves;
+        } else if (plan.groups > MAX_GROUPS) return fail(err, err_cap, "identical gemm: more than %d leaf groups", MAX_GROUPS);
         if (plan.kind == PLAN_FLAT || plan.kind == PLAN_DECODE) { plan.groups = 1; plan.group_leaves = g.leaves; }
     }
     g.group_leaves = plan.group_leaves;
@@ -438,6 +456,10 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         if (!decode_plan_fits(m, n, k, op, wkind) || !aligned(b, 16) || !aligned(a, 16))
             return fail(err, err_cap, "identical gemm: the decode plan needs op NT, m <= %d, k a multiple of 16 and 16-byte aligned weights", DECODE_MAX_M);
         g_launches += launch_decode_plan(g, sm_count(dev), st);
+    } else if (plan.kind == PLAN_TALL) {
+        launch_tall(g, st); // its own fold, the store epilogue included
+        g_launches += 2;
+        plan.groups = 1;
     } else if (plan.kind == PLAN_T128) {
         launch_tile<128, 128, 2, 2, 2>(g, plan.groups, st);
         g_launches++;
@@ -473,7 +495,7 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         const long long cells = (long long)m * n;
         launch_fold_groups(g.ws, c, cells, plan.groups, st, g.epi, g.n);
         g_launches++;
-    } else if (epilogue_on(g.epi) && plan.kind != PLAN_SKINNY && plan.kind != PLAN_DECODE) {
+    } else if (epilogue_on(g.epi) && plan.kind != PLAN_SKINNY && plan.kind != PLAN_DECODE && plan.kind != PLAN_TALL) {
         // the tiled, packed and flat plans store plain product words; their epilogue is a pass of its own
         const long long cells = (long long)m * n;
         epilogue_rows_kernel<<<grid_for(cells, 256, sm_count(dev)), 256, 0, st>>>(c, cells, (int)n, g.epi);
@@ -555,6 +577,7 @@ int64_t b200i_workspace_bytes(int64_t m, int64_t n, int64_t k) {
     if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); dev = -1; }
     Plan p = choose_plan(m, n, k, sm_count(dev));
     int groups = p.groups;
+    if (tall_candidate(m, n, k) && (int)leaf_count(k) > groups) groups = (int)leaf_count(k);
     if (packed_candidate(p.kind, m, n, k))
         return (int64_t)packed_need(m, n, k, packed_split(p, m, n, k, sm_count(dev)).groups);
     if (skinny_plan_fits(m, n, k, OP_NT)) { // the plan an NT product with aligned operands takes instead
@@ -599,6 +622,7 @@ int64_t b200i_plan_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t plan
     if (s > leaves) s = leaves;
     const int64_t groups = (plan == PLAN_FLAT || plan == PLAN_DECODE) ? 1 : (leaves + s - 1) / s;
     if (plan == PLAN_PACKED) return (int64_t)packed_need(m, n, k, (int)groups);
+    if (plan == PLAN_TALL) return (int64_t)tall_workspace_bytes(m, n, k);
     return groups > 1 ? groups * m * n * 4 : 0;
 }
 

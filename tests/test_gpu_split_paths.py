@@ -1,0 +1,32 @@
+"""GPU parity of the kernels that split a product by leaves, warps or SM pairs, at the sizes where a split can go wrong:
+tile and strip edges, ragged last leaves and windows, failed admission, the largest and smallest of each range. The bar
+is the CPU oracle's words."""
+import numpy as np
+import pytest
+
+import oracle
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from mojolearn_b200 import _native, linalg, torch_ops  # noqa: E402
+
+
+def _same(got, want):
+    return got.cpu().numpy().tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("m,n,k", [(32, 32, 20000), (27, 27, 3001), (1, 5, 2049), (128, 128, 2100), (33, 97, 140000), (4, 64, 257), (36, 36, 131088)])
+def test_tall_products(m, n, k):
+    """One warp per leaf and tile, both copy widths, leaves of 128 and longer ones, a ragged last leaf."""
+    rng = np.random.default_rng(m + n + k)
+    a, b = rng.standard_normal((k, m)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    a[k // 2, 0], b[k - 1, n - 1], a[0, m - 1] = 1e-41, 3e-39, np.inf  # leaves that fail admission
+    want = oracle.nan_canon(oracle.gemm_rows(a, b, oracle.OP_TN))
+    da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    assert _same(torch_ops.product(da, db, op=linalg.OP_TN, plan=torch_ops.PLAN_TALL), want)
+    assert _same(torch_ops.matmul(da, db, transpose_a=True), want)
+    if m % 4 == 0 and n % 4 == 0:  # rows of whole quads that do not start on 16 bytes
+        pad = torch.empty(k * m + 1, device="cuda")
+        pad[1:] = da.reshape(-1)
+        assert _same(torch_ops.product(pad[1:].view(k, m), db, op=linalg.OP_TN, plan=torch_ops.PLAN_TALL), want)
