@@ -709,7 +709,7 @@ int64_t b200i_quantize_int8(int64_t device, void *stream, int8_t *codes, int32_t
     if (!codes || !exponents || !x) return fail(err, err_cap, "quantize_int8: null storage");
     int dev;
     if (select_device(device, err, err_cap, &dev)) return 1;
-    quantize_int8_kernel<<<grid_for(rows * 32, 256, sm_count(dev)), 256, 0, static_cast<cudaStream_t>(stream)>>>(reinterpret_cast<signed char *>(codes), exponents, x, rows, cols);
+    launch_quantize_int8(reinterpret_cast<signed char *>(codes), exponents, x, rows, cols, sm_count(dev), static_cast<cudaStream_t>(stream));
     g_launches++;
     CUDA_TRY(cudaGetLastError());
     return 0;

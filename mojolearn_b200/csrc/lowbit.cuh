@@ -66,6 +66,105 @@ __global__ void quantize_int8_kernel(signed char *__restrict__ q, int *__restric
     }
 }
 
+// One value's code in three instructions: the product by the row's power of two (input and result flushed: a result that
+// the flush could touch rounds to code 0 either way), a conversion that rounds half to even, saturates and takes a NaN to
+// 0, and the lower clamp: quantize_int8_value's answer for every input.
+__device__ __forceinline__ unsigned quantize_int8_byte(float x, float scale) {
+    float s;
+    int q;
+    asm("mul.rn.ftz.f32 %0, %1, %2;" : "=f"(s) : "f"(x), "f"(scale));
+    asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(q) : "f"(s));
+    return (unsigned)max(q, -127) & 0xFFu;
+}
+__device__ __forceinline__ unsigned quantize_int8_quad(float4 v, float scale) {
+    return quantize_int8_byte(v.x, scale) | quantize_int8_byte(v.y, scale) << 8 | quantize_int8_byte(v.z, scale) << 16 | quantize_int8_byte(v.w, scale) << 24;
+}
+// fmaxf passes over a NaN, as the scalar walk does; a subnormal maximum is flushed by int8_row_exponent
+__device__ __forceinline__ float absmax4(float4 v, float best) {
+    return fmaxf(fmaxf(fmaxf(best, fabsf(v.x)), fmaxf(fabsf(v.y), fabsf(v.z))), fabsf(v.w));
+}
+
+// The same for rows that are whole float4s: WARPS warps share a row and keep it in registers between the maximum and the
+// rounding, so it is read once, 16 bytes a lane, and its codes leave 4 bytes a lane. Bound: HBM, 5 bytes per element
+// ([4096, 4096]: 84 MB). One row per 1024 * WARPS columns at most; a block of 256 threads holds 8 / WARPS rows.
+constexpr int QUANT_VEC = 8; // float4s a lane holds
+template <int WARPS>
+__global__ void __launch_bounds__(256) quantize_int8_rows_kernel(signed char *__restrict__ q, int *__restrict__ e, const float *__restrict__ x,
+                                                                 long long rows, int cols) {
+    __shared__ float part[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long r = (long long)blockIdx.x * (8 / WARPS) + warp / WARPS;
+    const int first = (warp % WARPS) * 32 + lane, quads = cols >> 2;
+    const bool live = r < rows;
+    const float4 *row = reinterpret_cast<const float4 *>(x + (live ? r : 0) * cols);
+    float4 v[QUANT_VEC];
+    float best = 0.f;
+#pragma unroll
+    for (int i = 0; i < QUANT_VEC; i++) {
+        const int c = first + i * 32 * WARPS;
+        v[i] = (live && c < quads) ? __ldg(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < QUANT_VEC; i++) best = absmax4(v[i], best);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) best = fmaxf(best, __shfl_xor_sync(0xFFFFFFFFu, best, off));
+    if (WARPS > 1) {
+        if (lane == 0) part[warp] = best;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) best = fmaxf(best, part[warp / WARPS * WARPS + w]);
+    }
+    if (!live) return;
+    const int ex = int8_row_exponent(best);
+    if (first == 0) e[r] = ex;
+    const float scale = pow2_f32(-ex);
+    unsigned *out = reinterpret_cast<unsigned *>(q + r * cols);
+#pragma unroll
+    for (int i = 0; i < QUANT_VEC; i++) {
+        const int c = first + i * 32 * WARPS;
+        if (c < quads) out[c] = quantize_int8_quad(v[i], scale);
+    }
+}
+
+// Rows too wide for that: a block of 512 threads per row, which is read twice (the second time from L2).
+__global__ void __launch_bounds__(512) quantize_int8_wide_kernel(signed char *__restrict__ q, int *__restrict__ e, const float *__restrict__ x, long long quads) {
+    __shared__ float part[16];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float4 *row = reinterpret_cast<const float4 *>(x) + (long long)blockIdx.x * quads;
+    unsigned *out = reinterpret_cast<unsigned *>(q) + (long long)blockIdx.x * quads;
+    float best = 0.f;
+#pragma unroll 4
+    for (long long c = threadIdx.x; c < quads; c += 512) best = absmax4(__ldg(row + c), best);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) best = fmaxf(best, __shfl_xor_sync(0xFFFFFFFFu, best, off));
+    if (lane == 0) part[warp] = best;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 16; w++) best = fmaxf(best, part[w]);
+    const int ex = int8_row_exponent(best);
+    if (threadIdx.x == 0) e[blockIdx.x] = ex;
+    const float scale = pow2_f32(-ex);
+#pragma unroll 4
+    for (long long c = threadIdx.x; c < quads; c += 512) out[c] = quantize_int8_quad(__ldg(row + c), scale);
+}
+
+// The row kernels where rows are whole aligned float4s; the walk over scalars elsewhere.
+inline void launch_quantize_int8(signed char *q, int *e, const float *x, long long rows, long long cols, int sms, cudaStream_t st) {
+    const bool quads = cols % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & 3) == 0;
+    const long long span = 32 * 4 * QUANT_VEC; // columns one warp holds
+    if (quads && rows <= 0x7FFFFFFFll) {
+        if (cols <= span) quantize_int8_rows_kernel<1><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(q, e, x, rows, (int)cols);
+        else if (cols <= 2 * span) quantize_int8_rows_kernel<2><<<(unsigned)((rows + 3) / 4), 256, 0, st>>>(q, e, x, rows, (int)cols);
+        else if (cols <= 4 * span) quantize_int8_rows_kernel<4><<<(unsigned)((rows + 1) / 2), 256, 0, st>>>(q, e, x, rows, (int)cols);
+        else if (cols <= 8 * span) quantize_int8_rows_kernel<8><<<(unsigned)rows, 256, 0, st>>>(q, e, x, rows, (int)cols);
+        else quantize_int8_wide_kernel<<<(unsigned)rows, 512, 0, st>>>(q, e, x, cols / 4);
+        return;
+    }
+    long long blocks = (rows * 32 + 255) / 256, cap = (long long)sms * 16;
+    if (blocks > cap) blocks = cap;
+    quantize_int8_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks), 256, 0, st>>>(q, e, x, rows, cols);
+}
+
 __global__ void dequantize_int8_kernel(float *__restrict__ y, const signed char *__restrict__ q,
                                        const int *__restrict__ e, long long rows, long long cols) {
     const long long stride = (long long)gridDim.x * blockDim.x;

@@ -30,3 +30,14 @@ def test_tall_products(m, n, k):
         pad = torch.empty(k * m + 1, device="cuda")
         pad[1:] = da.reshape(-1)
         assert _same(torch_ops.product(pad[1:].view(k, m), db, op=linalg.OP_TN, plan=torch_ops.PLAN_TALL), want)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 4), (9, 1024), (8, 1028), (5, 2052), (3, 4096), (2, 8192), (3, 8196), (7, 7), (4, 1001)])
+def test_quantised_rows(rows, cols):
+    rng = np.random.default_rng(cols)
+    x = (rng.standard_normal((rows, cols)) * np.exp2(rng.integers(-140, 120, (rows, 1)))).astype(np.float32)
+    x[0, :3] = [np.nan, 1e-41, -np.inf][:3]
+    x[rows - 1] = 0.0
+    q, e = torch_ops.quantize_int8(torch.from_numpy(x).cuda())
+    qo, eo = oracle.quantize_int8(x)
+    assert _same(q, qo) and _same(e, eo)
