@@ -1,5 +1,6 @@
 // The C ABI of libb200i.so: argument checks, plan selection, launches.
 // Declarations and the reference interfaces they replace are in include/b200i.h.
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -288,12 +289,6 @@ Plan packed_split(const Plan &tile_plan, long long m, long long n, long long k, 
     return p;
 }
 
-template <int WK>
-void launch_pack(const PackArgs &a, cudaStream_t st) {
-    dim3 grid((unsigned)a.leaves, (unsigned)((a.extent + PK_TILE - 1) / PK_TILE));
-    pack_operand_kernel<WK><<<grid, 256, 0, st>>>(a);
-}
-
 // Packs both operands into `scratch` (panels, then flags) and runs the packed kernel.
 void packed_configure() {
     static std::atomic<bool> configured[64];
@@ -304,11 +299,22 @@ void packed_configure() {
         configured[dev] = true;
     }
 }
-void launch_pack_b(const PackArgs &b, int wkind, cudaStream_t st) {
-    if (wkind == W_F32) launch_pack<W_F32>(b, st);
-    else if (wkind == W_BF16) launch_pack<W_BF16>(b, st);
-    else if (wkind == W_INT8_EXP) launch_pack<W_INT8_EXP>(b, st);
-    else launch_pack<W_INT8_SCALE>(b, st);
+// The packing passes of two operands as one launch (extent 0: no left operand).
+void launch_pack(const PackArgs &a, const PackArgs &b, int wkind, cudaStream_t st) {
+    const int ta = (a.extent + PK_TILE - 1) / PK_TILE, tb = (b.extent + PK_TILE - 1) / PK_TILE;
+    for (int y0 = 0; y0 < ta + tb; y0 += 65535) { // grid.y holds 65535 tiles (more than 8 million rows need a second launch)
+        const dim3 grid((unsigned)(a.leaves * ((a.wpl + 1) / 2)), (unsigned)std::min(ta + tb - y0, 65535));
+        if (wkind == W_F32) pack_operands_kernel<W_F32><<<grid, 256, 0, st>>>(a, b, ta, y0);
+        else if (wkind == W_BF16) pack_operands_kernel<W_BF16><<<grid, 256, 0, st>>>(a, b, ta, y0);
+        else if (wkind == W_INT8_EXP) pack_operands_kernel<W_INT8_EXP><<<grid, 256, 0, st>>>(a, b, ta, y0);
+        else pack_operands_kernel<W_INT8_SCALE><<<grid, 256, 0, st>>>(a, b, ta, y0);
+    }
+}
+
+void launch_pack_one(const PackArgs &x, int wkind, cudaStream_t st) {
+    PackArgs none = x;
+    none.extent = 0;
+    launch_pack(none, x, wkind, st);
 }
 
 int launch_packed(const GemmArgs &g, int groups, unsigned char *scratch, cudaStream_t st) {
@@ -318,18 +324,20 @@ int launch_packed(const GemmArgs &g, int groups, unsigned char *scratch, cudaStr
     float *pb = pa + pk_panel_floats(g.m, g.k);
     unsigned char *fa = reinterpret_cast<unsigned char *>(pb + pk_panel_floats(g.n, g.k));
     unsigned char *fb = fa + pk_flag_bytes(g.m, g.k);
-    const bool k8 = (g.k % 8 == 0) && (g.leaves == 1 || g.leaf % 8 == 0);
-    PackArgs a{pa, fa, g.a, nullptr, g.m, g.k, g.leaf, g.leaves, wpl, g.op != OP_TN, g.op != OP_TN && k8 && aligned(g.a, 16)};
-    launch_pack<W_F32>(a, st);
-    PackArgs b{pb, fb, g.b, g.bscale, g.n, g.k, g.leaf, g.leaves, wpl, g.op == OP_NT, g.op == OP_NT && k8 && aligned(g.b, 16)};
-    launch_pack_b(b, g.wkind, st);
+    // quads: k-contiguous rows need k and the leaves in whole quads, the other layout whole quads of rows
+    const bool k4 = (g.k % 4 == 0) && (g.leaves == 1 || g.leaf % 4 == 0);
+    const size_t balign = g.wkind == W_F32 ? 16 : (g.wkind == W_BF16 ? 8 : 4);
+    const bool a_kc = g.op != OP_TN, b_kc = g.op == OP_NT;
+    PackArgs a{pa, fa, g.a, nullptr, g.m, g.k, g.leaf, g.leaves, wpl, a_kc, (a_kc ? k4 : g.m % 4 == 0) && aligned(g.a, 16)};
+    PackArgs b{pb, fb, g.b, g.bscale, g.n, g.k, g.leaf, g.leaves, wpl, b_kc, (b_kc ? k4 : g.n % 4 == 0) && aligned(g.b, balign)};
+    launch_pack(a, b, g.wkind, st);
     PackedGemmArgs p{pa, pb, fa, fb, g.c, g.ws, g.m, g.n, g.k, g.leaf, g.leaves, wpl, g.group_leaves, groups,
                      (g.n + PK_TILE - 1) / PK_TILE, g.vec_c};
     dim3 grid((unsigned)(((g.m + PK_TILE - 1) / PK_TILE) * p.tiles_n), (unsigned)groups);
     const int tslot = timing_begin(st);
     gemm_packed_kernel<<<grid, PK_THREADS, PK_SMEM_BYTES, st>>>(p);
     timing_end(tslot, st);
-    return 3;
+    return 2;
 }
 
 template <int BM, int BN, int RM, int RN, int MINB>
@@ -1538,7 +1546,7 @@ static int64_t host_gemm_pipelined(int dev, HostPool &pool, float *c, const floa
     float *pb = pa + pk_panel_floats(m, k);
     unsigned char *fa = reinterpret_cast<unsigned char *>(pb + pk_panel_floats(n, k));
     unsigned char *fb = fa + pk_flag_bytes(m, k);
-    const bool k8 = (k % 8 == 0) && (leaves == 1 || leaf % 8 == 0);
+    const bool k4 = (k % 4 == 0) && (leaves == 1 || leaf % 4 == 0); // the device copies are aligned: whole quads where the extents are
     const int tiles_m = (int)((m + PK_TILE - 1) / PK_TILE), tiles_n = (int)((n + PK_TILE - 1) / PK_TILE);
     // everything queued below waits for whatever the compute stream still holds from an earlier call
     CUDA_TRY(cudaEventRecord(pool.ev[0], pool.stream));
@@ -1554,11 +1562,11 @@ static int64_t host_gemm_pipelined(int dev, HostPool &pool, float *c, const floa
     CUDA_TRY(cudaEventRecord(pool.ev[0], pool.s_in));
     CUDA_TRY(cudaStreamWaitEvent(pool.stream, pool.ev[0], 0));
     if (by_rows) {
-        PackArgs pbargs{pb, fb, db, ds, (int)n, (int)k, leaf, leaves, wpl, op == OP_NT, op == OP_NT && k8};
-        launch_pack_b(pbargs, wkind, pool.stream);
+        PackArgs pbargs{pb, fb, db, ds, (int)n, (int)k, leaf, leaves, wpl, op == OP_NT, op == OP_NT ? k4 : n % 4 == 0};
+        launch_pack_one(pbargs, wkind, pool.stream);
     } else {
-        PackArgs paargs{pa, fa, da, nullptr, (int)m, (int)k, leaf, leaves, wpl, 1, k8};
-        launch_pack<W_F32>(paargs, pool.stream);
+        PackArgs paargs{pa, fa, da, nullptr, (int)m, (int)k, leaf, leaves, wpl, 1, k4};
+        launch_pack_one(paargs, W_F32, pool.stream);
     }
     g_launches++;
     for (int i = 0; i < nch; i++) {
@@ -1571,8 +1579,8 @@ static int64_t host_gemm_pipelined(int dev, HostPool &pool, float *c, const floa
             CUDA_TRY(cudaStreamWaitEvent(pool.stream, pool.ev[1 + 2 * i], 0));
             float *pai = pa + (size_t)tile0 * k * PK_TILE;
             unsigned char *fai = fa + (size_t)tile0 * leaves * wpl;
-            PackArgs paargs{pai, fai, dai, nullptr, (int)cnt, (int)k, leaf, leaves, wpl, 1, k8};
-            launch_pack<W_F32>(paargs, pool.stream);
+            PackArgs paargs{pai, fai, dai, nullptr, (int)cnt, (int)k, leaf, leaves, wpl, 1, k4};
+            launch_pack_one(paargs, W_F32, pool.stream);
             PackedGemmArgs p{pai, pb, fai, fb, dci, nullptr, (int)cnt, (int)n, (int)k, leaf, leaves, wpl, leaves, 1, tiles_n, (n % 4 == 0) ? 1 : 0};
             dim3 grid((unsigned)(((cnt + PK_TILE - 1) / PK_TILE) * tiles_n), 1u);
             gemm_packed_kernel<<<grid, PK_THREADS, PK_SMEM_BYTES, pool.stream>>>(p);
@@ -1592,8 +1600,8 @@ static int64_t host_gemm_pipelined(int dev, HostPool &pool, float *c, const floa
             float *pbi = pb + (size_t)tile0 * k * PK_TILE;
             unsigned char *fbi = fb + (size_t)tile0 * leaves * wpl;
             PackArgs pbargs{pbi, fbi, dbi, sbytes ? static_cast<unsigned char *>(ds) + (size_t)x0 * 4 : nullptr, (int)cnt, (int)k, leaf, leaves,
-                            wpl, 1, k8};
-            launch_pack_b(pbargs, wkind, pool.stream);
+                            wpl, 1, k4};
+            launch_pack_one(pbargs, wkind, pool.stream);
             const int tiles_nc = (int)((cnt + PK_TILE - 1) / PK_TILE);
             PackedGemmArgs p{pa, pbi, fa, fbi, dci, nullptr, (int)m, (int)cnt, (int)k, leaf, leaves, wpl, leaves, 1, tiles_nc,
                              (cnt % 4 == 0 && (m * x0) % 4 == 0) ? 1 : 0};

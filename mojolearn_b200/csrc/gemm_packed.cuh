@@ -3,7 +3,7 @@
 //
 // Numerical plan: the contract's (see gemm_tile.cuh). Execution plan for B200:
 //
-//   1. pack_operand_kernel rewrites each operand once per product into tile-major
+//   1. pack_operands_kernel rewrites each operand once per product into tile-major
 //      panels P[tile][k][128]: 128 rows (or columns) of the operand side by side
 //      for every k, already materialised to float32 (bf16 widened, int8
 //      dequantised) and flushed, rows past the edge zero. It also writes one
@@ -54,7 +54,7 @@ struct PackArgs {
     const void *scale;
     int extent, k, leaf, leaves, wpl;
     int kcontig; // 1: x is [extent][k]; 0: x is [k][extent]
-    int vec;     // k-contiguous, every 8-step run of a thread starts on a 16-byte (float32) / element-size * 8 boundary
+    int vec;     // four consecutive elements may be read at once (every quad of a row starts on a 4-element boundary)
 };
 
 __device__ __forceinline__ float pk_element(const void *x, const void *scale, int wkind, size_t off, int row) {
@@ -64,65 +64,127 @@ __device__ __forceinline__ float pk_element(const void *x, const void *scale, in
     return dequant_int8_pow2((int)__ldg(static_cast<const signed char *>(x) + off), f);
 }
 
-// grid (leaves, tiles); 256 threads: thread (r = tid % 128, half = tid / 128) owns row r of the tile and 8 of a
-// window's 16 k-steps, so the panel is written in 512-byte runs
+// Both operands of a product in one launch: grid.x walks the (leaf, pair of windows) blocks, grid.y the tiles of A, then
+// those of B. A block of 256 threads moves 128 rows x 32 k-steps. k-contiguous operands are read 128 bytes of a row at a
+// time (eight lanes, four rows per warp instruction, four such reads in flight) and turned through shared memory, whose
+// 4-word groups are permuted by the lane's k group so that both the turned stores and the 16-byte reads are free of
+// conflicts; operands stored row by row of k are copied straight through registers. Every panel row leaves as 512
+// contiguous bytes. Bound: HBM, 8 bytes per float32 word. One block per leaf of 128 steps (the split before) left
+// 64 blocks on a 1000 x 1000 operand and a CTA barrier between its loads: 39 us there, 13 us at [128, 4096].
+constexpr int PACK_K = 2 * KS;
+
+// four consecutive elements starting at `off` as float32 words, exact
 template <int WK>
-__global__ void __launch_bounds__(256) pack_operand_kernel(const PackArgs a) {
-    const int t = blockIdx.x, tile = blockIdx.y;
-    const int r = threadIdx.x % PK_TILE, half = threadIdx.x / PK_TILE;
-    const int row = tile * PK_TILE + r;
-    const bool live = row < a.extent;
-    const int kb = t * a.leaf, leaf_len = min(a.leaf, a.k - kb);
-    float *panel = a.panel + (size_t)tile * (size_t)a.k * PK_TILE;
-    for (int w = 0, koff = 0; koff < leaf_len; w++, koff += KS) {
-        const int len = min(KS, leaf_len - koff);
-        unsigned key = 0xFFFFFFFFu;
-        float v[8];
-        if (a.vec && live && len == KS) { // this thread's 8 k-steps are contiguous in the operand: 32, 16 or 8 bytes
-            const size_t off = (size_t)row * a.k + kb + koff + half * 8;
-            if (WK == W_F32) {
-                const float4 lo = __ldg(reinterpret_cast<const float4 *>(static_cast<const float *>(a.x) + off));
-                const float4 hi = __ldg(reinterpret_cast<const float4 *>(static_cast<const float *>(a.x) + off) + 1);
-                v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
-#pragma unroll
-                for (int e = 0; e < 8; e++) v[e] = ftz_bits(v[e]);
-            } else if (WK == W_BF16) {
-                const uint4 w = __ldg(reinterpret_cast<const uint4 *>(static_cast<const unsigned short *>(a.x) + off));
-                const unsigned ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    v[2 * e] = ftz_bits(__uint_as_float(ws[e] << 16));
-                    v[2 * e + 1] = ftz_bits(__uint_as_float(ws[e] & 0xFFFF0000u));
-                }
-            } else {
-                const uint2 w = __ldg(reinterpret_cast<const uint2 *>(static_cast<const signed char *>(a.x) + off));
-                const float f = (WK == W_INT8_EXP) ? pow2_f32(__ldg(static_cast<const int *>(a.scale) + row))
-                                                   : __ldg(static_cast<const float *>(a.scale) + row);
-#pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const unsigned word = e < 4 ? w.x : w.y;
-                    v[e] = dequant_int8_pow2((int)(signed char)((word >> (8 * (e & 3))) & 0xFFu), f);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                const int kk = kb + koff + half * 8 + e;
-                v[e] = 0.f;
-                if (live && half * 8 + e < len)
-                    v[e] = pk_element(a.x, a.scale, WK, a.kcontig ? (size_t)row * a.k + kk : (size_t)kk * a.extent + row, row);
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            if (half * 8 + e < len) {
-                key = min(key, admit_key(v[e]));
-                panel[(size_t)(kb + koff + half * 8 + e) * PK_TILE + r] = v[e];
-            }
-        }
-        const int ok = __syncthreads_and(key >= ADMIT_MIN);
-        if (threadIdx.x == 0) a.flags[((size_t)tile * a.leaves + t) * a.wpl + w] = (unsigned char)(ok ? 1 : 0);
+__device__ __forceinline__ float4 pk_quad(const void *x, const void *scale, size_t off, int row) {
+    float4 v;
+    if (WK == W_F32) {
+        v = __ldg(reinterpret_cast<const float4 *>(static_cast<const float *>(x) + off));
+    } else if (WK == W_BF16) {
+        const uint2 w = __ldg(reinterpret_cast<const uint2 *>(static_cast<const unsigned short *>(x) + off));
+        v = make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xFFFF0000u), __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xFFFF0000u));
+    } else {
+        const unsigned w = __ldg(reinterpret_cast<const unsigned *>(static_cast<const signed char *>(x) + off));
+        const float f = (WK == W_INT8_EXP) ? pow2_f32(__ldg(static_cast<const int *>(scale) + row)) : __ldg(static_cast<const float *>(scale) + row);
+        v = make_float4(dequant_int8_pow2((int)(signed char)(w & 0xFFu), f), dequant_int8_pow2((int)(signed char)((w >> 8) & 0xFFu), f),
+                        dequant_int8_pow2((int)(signed char)((w >> 16) & 0xFFu), f), dequant_int8_pow2((int)(signed char)(w >> 24), f));
     }
+    return make_float4(ftz_bits(v.x), ftz_bits(v.y), ftz_bits(v.z), ftz_bits(v.w));
+}
+
+template <int WK>
+__device__ __forceinline__ void pack_block(const PackArgs &a, int tile, float (*turn)[PK_TILE], int (*ok)[2]) {
+    const int cpl = (a.wpl + 1) / 2; // blocks per leaf
+    const int t = blockIdx.x / cpl, w0 = (blockIdx.x % cpl) * 2;
+    const int kb = t * a.leaf, leaf_len = min(a.leaf, a.k - kb), k0 = kb + w0 * KS;
+    const int len = min(PACK_K, leaf_len - w0 * KS); // k-steps of this block; <= 0 past the end of a short last leaf
+    if (len <= 0) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row0 = tile * PK_TILE;
+    float *panel = a.panel + (size_t)tile * (size_t)a.k * PK_TILE + (size_t)k0 * PK_TILE;
+    unsigned key[2] = {0xFFFFFFFFu, 0xFFFFFFFFu}; // of the words this thread moved, by window
+    if (a.kcontig) {
+        const int kq = lane & 7; // k-steps kq * 4 .. + 3
+        float4 v[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            const int r = p * 32 + warp * 4 + (lane >> 3), row = row0 + r;
+            v[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row < a.extent && kq * 4 < len) {
+                const size_t off = (size_t)row * a.k + k0 + kq * 4;
+                if (a.vec && kq * 4 + 3 < len) {
+                    v[p] = pk_quad<WK>(a.x, a.scale, off, row);
+                } else {
+                    v[p].x = pk_element(a.x, a.scale, WK, off, row);
+                    if (kq * 4 + 1 < len) v[p].y = pk_element(a.x, a.scale, WK, off + 1, row);
+                    if (kq * 4 + 2 < len) v[p].z = pk_element(a.x, a.scale, WK, off + 2, row);
+                    if (kq * 4 + 3 < len) v[p].w = pk_element(a.x, a.scale, WK, off + 3, row);
+                }
+            }
+        }
+        unsigned mine = 0xFFFFFFFFu;
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            const int r = (p * 32 + warp * 4 + (lane >> 3)) ^ (kq * 4);
+            mine = key4(v[p], mine);
+            turn[kq * 4 + 0][r] = v[p].x;
+            turn[kq * 4 + 1][r] = v[p].y;
+            turn[kq * 4 + 2][r] = v[p].z;
+            turn[kq * 4 + 3][r] = v[p].w;
+        }
+        key[0] = kq < 4 ? mine : 0xFFFFFFFFu;
+        key[1] = kq < 4 ? 0xFFFFFFFFu : mine;
+        __syncthreads();
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            const int kk = p * 8 + warp;
+            if (kk < len)
+                *reinterpret_cast<float4 *>(panel + (size_t)kk * PK_TILE + lane * 4) = *reinterpret_cast<const float4 *>(&turn[kk][(lane * 4) ^ ((kk >> 2) * 4)]);
+        }
+    } else {
+        float4 v[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            const int kk = p * 8 + warp, row = row0 + lane * 4;
+            v[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (kk < len && row < a.extent) {
+                const size_t off = (size_t)(k0 + kk) * a.extent + row;
+                if (a.vec && row + 3 < a.extent) {
+                    v[p] = pk_quad<WK>(a.x, a.scale, off, row);
+                } else {
+                    v[p].x = pk_element(a.x, a.scale, WK, off, row);
+                    if (row + 1 < a.extent) v[p].y = pk_element(a.x, a.scale, WK, off + 1, row + 1);
+                    if (row + 2 < a.extent) v[p].z = pk_element(a.x, a.scale, WK, off + 2, row + 2);
+                    if (row + 3 < a.extent) v[p].w = pk_element(a.x, a.scale, WK, off + 3, row + 3);
+                }
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            const int kk = p * 8 + warp;
+            key[p >> 1] = key4(v[p], key[p >> 1]);
+            if (kk < len) *reinterpret_cast<float4 *>(panel + (size_t)kk * PK_TILE + lane * 4) = v[p];
+        }
+    }
+#pragma unroll
+    for (int w = 0; w < 2; w++) {
+        const bool all = __all_sync(0xFFFFFFFFu, key[w] >= ADMIT_MIN);
+        if (lane == 0) ok[warp][w] = all ? 1 : 0;
+    }
+    __syncthreads();
+    if (tid < 2 && tid * KS < len) {
+        int all = 1;
+#pragma unroll
+        for (int w = 0; w < 8; w++) all &= ok[w][tid];
+        a.flags[((size_t)tile * a.leaves + t) * a.wpl + w0 + tid] = (unsigned char)all;
+    }
+}
+
+template <int WK>
+__global__ void __launch_bounds__(256) pack_operands_kernel(const PackArgs a, const PackArgs b, int tiles_a, int first_tile) {
+    __shared__ __align__(16) float turn[PACK_K][PK_TILE];
+    __shared__ int ok[8][2];
+    const int tile = (int)blockIdx.y + first_tile;
+    if (tile < tiles_a) pack_block<W_F32>(a, tile, turn, ok);
+    else pack_block<WK>(b, tile - tiles_a, turn, ok);
 }
 
 struct PackedGemmArgs {
