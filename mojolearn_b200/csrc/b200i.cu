@@ -506,7 +506,9 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
     } else if (epilogue_on(g.epi) && plan.kind != PLAN_SKINNY && plan.kind != PLAN_DECODE && plan.kind != PLAN_TALL) {
         // the tiled, packed and flat plans store plain product words; their epilogue is a pass of its own
         const long long cells = (long long)m * n;
-        epilogue_rows_kernel<<<grid_for(cells, 256, sm_count(dev)), 256, 0, st>>>(c, cells, (int)n, g.epi);
+        if (n % 4 == 0 && aligned(c, 16))
+            epilogue_rows4_kernel<<<dim3((unsigned)((n / 4 + 255) / 256), (unsigned)std::min<int64_t>(m, 65535)), 256, 0, st>>>(c, (int)m, (int)n, g.epi);
+        else epilogue_rows_kernel<<<grid_for(cells, 256, sm_count(dev)), 256, 0, st>>>(c, cells, (int)n, g.epi);
         g_launches++;
     }
     CUDA_TRY(cudaGetLastError());
@@ -971,7 +973,17 @@ int64_t b200i_qkv_rope_cache(int64_t device, void *stream, float *qr, float *kca
     const long long total = b * l * (n_heads + 2 * n_kv) * head_dim;
     const long long ldq = src_ld ? src_ld : n_heads * head_dim, ldkv = src_ld ? src_ld : n_kv * head_dim;
     if (ldq < n_heads * head_dim || ldkv < n_kv * head_dim) return fail(err, err_cap, "qkv_rope_cache: the row pitch is below the row width");
-    qkv_rope_cache_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(qr, kcache, vcache, q, k, v, ldq, ldkv, cosv, sinv, (int)b, (int)l,
+    const bool quads = (cosv ? (rope_dim == head_dim && head_dim % 8 == 0) : head_dim % 4 == 0) && ldq % 4 == 0 && ldkv % 4 == 0 && aligned(qr, 16) &&
+                       aligned(kcache, 16) && aligned(vcache, 16) && aligned(q, 16) && aligned(k, 16) && aligned(v, 16) &&
+                       (!cosv || (aligned(cosv, 16) && aligned(sinv, 16)));
+    if (quads) {
+        const int64_t per_head = cosv ? head_dim / 8 : head_dim / 4, units = (n_heads + n_kv) * per_head + n_kv * (head_dim / 4);
+        const QkvArgs g{qr, kcache, vcache, q, k, v, cosv, sinv, ldq, ldkv, b * l, (int)l, (int)n_heads, (int)n_kv, (int)head_dim, (int)cap, (int)pos0,
+                        cosv ? 1 : 0, position};
+        const int threads = units >= 256 ? 256 : 128;
+        qkv_rope_cache4_kernel<<<dim3((unsigned)((units + threads - 1) / threads), (unsigned)std::min<int64_t>(b * l, 65535)), threads, 0, st>>>(g);
+    } else
+        qkv_rope_cache_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(qr, kcache, vcache, q, k, v, ldq, ldkv, cosv, sinv, (int)b, (int)l,
                                                                            (int)n_heads, (int)n_kv, (int)head_dim, (int)cap, (int)pos0,
                                                                            position, cosv ? 1 : 0, (int)rope_dim);
     g_launches++;
@@ -1266,7 +1278,10 @@ int64_t b200i_act_mul(int64_t device, void *stream, float *out, const float *gat
     if (rows <= 0 || width <= 0 || (!interleaved && in_ld < width) || !out || !up || kind < ACT_SWIGLU || kind > ACT_GEGLU_TANH)
         return fail(err, err_cap, "act_mul: bad arguments");
     if (gated && !gate) return fail(err, err_cap, "act_mul: a gated MLP needs its gate projection");
-    act_mul_kernel<<<grid_for(rows * width, 256, sm_count(dev)), 256, 0, st>>>(out, gate, up, rows, width, in_ld, (int)kind, interleaved ? 2 : 1);
+    if (interleaved && width % 4 == 0 && in_ld % 4 == 0 && width <= 0x3FFFFFFF && aligned(out, 16) && aligned(gate, 16))
+        act_mul_pairs_kernel<<<dim3((unsigned)((width / 4 + 255) / 256), (unsigned)std::min<int64_t>(rows, 65535)), 256, 0, st>>>(out, gate, rows, (int)width,
+                                                                                                                            in_ld, (int)kind);
+    else act_mul_kernel<<<grid_for(rows * width, 256, sm_count(dev)), 256, 0, st>>>(out, gate, up, rows, width, in_ld, (int)kind, interleaved ? 2 : 1);
     g_launches++;
     CUDA_TRY(cudaGetLastError());
     return 0;

@@ -44,6 +44,39 @@ constexpr unsigned NORM_ADMIT_MIN = 0u;
 #else
 constexpr unsigned NORM_ADMIT_MIN = (64u << 24) - 2u;
 #endif
+// A serial chain over a row in shared memory, p-ascending: acc = step(element, acc). Every lane reads the same words; 32
+// elements are requested while the 32 before them are consumed, so the chain waits on its own 4-cycle steps and not on
+// shared memory once per 16 elements (2048 wide, 32 rows: 15 us with a plain unrolled loop).
+template <class Step>
+__device__ __forceinline__ float row_chain(const float *xs, int dm, Step step) {
+    float acc = 0.f;
+    const int whole = dm & ~63;
+    float4 a[8], b[8];
+    auto fill = [&](float4 (&v)[8], int j) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = *reinterpret_cast<const float4 *>(xs + j + 4 * u);
+    };
+    auto walk = [&](const float4 (&v)[8]) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            acc = step(v[u].x, acc);
+            acc = step(v[u].y, acc);
+            acc = step(v[u].z, acc);
+            acc = step(v[u].w, acc);
+        }
+    };
+    if (whole) fill(a, 0);
+#pragma unroll 1
+    for (int j = 0; j < whole; j += 64) {
+        fill(b, j + 32);
+        walk(a);
+        if (j + 64 < whole) fill(a, j + 64);
+        walk(b);
+    }
+    for (int j = whole; j < dm; j++) acc = step(xs[j], acc);
+    return acc;
+}
+
 // With `delta` the row normalised is the residual sum ftz(ftz(src) + ftz(delta)) (seam S22 / S23), which is
 // also written to `sum_out`: the residual add and the norm that always follows it, in one pass over the row.
 constexpr int NORM_WREG = 16; // 128-bit words of the weight row a lane can hold: rows up to 2048 wide
@@ -109,15 +142,8 @@ __global__ void __launch_bounds__(128) norm_rows_kernel(float *__restrict__ out,
     }
     for (int j = dm + lane; j < pitch; j += 32) xs[j] = 0.f;
     __syncwarp();
-    const int dm4 = dm & ~3;
     if (kind == NORM_LAYER) {
-        float acc = 0.f;
-#pragma unroll 4
-        for (int j = 0; j < dm4; j += 4) {
-            const float4 v = *reinterpret_cast<const float4 *>(xs + j);
-            acc = add_flushed(add_flushed(add_flushed(add_flushed(acc, v.x), v.y), v.z), v.w);
-        }
-        for (int j = dm4; j < dm; j++) acc = add_flushed(acc, xs[j]);
+        const float acc = row_chain(xs, dm, [](float v, float acc) { return add_flushed(acc, v); });
         const float mean = ftz_bits(p_divf(acc, (float)dm));
         __syncwarp();
         key = 0xFFFFFFFFu;
@@ -129,28 +155,8 @@ __global__ void __launch_bounds__(128) norm_rows_kernel(float *__restrict__ out,
         __syncwarp();
     }
     const bool bare = __all_sync(0xFFFFFFFFu, key >= NORM_ADMIT_MIN);
-    float acc = 0.f;
-    if (bare) {
-#pragma unroll 4
-        for (int j = 0; j < dm4; j += 4) {
-            const float4 v = *reinterpret_cast<const float4 *>(xs + j);
-            acc = step_bare(v.x, v.x, acc);
-            acc = step_bare(v.y, v.y, acc);
-            acc = step_bare(v.z, v.z, acc);
-            acc = step_bare(v.w, v.w, acc);
-        }
-        for (int j = dm4; j < dm; j++) acc = step_bare(xs[j], xs[j], acc);
-    } else {
-#pragma unroll 2
-        for (int j = 0; j < dm4; j += 4) {
-            const float4 v = *reinterpret_cast<const float4 *>(xs + j);
-            acc = step_flush(v.x, v.x, acc);
-            acc = step_flush(v.y, v.y, acc);
-            acc = step_flush(v.z, v.z, acc);
-            acc = step_flush(v.w, v.w, acc);
-        }
-        for (int j = dm4; j < dm; j++) acc = step_flush(xs[j], xs[j], acc);
-    }
+    const float acc = bare ? row_chain(xs, dm, [](float v, float acc) { return step_bare(v, v, acc); })
+                           : row_chain(xs, dm, [](float v, float acc) { return step_flush(v, v, acc); });
     const float var = ftz_bits(p_divf(acc, (float)dm));
     const float rstd = ftz_bits(p_rsqrtf(ftz_bits(__fadd_rn(var, eps))));
     auto finish = [&](float xv, float wv, float bv) {
@@ -395,6 +401,56 @@ __global__ void qkv_rope_cache_kernel(float *__restrict__ qr, float *__restrict_
         float *cache = c < wq + wk ? kcache : vcache;
         const int kv = (int)(col / hd);
         cache[(((long long)bb * nkv + kv) * cap + pos0 + li) * hd + j] = val;
+    }
+}
+
+// The same over whole float4s: a thread owns four columns of the first half of a rotated head and the four they pair
+// with (eight outputs from eight words read once), or four columns of a head that is only copied (every v head; all of
+// them without rotation). One block row per token, so no index is divided but the column. Needs whole heads rotated,
+// head_dim a multiple of 8 and 16-byte aligned rows. Bound: HBM, 8 bytes per element (4096 tokens of 3 x 2048 columns:
+// 211 us one element per thread with 64-bit index divisions, against 31 us for its 201 MB).
+struct QkvArgs {
+    float *qr, *kcache, *vcache;
+    const float *q, *k, *v, *cosv, *sinv;
+    long long ldq, ldkv, rows;
+    int l, nh, nkv, hd, cap, pos0, rope;
+    const int *pos_dev;
+};
+__global__ void __launch_bounds__(256) qkv_rope_cache4_kernel(const QkvArgs g) {
+    const int pos0 = g.pos_dev ? *g.pos_dev : g.pos0;
+    const int per_head = g.rope ? g.hd / 8 : g.hd / 4, per_v = g.hd / 4; // threads a q or k head takes; a v head
+    const int turned = (g.nh + g.nkv) * per_head;
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= turned + g.nkv * per_v) return;
+    const bool is_v = u >= turned;
+    const int head = is_v ? (u - turned) / per_v : u / per_head;
+    const int j = (is_v ? (u - turned) % per_v : u % per_head) * 4, half = g.hd / 2;
+    for (long long t = blockIdx.y; t < g.rows; t += gridDim.y) {
+        const int li = (int)(t % g.l), bb = (int)(t / g.l);
+        const bool is_q = !is_v && head < g.nh;
+        const int kv = is_v ? head : head - g.nh;
+        const float *src = is_v ? g.v + t * g.ldkv + kv * g.hd : (is_q ? g.q + t * g.ldq + head * g.hd : g.k + t * g.ldkv + kv * g.hd);
+        float *dst;
+        if (is_q) {
+            dst = g.qr + t * ((long long)g.nh * g.hd) + head * g.hd;
+        } else {
+            if (pos0 + li >= g.cap) continue; // the host refuses such a call; a replayed graph must not write past the cache either
+            dst = (is_v ? g.vcache : g.kcache) + (((long long)bb * g.nkv + kv) * g.cap + pos0 + li) * g.hd;
+        }
+        const float4 lo = __ldg(reinterpret_cast<const float4 *>(src + j));
+        if (is_v || !g.rope) {
+            *reinterpret_cast<float4 *>(dst + j) = lo;
+            continue;
+        }
+        const float4 hi = __ldg(reinterpret_cast<const float4 *>(src + half + j));
+        const float4 cs = __ldg(reinterpret_cast<const float4 *>(g.cosv + li * half + j)), sn = __ldg(reinterpret_cast<const float4 *>(g.sinv + li * half + j));
+        auto turn = [](float x, float partner, float c, float s) { // S9-S10: two products and a sum, each flushed
+            return ftz_bits(__fadd_rn(ftz_bits(__fmul_rn(ftz_bits(x), ftz_bits(c))), ftz_bits(__fmul_rn(partner, ftz_bits(s)))));
+        };
+        *reinterpret_cast<float4 *>(dst + j) = make_float4(turn(lo.x, -ftz_bits(hi.x), cs.x, sn.x), turn(lo.y, -ftz_bits(hi.y), cs.y, sn.y),
+                                                           turn(lo.z, -ftz_bits(hi.z), cs.z, sn.z), turn(lo.w, -ftz_bits(hi.w), cs.w, sn.w));
+        *reinterpret_cast<float4 *>(dst + half + j) = make_float4(turn(hi.x, ftz_bits(lo.x), cs.x, sn.x), turn(hi.y, ftz_bits(lo.y), cs.y, sn.y),
+                                                                  turn(hi.z, ftz_bits(lo.z), cs.z, sn.z), turn(hi.w, ftz_bits(lo.w), cs.w, sn.w));
     }
 }
 
@@ -1319,6 +1375,31 @@ __global__ void act_mul_kernel(float *__restrict__ out, const float *gate, const
         else if (kind == ACT_GELU_TANH || kind == ACT_GEGLU_TANH) a = ftz_bits(p_gelu_tanh(z));
         else a = ftz_bits(p_gelu_erf(z));
         out[o] = gated ? ftz_bits(__fmul_rn(a, ftz_bits(up[i]))) : a;
+    }
+}
+
+// The same for a gated activation over interleaved columns (gate, up, gate, up, ...), four outputs a thread from two
+// 16-byte reads, one block row per row so that no index is divided. width % 4 == 0, 16-byte aligned rows. Bound: HBM
+// and the exponential's own instructions about evenly (4096 x 8192: 403 MB = 62 us; 170 us one output per thread with a
+// 64-bit division and remainder each).
+__global__ void __launch_bounds__(256) act_mul_pairs_kernel(float *__restrict__ out, const float *__restrict__ gu, long long rows, int width, long long ld,
+                                                            int kind) {
+    const int o = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (o >= width) return;
+    for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
+        const float4 p0 = __ldg(reinterpret_cast<const float4 *>(gu + r * ld + 2 * o)), p1 = __ldg(reinterpret_cast<const float4 *>(gu + r * ld + 2 * o + 4));
+        const float gate[4] = {p0.x, p0.z, p1.x, p1.z}, up[4] = {p0.y, p0.w, p1.y, p1.w};
+        float y[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const float z = ftz_bits(gate[e]);
+            float a;
+            if (kind == ACT_SWIGLU) a = ftz_bits(p_siluf(z));
+            else if (kind == ACT_GEGLU_TANH) a = ftz_bits(p_gelu_tanh(z));
+            else a = ftz_bits(p_gelu_erf(z));
+            y[e] = ftz_bits(__fmul_rn(a, ftz_bits(up[e])));
+        }
+        *reinterpret_cast<float4 *>(out + r * width + o) = make_float4(y[0], y[1], y[2], y[3]);
     }
 }
 

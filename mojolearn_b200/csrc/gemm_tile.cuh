@@ -412,6 +412,22 @@ __global__ void epilogue_rows_kernel(float *__restrict__ c, long long cells, int
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += stride) epilogue_cell(c + i, epi, i % n);
 }
 
+// The same four cells a thread, one block row per output row (n % 4 == 0, 16-byte aligned): no index is divided
+// (4096 x 3072 with GELU: 67 us one cell per thread with a 64-bit remainder each, against 15 us for its bytes).
+__global__ void __launch_bounds__(256) epilogue_rows4_kernel(float *__restrict__ c, int m, int n, Epilogue epi) {
+    const int col = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (col >= n) return;
+    for (int row = blockIdx.y; row < m; row += gridDim.y) {
+        float4 *cell = reinterpret_cast<float4 *>(c + (size_t)row * n + col);
+        float4 v = *cell;
+        v.x = epilogue_apply(v.x, epi.bias, epi.act, col);
+        v.y = epilogue_apply(v.y, epi.bias, epi.act, col + 1);
+        v.z = epilogue_apply(v.z, epi.bias, epi.act, col + 2);
+        v.w = epilogue_apply(v.w, epi.bias, epi.act, col + 3);
+        *cell = v;
+    }
+}
+
 // Folds the group nodes of a split product: node g of cell c is ws[g][c]; the
 // nodes are the level-log2(S) row of the contract's tree, so the same
 // adjacent-pair fold with an odd tail carried finishes it. The fold is streamed

@@ -41,3 +41,21 @@ def test_quantised_rows(rows, cols):
     q, e = torch_ops.quantize_int8(torch.from_numpy(x).cuda())
     qo, eo = oracle.quantize_int8(x)
     assert _same(q, qo) and _same(e, eo)
+
+
+def test_gated_activation_layouts_agree():
+    """Four outputs a thread on aligned rows against one output a thread on the same values off the 16-byte grid."""
+    import ctypes
+    rng = np.random.default_rng(5)
+    for kind in (0, 4, 5):
+        gu = torch.from_numpy((rng.standard_normal((5, 2 * 72)) * 4).astype(np.float32)).cuda()
+        gu[0, :4] = torch.tensor([float("inf"), float("nan"), 1e-41, -1e-40], device="cuda")
+        off = torch.empty(gu.numel() + 1, device="cuda")
+        off[1:] = gu.reshape(-1)
+        outs = []
+        for src in (gu.data_ptr(), off.data_ptr() + 4):
+            out = torch.empty((5, 72), device="cuda")
+            _native.call("b200i_act_mul", 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(src), None,
+                         5, 72, 144, kind, 1)
+            outs.append(out.view(torch.int32))
+        assert torch.equal(*outs)
