@@ -6,6 +6,7 @@ declared in include/b200i.h.
 """
 import ctypes
 import os
+import threading
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 #: MOJOLEARN_B200_LIB overrides the in-tree library (a differently built libb200i.so with the same ABI).
@@ -123,10 +124,20 @@ def _declare(l):
         fn.argtypes = args
 
 
+class _Errors(threading.local):
+    """The message buffer of the calling thread (a call writes it before it returns, and nothing reads it later)."""
+
+    def __init__(self):
+        self.buf = ctypes.create_string_buffer(ERR_CAP)
+
+
+_errors = _Errors()
+
+
 def call(name, *args):
     """Call an entry point whose last two arguments are the error buffer; raise on a refusal."""
-    buf = ctypes.create_string_buffer(ERR_CAP)
-    status = getattr(lib(), name)(*args, ctypes.cast(buf, VP), ERR_CAP)
+    buf = _errors.buf
+    status = getattr(_lib or lib(), name)(*args, buf, ERR_CAP)
     if status != 0:
         raise NativeError(buf.value.decode("utf-8", "replace") or ("%s failed with status %d" % (name, status)))
     return status

@@ -12,6 +12,7 @@ the library's message.
 `torch.ops.mojolearn_b200.matmul` / `.linear_w` are registered as custom ops so
 the product can sit inside a torch program (fake-tensor shapes included).
 """
+import contextlib
 import ctypes
 
 import torch
@@ -33,11 +34,19 @@ def _check(t, name, dtype):
 
 
 def _vp(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _stream(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return torch.cuda.current_stream(device).cuda_stream
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on(device):
+    """The device guard of a call: nothing to do (and to undo) on the current device."""
+    return _HERE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def check_status(device=None):
@@ -96,7 +105,7 @@ def product(a, b, bscale=None, wkind=W_F32, op=OP_NN, out=None, plan=PLAN_AUTO, 
         if tuple(out.shape) != (m, n_out):
             raise ValueError("out must be (%d, %d)" % (m, n_out))
     lib = _native.lib()
-    with torch.cuda.device(dev):
+    with _on(dev):
         ws_bytes = int(lib.b200i_plan_workspace_bytes(m, n, k, plan, group_leaves))
         ws = torch.empty((max(ws_bytes, 16),), dtype=torch.uint8, device=dev) if ws_bytes else None
         if bias is None and act == ACT_NONE:
@@ -134,7 +143,7 @@ def product_nodes(a, b, bscale=None, wkind=W_F32, bias=None, act=ACT_NONE):
     out = torch.empty((m, n_out), dtype=torch.float32, device=dev)
     lib = _native.lib()
     nodes = ctypes.c_int64(1)
-    with torch.cuda.device(dev):
+    with _on(dev):
         ws_bytes = int(lib.b200i_plan_workspace_bytes(m, n, k, PLAN_AUTO, 0))
         ws = torch.empty((max(ws_bytes, 16),), dtype=torch.uint8, device=dev) if ws_bytes else None
         _native.call("b200i_gemm_w_nodes", dev.index, _stream(dev), _vp(out), _vp(a), _vp(b), _vp(bscale), wkind, m, n, k, OP_NT,
@@ -174,7 +183,7 @@ def to_bf16(x):
     _check(x, "x", torch.float32)
     out = torch.empty(x.shape, dtype=torch.uint16, device=x.device)
     if x.numel():
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             _native.call("b200i_to_bf16", x.device.index, _stream(x.device), _vp(out), _vp(x), x.numel())
     return out
 
@@ -185,7 +194,7 @@ def from_bf16(bits):
     _check(bits, "bits", torch.uint16)
     out = torch.empty(bits.shape, dtype=torch.float32, device=bits.device)
     if bits.numel():
-        with torch.cuda.device(bits.device):
+        with _on(bits.device):
             _native.call("b200i_from_bf16", bits.device.index, _stream(bits.device), _vp(out), _vp(bits), bits.numel())
     return out
 
@@ -197,7 +206,7 @@ def quantize_int8(x):
     rows, cols = x.shape
     codes = torch.empty((rows, cols), dtype=torch.int8, device=x.device)
     exps = torch.empty((rows,), dtype=torch.int32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         _native.call("b200i_quantize_int8", x.device.index, _stream(x.device), _vp(codes), _vp(exps), _vp(x), rows, cols)
     return codes, exps
 
@@ -207,7 +216,7 @@ def dequantize_int8(codes, exponents):
     _check(exponents, "exponents", torch.int32)
     rows, cols = codes.shape
     y = torch.empty((rows, cols), dtype=torch.float32, device=codes.device)
-    with torch.cuda.device(codes.device):
+    with _on(codes.device):
         _native.call("b200i_dequantize_int8", codes.device.index, _stream(codes.device), _vp(y), _vp(codes), _vp(exponents),
                      rows, cols)
     return y
@@ -223,7 +232,7 @@ def matmul_int8(qa, ea, qb, eb):
     if k != k2:
         raise ValueError("contracted extents disagree")
     c = torch.empty((m, n), dtype=torch.float32, device=qa.device)
-    with torch.cuda.device(qa.device):
+    with _on(qa.device):
         _native.call("b200i_gemm_int8", qa.device.index, _stream(qa.device), _vp(c), _vp(qa), _vp(ea), _vp(qb), _vp(eb), m, n, k)
     return c
 
@@ -238,7 +247,7 @@ def matmul_int15(ah, al, ea, bh, bl, eb):
     if k != k2 or al.shape != ah.shape or bl.shape != bh.shape:
         raise ValueError("planes of one operand must have one shape and the contracted extents must agree")
     c = torch.empty((m, n), dtype=torch.float32, device=ah.device)
-    with torch.cuda.device(ah.device):
+    with _on(ah.device):
         _native.call("b200i_gemm_int15", ah.device.index, _stream(ah.device), _vp(c), _vp(ah), _vp(al), _vp(ea), _vp(bh), _vp(bl), _vp(eb), m, n, k)
     return c
 

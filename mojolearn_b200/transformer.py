@@ -33,11 +33,11 @@ MAX_POSITIONS = 8192
 
 
 def _vp(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _stream(dev):
-    return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    return torch.cuda.current_stream(dev).cuda_stream
 
 
 def _vector(x, name, device):
