@@ -14,6 +14,7 @@
 #include "decode_pair.cuh"
 #include "gemm_int8_mma.cuh"
 #include "gemm_int8_tma.cuh"
+#include "gemm_int8_pair.cuh"
 #include "gemm_int15.cuh"
 #include "decoder.cuh"
 #include "gemm_tile.cuh"
@@ -751,9 +752,13 @@ int64_t b200i_gemm_int8(int64_t device, void *stream, float *c, const int8_t *qa
     if (gemm_int8_mma_fits(qa, qb, m, n, k)) {
         const signed char *sa = reinterpret_cast<const signed char *>(qa), *sb = reinterpret_cast<const signed char *>(qb);
         const int sms = sm_count(dev);
-        // enough 128 x 256 tiles for every SM: the persistent kernel fed by tensor-map copies; else the per-tile kernel
+        // SM pairs at every size (1024 x 4096 x 4096: 23 us against 100 for the per-tile kernel, 4096^3 60 against 62 for one CTA
+        // per tile), except where the contraction is so short that the store is all there is and the one-CTA kernel's wider
+        // spread of it wins (2048 x 50304 x 768: 157 against 174 us); the per-tile kernel where no tensor map can be made
         const long long wide = ((m + T8_BM - 1) / T8_BM) * ((n + T8_BN - 1) / T8_BN);
-        if (wide < sms || !launch_gemm_int8_tma(c, sa, ea, sb, eb, (int)m, (int)n, (int)k, sms, static_cast<cudaStream_t>(stream)))
+        const bool single = wide >= 4ll * sms && k < 1024;
+        if ((single || !launch_gemm_int8_pair(c, sa, ea, sb, eb, (int)m, (int)n, (int)k, static_cast<cudaStream_t>(stream))) &&
+            !launch_gemm_int8_tma(c, sa, ea, sb, eb, (int)m, (int)n, (int)k, sms, static_cast<cudaStream_t>(stream)))
             launch_gemm_int8_mma(c, sa, ea, sb, eb, (int)m, (int)n, (int)k, sms, static_cast<cudaStream_t>(stream));
     }
     else

@@ -36,6 +36,62 @@ __device__ __forceinline__ void t8_tma_load(void *dst, const CUtensorMap *map, u
                  : "memory");
 }
 
+// One 32 x 32 block of an accumulator, tensor memory to global: read by lanes (a lane holds a row), turned through the warp's
+// 32 x 33 words of shared memory so that a store covers 128 contiguous bytes of a row, converted and scaled on the way.
+__device__ __forceinline__ void i8_store_block(unsigned taddr, unsigned *turn, float *__restrict__ c, const int *__restrict__ eb, int ea_mine, int rbase,
+                                               int cbase, int m, int n, int lane) {
+    const int eb_mine = cbase + lane < n ? __ldg(eb + cbase + lane) : 0; // asked for before the accumulator is read
+    unsigned v[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
+        "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
+          "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
+          "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    // An exact int32 rounded once to float32 is what i32_to_f32_pinned spells, and what the conversion instruction does. With
+    // both exponents within +-63 the two power-of-two factors multiply it exactly (nothing underflows, an overflow is the
+    // same infinity), so a cell costs one conversion and two products; other blocks take the spelling cell by cell.
+    const bool plain = __all_sync(0xFFFFFFFFu, ea_mine >= -63 && ea_mine <= 63 && eb_mine >= -63 && eb_mine <= 63);
+    if (plain && (n & 3) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0) {
+        const float fa = pow2_f32(ea_mine), fb = pow2_f32(eb_mine); // of this lane's row; of this lane's column
+        float *ft = reinterpret_cast<float *>(turn);
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) { // 16-byte words, the lane's row permuted so that eight lanes fill the banks
+            const float4 w = make_float4(__int2float_rn((int)v[j]) * fa, __int2float_rn((int)v[j + 1]) * fa, __int2float_rn((int)v[j + 2]) * fa,
+                                         __int2float_rn((int)v[j + 3]) * fa);
+            *reinterpret_cast<float4 *>(ft + lane * 32 + ((j >> 2) ^ (lane & 7)) * 4) = w;
+        }
+        __syncwarp();
+        const int q = lane & 7, col = cbase + q * 4; // eight lanes a row, four rows an instruction: 128 contiguous bytes a row
+        const float b0 = __shfl_sync(0xFFFFFFFFu, fb, q * 4), b1 = __shfl_sync(0xFFFFFFFFu, fb, q * 4 + 1), b2 = __shfl_sync(0xFFFFFFFFu, fb, q * 4 + 2),
+                    b3 = __shfl_sync(0xFFFFFFFFu, fb, q * 4 + 3);
+        float *dst = c + (size_t)(rbase + (lane >> 3)) * n + col;
+#pragma unroll
+        for (int rr = 0; rr < 32; rr += 4) {
+            const int r = rr + (lane >> 3);
+            const float4 w = *reinterpret_cast<const float4 *>(ft + r * 32 + (q ^ (r & 7)) * 4);
+            if (rbase + r < m && col < n) *reinterpret_cast<float4 *>(dst + (size_t)rr * n) = make_float4(w.x * b0, w.y * b1, w.z * b2, w.w * b3);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j++) turn[lane * 33 + j] = v[j];
+        __syncwarp();
+        const int col = cbase + lane;
+#pragma unroll 4
+        for (int rr = 0; rr < 32; rr++) {
+            const long long esum = (long long)__shfl_sync(0xFFFFFFFFu, ea_mine, rr) + (long long)eb_mine;
+            const int eclamped = esum > 1000 ? 1000 : (esum < -1000 ? -1000 : (int)esum);
+            if (rbase + rr < m && col < n)
+                c[(size_t)(rbase + rr) * n + col] = nan_canon(ftz_bits(__fmul_rn(i32_to_f32_pinned((int)turn[rr * 33 + lane]), pow2_f32(eclamped))));
+        }
+    }
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(T8_THREADS, 1) gemm_int8_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                                                       float *__restrict__ c, const int *__restrict__ ea, const int *__restrict__ eb,
                                                                       int m, int n, int k, int tiles_n, int tiles) {
@@ -139,30 +195,7 @@ __global__ void __launch_bounds__(T8_THREADS, 1) gemm_int8_tma_kernel(const __gr
 #pragma unroll 1
             for (int cb = half * (T8_BN / 2); cb < (half + 1) * (T8_BN / 2); cb += 32) {
                 if (col0 + cb >= n) break; // uniform over the warp
-                unsigned v[32];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
-                    "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                      "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-                      "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                      "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(tmem + ((unsigned)(q * 32) << 16) + (unsigned)(acc * T8_BN + cb))
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int j = 0; j < 32; j++) turn[lane * 33 + j] = v[j];
-                __syncwarp();
-                const int col = col0 + cb + lane;
-                const long long eb_mine = col < n ? (long long)__ldg(eb + col) : 0;
-#pragma unroll 4
-                for (int rr = 0; rr < 32; rr++) {
-                    const long long esum = (long long)__shfl_sync(0xFFFFFFFFu, ea_mine, rr) + eb_mine;
-                    const int eclamped = esum > 1000 ? 1000 : (esum < -1000 ? -1000 : (int)esum);
-                    if (rbase + rr < m && col < n)
-                        c[(size_t)(rbase + rr) * n + col] = nan_canon(ftz_bits(__fmul_rn(i32_to_f32_pinned((int)turn[rr * 33 + lane]), pow2_f32(eclamped))));
-                }
-                __syncwarp();
+                i8_store_block(tmem + ((unsigned)(q * 32) << 16) + (unsigned)(acc * T8_BN + cb), turn, c, eb, ea_mine, rbase, col0 + cb, m, n, lane);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();

@@ -59,3 +59,16 @@ def test_gated_activation_layouts_agree():
                          5, 72, 144, kind, 1)
             outs.append(out.view(torch.int32))
         assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("m,n,k", [(2304, 2304, 144), (2500, 2060, 272), (130, 38000, 128), (4000, 2600, 16)])
+def test_int8_products_on_sm_pairs(m, n, k):
+    """Whole tiles, the halved last round, rows and columns past the edge, k below and across a stage."""
+    rng = np.random.default_rng(m)
+    qa, qb = rng.integers(-127, 128, (m, k)).astype(np.int8), rng.integers(-127, 128, (n, k)).astype(np.int8)
+    ea, eb = rng.integers(-60, 30, m).astype(np.int32), rng.integers(-60, 30, n).astype(np.int32)
+    got = torch_ops.matmul_int8(*(torch.from_numpy(t).cuda() for t in (qa, ea, qb, eb))).cpu().numpy()
+    rows = np.unique(np.r_[0, 127, 128, 255, 256, m - 1, rng.integers(0, m, 24)] % m)
+    want = oracle.nan_canon(oracle.gemm_int8(np.ascontiguousarray(qa[rows]), ea[rows], qb, eb))
+    assert got[rows].tobytes() == want.tobytes()
+    assert _native.lib().b200i_decode_status(-1) == 0
