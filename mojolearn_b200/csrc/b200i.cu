@@ -5,7 +5,9 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "../../include/b200i.h"
@@ -21,6 +23,7 @@
 #include "gemm_skinny.cuh"
 #include "gemm_packed.cuh"
 #include "gemm_tall.cuh"
+#include "host_copy.cuh"
 #include "gemm_skinny_reg.cuh"
 #include "lowbit.cuh"
 
@@ -519,8 +522,9 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
 // Grow-only per-device scratch for the host-pointer twins.
 constexpr int HOST_CHUNKS = 8; // row chunks of a pipelined host-pointer product
 struct HostPool {
-    void *buf[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    size_t cap[5] = {0, 0, 0, 0, 0};
+    void *buf[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    size_t cap[6] = {0, 0, 0, 0, 0, 0};
+    HostStage stage;                                    // pinned pieces for pageable arrays (host_copy.cuh)
     cudaStream_t stream = nullptr;                      // compute (and the only stream of the unpipelined twins)
     cudaStream_t s_in = nullptr, s_out = nullptr;       // host-to-device and device-to-host copies of the pipelined product
     cudaEvent_t ev[1 + 2 * HOST_CHUNKS] = {};           // weight landed; chunk landed / chunk computed
@@ -1177,7 +1181,7 @@ static int64_t attention_launch(int dev, cudaStream_t st, float *ctx, const floa
         const long long rows = b * n_heads * l;
         long long per_sm = (rows + sm_count(dev) - 1) / sm_count(dev);
         if (per_sm > 4) per_sm = 4;
-        long long stages = ((226ll * 1024 / per_sm - 1280) / 4 - ((s_grid + 3) & ~3)) / (CTX_NB * head_dim);
+        long long stages = ((226ll * 1024 / per_sm - 1664) / 4 - ((s_grid + 3) & ~3)) / (CTX_NB * head_dim);
         if (stages > CTX_ST_MAX) stages = CTX_ST_MAX;
         if (stages < CTX_ST) stages = CTX_ST;
         attn_context_row_kernel<<<(unsigned)rows, 128, attn_context_row_smem(s_grid, (int)head_dim, (int)stages), st>>>(
@@ -1523,6 +1527,54 @@ int64_t b200i_comm_destroy(void *comm) {
 
 // ---- host-pointer twins -------------------------------------------------------------------
 
+// The copies of one host-pointer call: through the worker threads for pageable arrays when there are megabytes of them
+// (see host_copy.cuh), else plain asynchronous copies.
+constexpr size_t HOST_STAGED_MIN = 4u << 20;
+struct HostTransfers {
+    struct Span {
+        const void *p;
+        size_t bytes;
+    };
+    HostTransfers(HostPool &pool, int dev, std::initializer_list<Span> spans) {
+        size_t total = 0;
+        for (const Span &s : spans)
+            if (host_is_pageable(s.p)) total += s.bytes;
+        if (total < HOST_STAGED_MIN) return;
+        if (host_stage_prepare(pool.stage) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        copier = new (std::nothrow) HostCopier(pool.stage, dev, total);
+        if (copier && !copier->ok()) {
+            delete copier;
+            copier = nullptr;
+        }
+    }
+    ~HostTransfers() { delete copier; } // joins the workers
+    HostTransfers(const HostTransfers &) = delete;
+    HostTransfers &operator=(const HostTransfers &) = delete;
+    cudaError_t to_device(void *dst, const void *src, size_t bytes, cudaStream_t st, int *segment) {
+        *segment = -1;
+        if (!copier || !host_is_pageable(src)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+        *segment = copier->add(true, dst, const_cast<void *>(src), bytes, bytes, 1, st);
+        return cudaSuccess;
+    }
+    void wait(int segment) { // until the segment's transfers are queued on its stream
+        if (copier) copier->wait(segment);
+    }
+    cudaError_t to_host(void *dst, size_t pitch, size_t width, const void *src, size_t rows, cudaStream_t st) {
+        if (!copier || !host_is_pageable(dst)) {
+            if (rows == 1) return cudaMemcpyAsync(dst, src, width, cudaMemcpyDeviceToHost, st);
+            return cudaMemcpy2DAsync(dst, pitch, src, width, width, rows, cudaMemcpyDeviceToHost, st);
+        }
+        const int seg = copier->add(false, const_cast<void *>(src), dst, width, rows == 1 ? width : pitch, rows, st);
+        if (seg < 0) return cudaErrorInvalidValue;
+        return cudaSuccess;
+    }
+    cudaError_t finish() { return copier ? copier->finish() : cudaSuccess; }
+    HostCopier *copier = nullptr;
+};
+
 // The host-pointer product, pipelined over three streams (PCIe is full duplex): host-to-device copies, packing and
 // multiplying, device-to-host copies. A tall left operand (m >= 1024) is cut by ROWS: the weight crosses and is
 // packed once, the rows of A cross in chunks while earlier chunks are multiplied and their rows of C return. A wide
@@ -1561,24 +1613,51 @@ static int64_t host_gemm_pipelined(int dev, HostPool &pool, float *c, const floa
     if (sbytes) CUDA_TRY(pool_get(dev, 3, sbytes, &ds));
     CUDA_TRY(pool_get(dev, 4, wsbytes, &dw));
     packed_configure();
+    const int sms = sm_count(dev);
     const int leaf = (int)leaf_size(k), leaves = (int)leaf_count(k), wpl = pk_windows_per_leaf(leaf);
     float *pa = static_cast<float *>(dw);
     float *pb = pa + pk_panel_floats(m, k);
     unsigned char *fa = reinterpret_cast<unsigned char *>(pb + pk_panel_floats(n, k));
     unsigned char *fb = fa + pk_flag_bytes(m, k);
     const bool k4 = (k % 4 == 0) && (leaves == 1 || leaf % 4 == 0); // the device copies are aligned: whole quads where the extents are
-    const int tiles_m = (int)((m + PK_TILE - 1) / PK_TILE), tiles_n = (int)((n + PK_TILE - 1) / PK_TILE);
+    // a chunk's tiles alone rarely fill the device: its leaves are split like any other product's
+    const Plan split = by_rows ? packed_split(Plan{PLAN_PACKED, leaves, 1}, std::min(per, m), n, k, sms)
+                               : packed_split(Plan{PLAN_PACKED, leaves, 1}, m, std::min(per, n), k, sms);
+    void *dn = nullptr;
+    if (split.groups > 1) CUDA_TRY(pool_get(dev, 5, (size_t)split.groups * (by_rows ? std::min(per, m) * n : m * std::min(per, n)) * 4, &dn));
+    auto product = [&](const float *pai, const unsigned char *fai, const float *pbi, const unsigned char *fbi, float *out, int64_t mm, int64_t nn) {
+        const int tn = (int)((nn + PK_TILE - 1) / PK_TILE);
+        PackedGemmArgs p{pai, pbi, fai, fbi, out, static_cast<float *>(dn), (int)mm, (int)nn, (int)k, leaf, leaves, wpl, split.group_leaves, split.groups, tn,
+                         (nn % 4 == 0 && aligned(out, 16)) ? 1 : 0};
+        gemm_packed_kernel<<<dim3((unsigned)(((mm + PK_TILE - 1) / PK_TILE) * tn), (unsigned)split.groups), PK_THREADS, PK_SMEM_BYTES, pool.stream>>>(p);
+        if (split.groups > 1) launch_fold_groups(static_cast<const float *>(dn), out, mm * nn, split.groups, pool.stream);
+        g_launches += split.groups > 1 ? 3 : 2; // with its packing pass
+    };
     // everything queued below waits for whatever the compute stream still holds from an earlier call
     CUDA_TRY(cudaEventRecord(pool.ev[0], pool.stream));
     CUDA_TRY(cudaStreamWaitEvent(pool.s_in, pool.ev[0], 0));
     CUDA_TRY(cudaStreamWaitEvent(pool.s_out, pool.ev[0], 0));
     // the operand that is not cut crosses first and is packed once
-    if (by_rows) {
-        CUDA_TRY(cudaMemcpyAsync(db, b, bbytes, cudaMemcpyHostToDevice, pool.s_in));
-        if (sbytes) CUDA_TRY(cudaMemcpyAsync(ds, bscale, sbytes, cudaMemcpyHostToDevice, pool.s_in));
-    } else {
-        CUDA_TRY(cudaMemcpyAsync(da, a, abytes, cudaMemcpyHostToDevice, pool.s_in));
-    }
+    HostTransfers io(pool, dev, {{a, abytes}, {b, bbytes}, {c, cbytes}});
+    const void *first = by_rows ? b : static_cast<const void *>(a);
+    int seg_first = -1, seg_in[HOST_CHUNKS + 1];
+    CUDA_TRY(io.to_device(by_rows ? db : da, first, by_rows ? bbytes : abytes, pool.s_in, &seg_first));
+    if (by_rows && sbytes) CUDA_TRY(cudaMemcpyAsync(ds, bscale, sbytes, cudaMemcpyHostToDevice, pool.s_in));
+    auto chunk_in = [&](int i) { // chunk i of the operand that is cut
+        const int64_t x0 = i * per, cnt = (extent - x0 < per) ? extent - x0 : per;
+        if (by_rows) return io.to_device(static_cast<float *>(da) + (size_t)x0 * k, a + (size_t)x0 * k, (size_t)cnt * k * 4, pool.s_in, &seg_in[i]);
+        return io.to_device(static_cast<unsigned char *>(db) + (size_t)x0 * k * es, static_cast<const unsigned char *>(b) + (size_t)x0 * k * es,
+                            (size_t)cnt * k * es, pool.s_in, &seg_in[i]);
+    };
+    auto chunk_out = [&](int i) { // chunk i of C, behind the kernel that wrote it
+        const int64_t x0 = i * per, cnt = (extent - x0 < per) ? extent - x0 : per;
+        cudaError_t e = cudaStreamWaitEvent(pool.s_out, pool.ev[2 + 2 * i], 0);
+        if (e != cudaSuccess) return e;
+        if (by_rows) return io.to_host(c + (size_t)x0 * n, (size_t)cnt * n * 4, (size_t)cnt * n * 4, static_cast<float *>(dc) + (size_t)x0 * n, 1, pool.s_out);
+        return io.to_host(c + x0, (size_t)n * 4, (size_t)cnt * 4, static_cast<float *>(dc) + (size_t)m * x0, (size_t)m, pool.s_out);
+    };
+    CUDA_TRY(chunk_in(0));
+    io.wait(seg_first);
     CUDA_TRY(cudaEventRecord(pool.ev[0], pool.s_in));
     CUDA_TRY(cudaStreamWaitEvent(pool.stream, pool.ev[0], 0));
     if (by_rows) {
@@ -1592,47 +1671,32 @@ static int64_t host_gemm_pipelined(int dev, HostPool &pool, float *c, const floa
     for (int i = 0; i < nch; i++) {
         const int64_t x0 = i * per, cnt = (extent - x0 < per) ? extent - x0 : per;
         const int64_t tile0 = x0 / PK_TILE;
+        if (i + 1 < nch) CUDA_TRY(chunk_in(i + 1)); // its copies go on while this chunk's kernels are queued
+        io.wait(seg_in[i]);
+        if (!by_rows && sbytes)
+            CUDA_TRY(cudaMemcpyAsync(static_cast<unsigned char *>(ds) + (size_t)x0 * 4, static_cast<const unsigned char *>(bscale) + (size_t)x0 * 4,
+                                     (size_t)cnt * 4, cudaMemcpyHostToDevice, pool.s_in));
+        CUDA_TRY(cudaEventRecord(pool.ev[1 + 2 * i], pool.s_in));
+        CUDA_TRY(cudaStreamWaitEvent(pool.stream, pool.ev[1 + 2 * i], 0));
         if (by_rows) {
-            float *dai = static_cast<float *>(da) + (size_t)x0 * k, *dci = static_cast<float *>(dc) + (size_t)x0 * n;
-            CUDA_TRY(cudaMemcpyAsync(dai, a + (size_t)x0 * k, (size_t)cnt * k * 4, cudaMemcpyHostToDevice, pool.s_in));
-            CUDA_TRY(cudaEventRecord(pool.ev[1 + 2 * i], pool.s_in));
-            CUDA_TRY(cudaStreamWaitEvent(pool.stream, pool.ev[1 + 2 * i], 0));
             float *pai = pa + (size_t)tile0 * k * PK_TILE;
             unsigned char *fai = fa + (size_t)tile0 * leaves * wpl;
-            PackArgs paargs{pai, fai, dai, nullptr, (int)cnt, (int)k, leaf, leaves, wpl, 1, k4};
+            PackArgs paargs{pai, fai, static_cast<float *>(da) + (size_t)x0 * k, nullptr, (int)cnt, (int)k, leaf, leaves, wpl, 1, k4};
             launch_pack_one(paargs, W_F32, pool.stream);
-            PackedGemmArgs p{pai, pb, fai, fb, dci, nullptr, (int)cnt, (int)n, (int)k, leaf, leaves, wpl, leaves, 1, tiles_n, (n % 4 == 0) ? 1 : 0};
-            dim3 grid((unsigned)(((cnt + PK_TILE - 1) / PK_TILE) * tiles_n), 1u);
-            gemm_packed_kernel<<<grid, PK_THREADS, PK_SMEM_BYTES, pool.stream>>>(p);
-            CUDA_TRY(cudaEventRecord(pool.ev[2 + 2 * i], pool.stream));
-            CUDA_TRY(cudaStreamWaitEvent(pool.s_out, pool.ev[2 + 2 * i], 0));
-            CUDA_TRY(cudaMemcpyAsync(c + (size_t)x0 * n, dci, (size_t)cnt * n * 4, cudaMemcpyDeviceToHost, pool.s_out));
+            product(pai, fai, pb, fb, static_cast<float *>(dc) + (size_t)x0 * n, cnt, n);
         } else {
-            unsigned char *dbi = static_cast<unsigned char *>(db) + (size_t)x0 * k * es;
-            float *dci = static_cast<float *>(dc) + (size_t)m * x0; // a dense [m, cnt] block
-            CUDA_TRY(cudaMemcpyAsync(dbi, static_cast<const unsigned char *>(b) + (size_t)x0 * k * es, (size_t)cnt * k * es,
-                                     cudaMemcpyHostToDevice, pool.s_in));
-            if (sbytes)
-                CUDA_TRY(cudaMemcpyAsync(static_cast<unsigned char *>(ds) + (size_t)x0 * 4, static_cast<const unsigned char *>(bscale) + (size_t)x0 * 4,
-                                         (size_t)cnt * 4, cudaMemcpyHostToDevice, pool.s_in));
-            CUDA_TRY(cudaEventRecord(pool.ev[1 + 2 * i], pool.s_in));
-            CUDA_TRY(cudaStreamWaitEvent(pool.stream, pool.ev[1 + 2 * i], 0));
             float *pbi = pb + (size_t)tile0 * k * PK_TILE;
             unsigned char *fbi = fb + (size_t)tile0 * leaves * wpl;
-            PackArgs pbargs{pbi, fbi, dbi, sbytes ? static_cast<unsigned char *>(ds) + (size_t)x0 * 4 : nullptr, (int)cnt, (int)k, leaf, leaves,
-                            wpl, 1, k4};
+            PackArgs pbargs{pbi, fbi, static_cast<unsigned char *>(db) + (size_t)x0 * k * es, sbytes ? static_cast<unsigned char *>(ds) + (size_t)x0 * 4 : nullptr,
+                            (int)cnt, (int)k, leaf, leaves, wpl, 1, k4};
             launch_pack_one(pbargs, wkind, pool.stream);
-            const int tiles_nc = (int)((cnt + PK_TILE - 1) / PK_TILE);
-            PackedGemmArgs p{pa, pbi, fa, fbi, dci, nullptr, (int)m, (int)cnt, (int)k, leaf, leaves, wpl, leaves, 1, tiles_nc,
-                             (cnt % 4 == 0 && (m * x0) % 4 == 0) ? 1 : 0};
-            dim3 grid((unsigned)(tiles_m * tiles_nc), 1u);
-            gemm_packed_kernel<<<grid, PK_THREADS, PK_SMEM_BYTES, pool.stream>>>(p);
-            CUDA_TRY(cudaEventRecord(pool.ev[2 + 2 * i], pool.stream));
-            CUDA_TRY(cudaStreamWaitEvent(pool.s_out, pool.ev[2 + 2 * i], 0));
-            CUDA_TRY(cudaMemcpy2DAsync(c + x0, (size_t)n * 4, dci, (size_t)cnt * 4, (size_t)cnt * 4, (size_t)m, cudaMemcpyDeviceToHost, pool.s_out));
+            product(pa, fa, pbi, fbi, static_cast<float *>(dc) + (size_t)m * x0, m, cnt); // a dense [m, cnt] block
         }
-        g_launches += 2;
+        CUDA_TRY(cudaEventRecord(pool.ev[2 + 2 * i], pool.stream));
+        if (i > 0) CUDA_TRY(chunk_out(i - 1));
     }
+    CUDA_TRY(chunk_out(nch - 1));
+    CUDA_TRY(io.finish());
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(pool.s_out));
     CUDA_TRY(cudaStreamSynchronize(pool.stream));
@@ -1669,16 +1733,21 @@ int64_t b200i_host_gemm_w(int64_t device, float *c, const float *a, const void *
     CUDA_TRY(pool_get(dev, 2, cbytes, &dc));
     if (sbytes) CUDA_TRY(pool_get(dev, 3, sbytes, &ds));
     if (wsbytes) CUDA_TRY(pool_get(dev, 4, (size_t)wsbytes, &dw));
-    CUDA_TRY(cudaMemcpyAsync(da, a, abytes, cudaMemcpyHostToDevice, pool.stream));
-    CUDA_TRY(cudaMemcpyAsync(db, b, bbytes, cudaMemcpyHostToDevice, pool.stream));
+    HostTransfers io(pool, dev, {{a, abytes}, {b, bbytes}, {c, cbytes}});
+    int seg_a, seg_b;
+    CUDA_TRY(io.to_device(da, a, abytes, pool.stream, &seg_a));
+    CUDA_TRY(io.to_device(db, b, bbytes, pool.stream, &seg_b));
     if (sbytes) {
         if (!bscale) return fail(err, err_cap, "identical gemm: int8 weight storage needs its per-row exponents or scales");
         CUDA_TRY(cudaMemcpyAsync(ds, bscale, sbytes, cudaMemcpyHostToDevice, pool.stream));
     }
+    io.wait(seg_a);
+    io.wait(seg_b);
     if (launch_product(dev, pool.stream, static_cast<float *>(dc), static_cast<const float *>(da), db, ds, (int)wkind, m, n, k,
                        (int)op, PLAN_AUTO, 0, dw, wsbytes, err, err_cap))
         return 1;
-    CUDA_TRY(cudaMemcpyAsync(c, dc, cbytes, cudaMemcpyDeviceToHost, pool.stream));
+    CUDA_TRY(io.to_host(c, cbytes, cbytes, dc, 1, pool.stream));
+    CUDA_TRY(io.finish());
     CUDA_TRY(cudaStreamSynchronize(pool.stream));
     return check_wait_status(err, err_cap, "identical gemm");
 }

@@ -72,3 +72,16 @@ def test_int8_products_on_sm_pairs(m, n, k):
     want = oracle.nan_canon(oracle.gemm_int8(np.ascontiguousarray(qa[rows]), ea[rows], qb, eb))
     assert got[rows].tobytes() == want.tobytes()
     assert _native.lib().b200i_decode_status(-1) == 0
+
+
+@pytest.mark.parametrize("m,n,k,opname", [(96, 2304, 1500, "NT"), (1100, 1000, 1030, "NN"), (40, 1500, 3000, "NN"), (2000, 70, 900, "TN")])
+def test_host_arrays_through_the_copy_threads(m, n, k, opname):
+    """Megabytes of pageable arrays: both ways of cutting the product, and the plain path."""
+    op = {"NN": linalg.OP_NN, "NT": linalg.OP_NT, "TN": linalg.OP_TN}[opname]
+    rng = np.random.default_rng(k)
+    a = rng.standard_normal((k, m) if opname == "TN" else (m, k)).astype(np.float32)
+    b = rng.standard_normal((n, k) if opname == "NT" else (k, n)).astype(np.float32)
+    want = torch_ops.product(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), op=op).cpu().numpy()
+    for _ in range(2):
+        got = linalg.matmul(a, b, transpose_a=opname == "TN", transpose_b=opname == "NT")
+        assert got.tobytes() == want.tobytes()
