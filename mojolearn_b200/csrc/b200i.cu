@@ -25,6 +25,7 @@
 #include "gemm_tall.cuh"
 #include "host_copy.cuh"
 #include "gemm_skinny_reg.cuh"
+#include "gemm_rows.cuh"
 #include "lowbit.cuh"
 
 using namespace b200i;
@@ -96,7 +97,7 @@ int64_t check_wait_status(char *err, int64_t err_cap, const char *who) {
 }
 
 // ---- plans -----------------------------------------------------------------------------
-enum { PLAN_AUTO = -1, PLAN_FLAT = 0, PLAN_T128 = 1, PLAN_T64 = 2, PLAN_DECODE = 3, PLAN_T32 = 4, PLAN_T128X64 = 5, PLAN_SKINNY = 6, PLAN_PACKED = 7, PLAN_TALL = 8 };
+enum { PLAN_AUTO = -1, PLAN_FLAT = 0, PLAN_T128 = 1, PLAN_T64 = 2, PLAN_DECODE = 3, PLAN_T32 = 4, PLAN_T128X64 = 5, PLAN_SKINNY = 6, PLAN_PACKED = 7, PLAN_TALL = 8, PLAN_ROWS = 9 };
 
 // Up to this many rows the weight-streaming decode plan wins; above, the skinny plan. Low-bit weights
 // switch earlier: at three and four rows the decode kernel's serial chains cost more than the register
@@ -248,6 +249,28 @@ inline bool packed_candidate(int tile_kind, long long m, long long n, long long 
 }
 size_t packed_need(long long m, long long n, long long k, int groups) {
     return round256(groups > 1 ? (size_t)groups * m * n * 4 : 0) + pk_workspace_bytes(m, n, k);
+}
+
+// A small decode batch with a column's whole contraction in one CTA (gemm_rows.cuh) up to sixteen leaves. Past that the
+// activations of all leaves leave too short a ring, and groups of eight leaves on as many more CTAs win in spite of the
+// second launch (float32 [11008, 4096] at 8 rows: 57 us against 67 in sixteens and 140 whole).
+Plan choose_rows(long long k) {
+    const int leaves = (int)leaf_count(k);
+    if (leaves <= 16) return Plan{PLAN_ROWS, leaves, 1};
+    int run = 8;
+    while ((leaves + run - 1) / run > MAX_GROUPS) run *= 2;
+    return Plan{PLAN_ROWS, run, (leaves + run - 1) / run};
+}
+// Where it wins (graph replay, folds included): float32 at 4 to 8 rows ([2304, 768] 6.5 against 14 us, [768, 3072] 8.6 against
+// 13.9, [50304, 768] 54 against 66, [11008, 4096] 57 against 80); low-bit weights while they are small enough to be bound by
+// latency, int8 ones also where they are deep (int8 [2304, 768] 5.3 against 9.4, [768, 3072] 7.3 against 8.9, [4096, 8192] 29
+// against 31, but [6144, 2048] 17.2 against 15.8 and bf16 [11008, 4096] no faster), and not at four rows where the leaf-pair kernel streams a large weight; 9 to 16 rows while
+// a CTA has one strip of sixteen columns (float32 [2304, 768] 8.9 against 16, [768, 3072] 11.5 against 15.8, but [3072, 768]
+// 16.4 against 15.7).
+inline bool rows_preferred(long long m, long long n, long long k, int wkind, int sms) {
+    if (m < 4 || (leaf_count(k) > 16 && rows_group_leaves(m) < choose_rows(k).group_leaves)) return false;
+    if (m <= 8) return wkind == W_F32 || n <= 3072 || (wkind != W_BF16 && m > 4 && k >= 4096);
+    return n <= 16ll * sms && (wkind == W_F32 || k <= 1024);
 }
 
 // A^T B of few cells over many rows: every leaf of every 32 x 32 tile as a warp of its own (gemm_tall.cuh).
@@ -413,6 +436,7 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         if (dec && m <= prefer_m && !(skinny && epilogue_pairs(g.epi))) plan = Plan{PLAN_DECODE, g.leaves, 1}; // (a gated store needs the skinny plan)
         else if (skinny) plan = choose_skinny(m, n, k, sm_count(dev), wkind != W_F32);
         else if (dec) plan = Plan{PLAN_DECODE, g.leaves, 1};
+        if (rows_plan_fits(m, n, k, op) && al16 && rows_preferred(m, n, k, wkind, sm_count(dev))) plan = choose_rows(k);
         if (tall_fits(m, n, k, op, wkind) && tall_candidate(m, n, k) && !leave_nodes && !epilogue_pairs(g.epi) && ws && aligned(ws, 4) &&
             (size_t)ws_bytes >= tall_workspace_bytes(m, n, k))
             plan = Plan{PLAN_TALL, 1, g.leaves};
@@ -455,7 +479,7 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         // a gated activation needs both columns of a pair in one thread: the skinny plans, whose threads own adjacent
         // columns, apply it in their own store or in the group fold; no other plan spells it
         const bool fold_ok = plan.groups == 1 || (((long long)m * n) % 4 == 0 && aligned(ws, 16) && aligned(c, 8));
-        if (plan.kind != PLAN_SKINNY || n % 4 != 0 || !fold_ok)
+        if ((plan.kind != PLAN_SKINNY && plan.kind != PLAN_ROWS) || n % 4 != 0 || !fold_ok)
             return fail(err, err_cap, "identical gemm: the gated store activation needs the skinny plan (up to 32 rows, op NT, k a multiple of 16) and n a multiple of 4");
     }
     int tslot = -1;
@@ -468,6 +492,12 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         if (!decode_plan_fits(m, n, k, op, wkind) || !aligned(b, 16) || !aligned(a, 16))
             return fail(err, err_cap, "identical gemm: the decode plan needs op NT, m <= %d, k a multiple of 16 and 16-byte aligned weights", DECODE_MAX_M);
         g_launches += launch_decode_plan(g, sm_count(dev), st);
+    } else if (plan.kind == PLAN_ROWS) {
+        if (!rows_plan_fits(m, n, k, op) || !aligned(b, 16) || !aligned(a, 16) || plan.group_leaves > rows_group_leaves(m))
+            return fail(err, err_cap, "identical gemm: the rows plan needs op NT, m <= %d, k a multiple of 16, 16-byte aligned operands and leaf groups of at most %d", RW_MAX_ROWS,
+                        rows_group_leaves(m));
+        launch_rows(g, sm_count(dev), st);
+        g_launches++;
     } else if (plan.kind == PLAN_TALL) {
         launch_tall(g, st); // its own fold, the store epilogue included
         g_launches += 2;
@@ -507,7 +537,8 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         const long long cells = (long long)m * n;
         launch_fold_groups(g.ws, c, cells, plan.groups, st, g.epi, g.n);
         g_launches++;
-    } else if (epilogue_on(g.epi) && plan.kind != PLAN_SKINNY && plan.kind != PLAN_DECODE && plan.kind != PLAN_TALL) {
+    } else if (epilogue_on(g.epi) && plan.kind != PLAN_SKINNY && plan.kind != PLAN_DECODE && plan.kind != PLAN_TALL &&
+               plan.kind != PLAN_ROWS) {
         // the tiled, packed and flat plans store plain product words; their epilogue is a pass of its own
         const long long cells = (long long)m * n;
         if (n % 4 == 0 && aligned(c, 16))
@@ -600,6 +631,7 @@ int64_t b200i_workspace_bytes(int64_t m, int64_t n, int64_t k) {
             const Plan q = choose_skinny(m, n, k, sm_count(dev), lowbit != 0);
             if (q.groups > groups) groups = q.groups;
         }
+        if (rows_plan_fits(m, n, k, OP_NT)) groups = std::max(groups, choose_rows(k).groups);
     }
     return groups > 1 ? (int64_t)groups * m * n * 4 : 0;
 }

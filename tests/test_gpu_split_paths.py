@@ -85,3 +85,54 @@ def test_host_arrays_through_the_copy_threads(m, n, k, opname):
     for _ in range(2):
         got = linalg.matmul(a, b, transpose_a=opname == "TN", transpose_b=opname == "NT")
         assert got.tobytes() == want.tobytes()
+
+
+def _weight(rng, n, k, kind):
+    if kind == linalg.W_F32:
+        w = rng.standard_normal((n, k)).astype(np.float32)
+        return w, None, w
+    if kind == linalg.W_BF16:
+        bits = oracle.to_bf16(rng.standard_normal((n, k)).astype(np.float32))
+        return bits, None, oracle.from_bf16(bits)
+    codes = rng.integers(-127, 128, (n, k)).astype(np.int8)
+    if kind == linalg.W_INT8_EXP:
+        e = rng.integers(-13, -9, n).astype(np.int32)
+        e[0], e[n // 2], e[n - 1] = -100, 118, -140  # factors past the short spellings
+        return codes, e, oracle.dequantize_int8(codes, e)
+    s = rng.uniform(0.001, 0.02, n).astype(np.float32)
+    s[0] = 1e-36
+    return codes, s, oracle.dequantize_int8_scaled(codes, s)
+
+
+ROWS_SHAPES = [(2, 16), (24, 128), (768, 768), (305, 784), (1186, 144), (770, 3072), (300, 5136), (9600, 256), (20001, 128)]
+
+
+@pytest.mark.parametrize("kind", [linalg.W_F32, linalg.W_BF16, linalg.W_INT8_EXP, linalg.W_INT8_SCALE])
+@pytest.mark.parametrize("m", [1, 5, 8, 9, 16])
+def test_rows_plan(m, kind):
+    """A column's whole contraction in one CTA: every strip width, runs of one to four leaves, leaf groups past 4096 / 2048
+    steps, strips past the last column, rows past m."""
+    for n, k in ROWS_SHAPES:
+        rng = np.random.default_rng(m * 31 + n + k + kind)
+        w, scale, dense = _weight(rng, n, k, kind)
+        a = rng.standard_normal((m, k)).astype(np.float32)
+        a[m // 2, k // 3] = 1e-41
+        want = oracle.nan_canon(oracle.gemm_rows(a, dense, oracle.OP_NT))
+        da, dw = torch.from_numpy(a).cuda(), torch.from_numpy(w).cuda()
+        ds = torch.from_numpy(scale).cuda() if scale is not None else None
+        cap = 32 if m <= 8 else 16
+        gl = cap if oracle.leaf_count(k) > cap else 0
+        assert _same(torch_ops.product(da, dw, ds, kind, linalg.OP_NT, plan=torch_ops.PLAN_ROWS, group_leaves=gl), want), (n, k)
+        assert _same(torch_ops.product(da, dw, ds, kind, linalg.OP_NT), want), (n, k)
+
+
+@pytest.mark.parametrize("act", [torch_ops.ACT_GELU_ERF, torch_ops.ACT_SILU, torch_ops.ACT_PAIR_SWIGLU, torch_ops.ACT_PAIR_GEGLU_TANH])
+@pytest.mark.parametrize("n,k", [(1000, 768), (48, 5136)])
+def test_rows_plan_store_epilogues(n, k, act):
+    rng = np.random.default_rng(n + act)
+    a, w = torch.from_numpy(rng.standard_normal((7, k)).astype(np.float32)).cuda(), torch.from_numpy(rng.standard_normal((n, k)).astype(np.float32)).cuda()
+    bias = torch.from_numpy(rng.standard_normal(n).astype(np.float32)).cuda()
+    gl = 32 if k > 4096 else 0
+    want = torch_ops.product(a, w, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_SKINNY, bias=bias, act=act)
+    got = torch_ops.product(a, w, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_ROWS, group_leaves=gl, bias=bias, act=act)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
