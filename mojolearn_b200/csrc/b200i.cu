@@ -26,6 +26,7 @@
 #include "host_copy.cuh"
 #include "gemm_skinny_reg.cuh"
 #include "gemm_rows.cuh"
+#include "gemm_band.cuh"
 #include "lowbit.cuh"
 
 using namespace b200i;
@@ -97,7 +98,7 @@ int64_t check_wait_status(char *err, int64_t err_cap, const char *who) {
 }
 
 // ---- plans -----------------------------------------------------------------------------
-enum { PLAN_AUTO = -1, PLAN_FLAT = 0, PLAN_T128 = 1, PLAN_T64 = 2, PLAN_DECODE = 3, PLAN_T32 = 4, PLAN_T128X64 = 5, PLAN_SKINNY = 6, PLAN_PACKED = 7, PLAN_TALL = 8, PLAN_ROWS = 9 };
+enum { PLAN_AUTO = -1, PLAN_FLAT = 0, PLAN_T128 = 1, PLAN_T64 = 2, PLAN_DECODE = 3, PLAN_T32 = 4, PLAN_T128X64 = 5, PLAN_SKINNY = 6, PLAN_PACKED = 7, PLAN_TALL = 8, PLAN_ROWS = 9, PLAN_BAND = 10 };
 
 // Up to this many rows the weight-streaming decode plan wins; above, the skinny plan. Low-bit weights
 // switch earlier: at three and four rows the decode kernel's serial chains cost more than the register
@@ -273,6 +274,33 @@ inline bool rows_preferred(long long m, long long n, long long k, int wkind, int
     return n <= 16ll * sms && (wkind == W_F32 || k <= 1024);
 }
 
+// 9 to 32 rows: the leaf split of the band kernel. Modelled time in microseconds: waves of CTAs over two slots per SM
+// (leaves per CTA at the kernel's rate, a last wave that fills at most half the slots counting 0.55 because its CTAs are
+// alone on their SMs, + 1 us to start), plus the second launch and the L2-resident node traffic of the fold.
+Plan choose_band(long long m, long long n, long long k, int sms) {
+    const int leaves = (int)leaf_count(k) > 0 ? (int)leaf_count(k) : 1;
+    const int max_s = pow2_floor(leaves) * ((leaves & (leaves - 1)) ? 2 : 1);
+    const long long tiles = (n + BD_BN - 1) / BD_BN, slots = 2ll * sms;
+    const double leaf_us = m <= 16 ? 5.5 : 9.5;
+    int min_s = 1;
+    while ((leaves + min_s - 1) / min_s > MAX_GROUPS) min_s *= 2;
+    int best = max_s;
+    double best_t = 1e300;
+    for (int sl = max_s; sl >= min_s; sl /= 2) {
+        const int groups = (leaves + sl - 1) / sl;
+        const long long ctas = tiles * groups, whole = ctas / slots, rest = ctas % slots;
+        const double waves = (double)whole + (rest == 0 ? 0.0 : (2 * rest <= slots ? 0.55 : 1.0));
+        double t = waves * (std::min(sl, leaves) * leaf_us + 1.0);
+        if (groups > 1) t += 2.5 + (double)groups * m * n * 8.0 / 7.5e6;
+        if (t < best_t) { best_t = t; best = sl; }
+    }
+    Plan p{PLAN_BAND, best, (leaves + best - 1) / best};
+    if (p.groups <= 1) p.group_leaves = leaves;
+    return p;
+}
+// Float32 weights from ten million words up (the sizes on both sides of the line stand in gemm_band.cuh).
+inline bool band_preferred(long long n, long long k, int wkind) { return wkind == W_F32 && (double)n * (double)k >= 1.0e7; }
+
 // A^T B of few cells over many rows: every leaf of every 32 x 32 tile as a warp of its own (gemm_tall.cuh).
 constexpr long long TALL_MIN_LEAVES = 16;
 inline bool tall_fits(long long m, long long n, long long k, int op, int wkind) {
@@ -437,6 +465,7 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         else if (skinny) plan = choose_skinny(m, n, k, sm_count(dev), wkind != W_F32);
         else if (dec) plan = Plan{PLAN_DECODE, g.leaves, 1};
         if (rows_plan_fits(m, n, k, op) && al16 && rows_preferred(m, n, k, wkind, sm_count(dev))) plan = choose_rows(k);
+        if (skinny && m > 8 && band_preferred(n, k, wkind)) plan = choose_band(m, n, k, sm_count(dev));
         if (tall_fits(m, n, k, op, wkind) && tall_candidate(m, n, k) && !leave_nodes && !epilogue_pairs(g.epi) && ws && aligned(ws, 4) &&
             (size_t)ws_bytes >= tall_workspace_bytes(m, n, k))
             plan = Plan{PLAN_TALL, 1, g.leaves};
@@ -479,7 +508,7 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         // a gated activation needs both columns of a pair in one thread: the skinny plans, whose threads own adjacent
         // columns, apply it in their own store or in the group fold; no other plan spells it
         const bool fold_ok = plan.groups == 1 || (((long long)m * n) % 4 == 0 && aligned(ws, 16) && aligned(c, 8));
-        if ((plan.kind != PLAN_SKINNY && plan.kind != PLAN_ROWS) || n % 4 != 0 || !fold_ok)
+        if ((plan.kind != PLAN_SKINNY && plan.kind != PLAN_ROWS && plan.kind != PLAN_BAND) || n % 4 != 0 || !fold_ok)
             return fail(err, err_cap, "identical gemm: the gated store activation needs the skinny plan (up to 32 rows, op NT, k a multiple of 16) and n a multiple of 4");
     }
     int tslot = -1;
@@ -497,6 +526,11 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
             return fail(err, err_cap, "identical gemm: the rows plan needs op NT, m <= %d, k a multiple of 16, 16-byte aligned operands and leaf groups of at most %d", RW_MAX_ROWS,
                         rows_group_leaves(m));
         launch_rows(g, sm_count(dev), st);
+        g_launches++;
+    } else if (plan.kind == PLAN_BAND) {
+        if (!skinny_plan_fits(m, n, k, op) || wkind != W_F32 || !aligned(b, 16) || !aligned(a, 16))
+            return fail(err, err_cap, "identical gemm: the band plan needs op NT, m <= 32, float32 weights, k a multiple of 16 and 16-byte aligned operands");
+        launch_band(g, st);
         g_launches++;
     } else if (plan.kind == PLAN_TALL) {
         launch_tall(g, st); // its own fold, the store epilogue included
@@ -538,7 +572,7 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         launch_fold_groups(g.ws, c, cells, plan.groups, st, g.epi, g.n);
         g_launches++;
     } else if (epilogue_on(g.epi) && plan.kind != PLAN_SKINNY && plan.kind != PLAN_DECODE && plan.kind != PLAN_TALL &&
-               plan.kind != PLAN_ROWS) {
+               plan.kind != PLAN_ROWS && plan.kind != PLAN_BAND) {
         // the tiled, packed and flat plans store plain product words; their epilogue is a pass of its own
         const long long cells = (long long)m * n;
         if (n % 4 == 0 && aligned(c, 16))
@@ -632,6 +666,7 @@ int64_t b200i_workspace_bytes(int64_t m, int64_t n, int64_t k) {
             if (q.groups > groups) groups = q.groups;
         }
         if (rows_plan_fits(m, n, k, OP_NT)) groups = std::max(groups, choose_rows(k).groups);
+        groups = std::max(groups, choose_band(m, n, k, sm_count(dev)).groups);
     }
     return groups > 1 ? (int64_t)groups * m * n * 4 : 0;
 }

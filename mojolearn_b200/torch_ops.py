@@ -14,13 +14,14 @@ the product can sit inside a torch program (fake-tensor shapes included).
 """
 import contextlib
 import ctypes
+import functools
 
 import torch
 
 from . import _native
 from .linalg import OP_NN, OP_NT, OP_TN, W_BF16, W_F32, W_INT8_EXP, W_INT8_SCALE, leaf_count
 
-PLAN_AUTO, PLAN_FLAT, PLAN_T128, PLAN_T64, PLAN_DECODE, PLAN_T32, PLAN_T128X64, PLAN_SKINNY, PLAN_PACKED, PLAN_TALL, PLAN_ROWS = -1, 0, 1, 2, 3, 4, 5, 6, 7, 8, 9
+PLAN_AUTO, PLAN_FLAT, PLAN_T128, PLAN_T64, PLAN_DECODE, PLAN_T32, PLAN_T128X64, PLAN_SKINNY, PLAN_PACKED, PLAN_TALL, PLAN_ROWS, PLAN_BAND = -1, 0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10
 
 
 def _check(t, name, dtype):
@@ -37,8 +38,19 @@ def _vp(t):
     return t.data_ptr() if t is not None else None
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # the handle without a Stream object around it
+
+
 def _stream(device):
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
     return torch.cuda.current_stream(device).cuda_stream
+
+
+@functools.lru_cache(maxsize=4096)
+def _workspace_bytes(device_index, m, n, k, plan, group_leaves):
+    """A pure function of the shape, the plan and the device's SM count (the device is current when this is called)."""
+    return int(_native.lib().b200i_plan_workspace_bytes(m, n, k, plan, group_leaves))
 
 
 _HERE = contextlib.nullcontext()
@@ -104,9 +116,8 @@ def product(a, b, bscale=None, wkind=W_F32, op=OP_NN, out=None, plan=PLAN_AUTO, 
         _check(out, "out", torch.float32)
         if tuple(out.shape) != (m, n_out):
             raise ValueError("out must be (%d, %d)" % (m, n_out))
-    lib = _native.lib()
     with _on(dev):
-        ws_bytes = int(lib.b200i_plan_workspace_bytes(m, n, k, plan, group_leaves))
+        ws_bytes = _workspace_bytes(dev.index, m, n, k, plan, group_leaves)
         ws = torch.empty((max(ws_bytes, 16),), dtype=torch.uint8, device=dev) if ws_bytes else None
         if bias is None and act == ACT_NONE:
             _native.call("b200i_gemm_w_plan", dev.index, _stream(dev), _vp(out), _vp(a), _vp(b), _vp(bscale), wkind, m, n, k,

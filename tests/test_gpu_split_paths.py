@@ -136,3 +136,17 @@ def test_rows_plan_store_epilogues(n, k, act):
     want = torch_ops.product(a, w, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_SKINNY, bias=bias, act=act)
     got = torch_ops.product(a, w, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_ROWS, group_leaves=gl, bias=bias, act=act)
     assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("m", [9, 16, 17, 32])
+@pytest.mark.parametrize("n,k", [(24, 128), (770, 784), (255, 16), (1001, 144), (300, 5136)])
+def test_band_plan(m, n, k):
+    """256-column tiles with ragged edges, leaf groups, a chunk of activations restaged every two leaves."""
+    rng = np.random.default_rng(m + n + k)
+    a, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    a[m // 2, k // 3], w[n - 1, k - 1], w[7, 3] = 1e-41, np.inf, 3e-39
+    want = oracle.nan_canon(oracle.gemm_rows(a, w, oracle.OP_NT))
+    da, dw = torch.from_numpy(a).cuda(), torch.from_numpy(w).cuda()
+    for gl in (0, 1, 4):
+        if gl <= oracle.leaf_count(k):
+            assert _same(torch_ops.product(da, dw, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_BAND, group_leaves=gl), want), gl
