@@ -350,7 +350,8 @@ void packed_configure() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaFuncSetAttribute(gemm_packed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PK_SMEM_BYTES);
+        cudaFuncSetAttribute(gemm_packed_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PK_SMEM_BYTES);
+        cudaFuncSetAttribute(gemm_packed_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PK_RAW_SMEM_BYTES);
         configured[dev] = true;
     }
 }
@@ -385,12 +386,17 @@ int launch_packed(const GemmArgs &g, int groups, unsigned char *scratch, cudaStr
     const bool a_kc = g.op != OP_TN, b_kc = g.op == OP_NT;
     PackArgs a{pa, fa, g.a, nullptr, g.m, g.k, g.leaf, g.leaves, wpl, a_kc, (a_kc ? k4 : g.m % 4 == 0) && aligned(g.a, 16)};
     PackArgs b{pb, fb, g.b, g.bscale, g.n, g.k, g.leaf, g.leaves, wpl, b_kc, (b_kc ? k4 : g.n % 4 == 0) && aligned(g.b, balign)};
-    launch_pack(a, b, g.wkind, st);
+    // one row of tiles over float32 rows of whole quads, and leaves of whole stages: B is read where it lies
+    const bool raw = g.m <= PK_TILE && g.wkind == W_F32 && b.kcontig && b.vec && (g.leaves == 1 || g.leaf % PK_SK == 0);
+    if (raw) launch_pack_one(a, W_F32, st);
+    else launch_pack(a, b, g.wkind, st);
     PackedGemmArgs p{pa, pb, fa, fb, g.c, g.ws, g.m, g.n, g.k, g.leaf, g.leaves, wpl, g.group_leaves, groups,
                      (g.n + PK_TILE - 1) / PK_TILE, g.vec_c};
     dim3 grid((unsigned)(((g.m + PK_TILE - 1) / PK_TILE) * p.tiles_n), (unsigned)groups);
     const int tslot = timing_begin(st);
-    gemm_packed_kernel<<<grid, PK_THREADS, PK_SMEM_BYTES, st>>>(p);
+    p.braw = static_cast<const float *>(g.b);
+    if (raw) gemm_packed_kernel<true><<<grid, PK_THREADS, PK_RAW_SMEM_BYTES, st>>>(p);
+    else gemm_packed_kernel<false><<<grid, PK_THREADS, PK_SMEM_BYTES, st>>>(p);
     timing_end(tslot, st);
     return 2;
 }
@@ -1696,7 +1702,7 @@ static int64_t host_gemm_pipelined(int dev, HostPool &pool, float *c, const floa
         const int tn = (int)((nn + PK_TILE - 1) / PK_TILE);
         PackedGemmArgs p{pai, pbi, fai, fbi, out, static_cast<float *>(dn), (int)mm, (int)nn, (int)k, leaf, leaves, wpl, split.group_leaves, split.groups, tn,
                          (nn % 4 == 0 && aligned(out, 16)) ? 1 : 0};
-        gemm_packed_kernel<<<dim3((unsigned)(((mm + PK_TILE - 1) / PK_TILE) * tn), (unsigned)split.groups), PK_THREADS, PK_SMEM_BYTES, pool.stream>>>(p);
+        gemm_packed_kernel<false><<<dim3((unsigned)(((mm + PK_TILE - 1) / PK_TILE) * tn), (unsigned)split.groups), PK_THREADS, PK_SMEM_BYTES, pool.stream>>>(p);
         if (split.groups > 1) launch_fold_groups(static_cast<const float *>(dn), out, mm * nn, split.groups, pool.stream);
         g_launches += split.groups > 1 ? 3 : 2; // with its packing pass
     };
