@@ -980,22 +980,31 @@ int64_t b200i_gemm_f32_noalloc(int64_t device, void *stream, float *c, const flo
     if (select_device(device, err, err_cap, &dev)) return 1;     \
     cudaStream_t st = static_cast<cudaStream_t>(stream)
 
+// A CTA of four warps per row while that leaves at most two on an SM (a decode step), else a warp per row.
+static cudaError_t launch_norm_rows(int dev, cudaStream_t st, float *out, const float *x, const float *w, const float *bias, int64_t rows, int width, float eps,
+                                    int kind, const float *delta, float *sum_out, int wpc, size_t smem) {
+    static std::atomic<bool> configured[64];
+    if (dev >= 0 && dev < 64 && !configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(norm_rows_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(norm_rows_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e != cudaSuccess) return e;
+        configured[dev] = true;
+    }
+    if (rows <= 2 * sm_count(dev)) norm_rows_kernel<4><<<(unsigned)rows, 128, smem, st>>>(out, x, w, bias, rows, width, eps, kind, delta, sum_out);
+    else norm_rows_kernel<1><<<(unsigned)((rows + wpc - 1) / wpc), 32 * wpc, smem, st>>>(out, x, w, bias, rows, width, eps, kind, delta, sum_out);
+    return cudaSuccess;
+}
+
 int64_t b200i_norm(int64_t device, void *stream, float *out, const float *x, const float *w, const float *bias, int64_t rows,
                    int64_t width, double eps, int64_t kind, char *err, int64_t err_cap) {
     SEAM_PROLOGUE();
     if (rows <= 0 || width <= 0 || !out || !x || !w) return fail(err, err_cap, "norm: bad arguments");
     if (kind < NORM_RMS || kind > NORM_RMS_OFFSET) return fail(err, err_cap, "norm: norm kind %lld is not spelled", (long long)kind);
     if (bias && kind != NORM_LAYER) return fail(err, err_cap, "norm: an RMSNorm carries no bias (norm_bias needs layernorm)");
-    const int wpc = rows >= 1024 ? 4 : 1; // warps (rows) per CTA: few rows spread over the SMs
+    const int wpc = rows >= 1024 ? 4 : 1; // rows per CTA: few rows spread over the SMs
     const size_t smem = (size_t)wpc * (size_t)((width + 3) & ~3ll) * sizeof(float);
     if (smem <= 200 * 1024) {
-        static std::atomic<bool> configured[64];
-        if (dev >= 0 && dev < 64 && !configured[dev]) {
-            CUDA_TRY(cudaFuncSetAttribute(norm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            configured[dev] = true;
-        }
-        norm_rows_kernel<<<(unsigned)((rows + wpc - 1) / wpc), 32 * wpc, smem, st>>>(out, x, w, bias, rows, (int)width, (float)eps, (int)kind,
-                                                                                     nullptr, nullptr);
+        CUDA_TRY(launch_norm_rows(dev, st, out, x, w, bias, rows, (int)width, (float)eps, (int)kind, nullptr, nullptr, wpc, smem));
     } else {
         const long long threads = rows * 32;
         norm_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(out, x, w, bias, rows, (int)width, (float)eps, (int)kind);
@@ -1014,13 +1023,7 @@ int64_t b200i_add_norm(int64_t device, void *stream, float *out, float *sum_out,
     const int wpc = rows >= 1024 ? 4 : 1;
     const size_t smem = (size_t)wpc * (size_t)((width + 3) & ~3ll) * sizeof(float);
     if (smem <= 200 * 1024) {
-        static std::atomic<bool> configured[64];
-        if (dev >= 0 && dev < 64 && !configured[dev]) {
-            CUDA_TRY(cudaFuncSetAttribute(norm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            configured[dev] = true;
-        }
-        norm_rows_kernel<<<(unsigned)((rows + wpc - 1) / wpc), 32 * wpc, smem, st>>>(out, x, w, bias, rows, (int)width, (float)eps, (int)kind,
-                                                                                     delta, sum_out);
+        CUDA_TRY(launch_norm_rows(dev, st, out, x, w, bias, rows, (int)width, (float)eps, (int)kind, delta, sum_out, wpc, smem));
         g_launches++;
     } else { // a row too wide for shared memory: the two seams one after the other
         const long long count = rows * width;
@@ -1227,10 +1230,10 @@ static int64_t attention_launch(int dev, cudaStream_t st, float *ctx, const floa
         static std::atomic<bool> configured[64];                                                                                          \
         if (dev >= 0 && dev < 64 && !configured[dev]) {                                                                           \
             CUDA_TRY(cudaFuncSetAttribute(attn_scores_small_kernel<LQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,              \
-                                          attn_scores_small_smem<LQ>()));                                                         \
+                                          attn_scores_small_smem<LQ>(K_LEAF_MIN)));                                               \
             configured[dev] = true;                                                                                               \
         }                                                                                                                         \
-        attn_scores_small_kernel<LQ><<<gs, 128, attn_scores_small_smem<LQ>(), st>>>(\
+        attn_scores_small_kernel<LQ><<<gs, 128, attn_scores_small_smem<LQ>((int)head_dim), st>>>(\
             scores, q, kcache, (int)b, (int)l, (int)n_heads, (int)n_kv, (int)head_dim, (int)cap, key_lo, s, own0, (int)window,    \
             position, softcap);                                                                                                   \
     } while (0)

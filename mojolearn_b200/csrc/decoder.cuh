@@ -79,22 +79,30 @@ __device__ __forceinline__ float row_chain(const float *xs, int dm, Step step) {
 
 // With `delta` the row normalised is the residual sum ftz(ftz(src) + ftz(delta)) (seam S22 / S23), which is
 // also written to `sum_out`: the residual add and the norm that always follows it, in one pass over the row.
-constexpr int NORM_WREG = 16; // 128-bit words of the weight row a lane can hold: rows up to 2048 wide
+// WPR warps share a row: one where there are rows enough to fill the device, four (a CTA to itself) for the few rows of a
+// decode step, where a lone warp's loads, conversions and stores take longer than the chain (2134 instructions at 768
+// wide). Every warp of a row walks the whole chain, so none waits for another's result.
+constexpr int NORM_WREG = 16; // 128-bit words of the weight row the lanes of a warp's width can hold: rows up to 2048 wide
+template <int WPR>
 __global__ void __launch_bounds__(128) norm_rows_kernel(float *__restrict__ out, const float *__restrict__ src, const float *__restrict__ w,
                                                         const float *__restrict__ bias, long long rows, int dm, float eps, int kind,
                                                         const float *__restrict__ delta, float *__restrict__ sum_out) {
     extern __shared__ __align__(16) float norm_smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
-    if (row >= rows) return; // warps are independent: only warp-level barriers below
+    constexpr int NT = 32 * WPR, AHEAD = 8 / WPR > 4 ? 8 : 4; // threads of a row; 128-bit loads a thread has in flight
+    static_assert(WPR == 1 || NT == 128, "several warps to a row: the row has the CTA");
+    const int lane = threadIdx.x % NT, warp = threadIdx.x / NT;
+    const long long row = (long long)blockIdx.x * (blockDim.x / NT) + warp;
+    if (row >= rows) return; // rows are independent: only barriers of a row's own threads below
+    auto row_sync = [] { if (WPR == 1) __syncwarp(); else __syncthreads(); };
+    auto row_all = [](bool p) { return WPR == 1 ? (bool)__all_sync(0xFFFFFFFFu, p) : (bool)__syncthreads_and(p); };
     // The weight row does not depend on the chain: a lane asks for its words of it before anything else, so that the
     // last phase finds them in registers instead of paying a round trip to L2 per 512 columns after the chain.
     const bool w_early = (dm % 4 == 0) && dm <= NORM_WREG * 128 && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
-    float4 wreg[NORM_WREG];
+    float4 wreg[NORM_WREG / WPR];
     if (w_early) {
 #pragma unroll
-        for (int u = 0; u < NORM_WREG; u++)
-            wreg[u] = (lane * 4 + u * 128 < dm) ? __ldg(reinterpret_cast<const float4 *>(w + lane * 4 + u * 128)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int u = 0; u < NORM_WREG / WPR; u++)
+            wreg[u] = (lane * 4 + u * 4 * NT < dm) ? __ldg(reinterpret_cast<const float4 *>(w + lane * 4 + u * 4 * NT)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     const int pitch = (dm + 3) & ~3;
     float *xs = norm_smem + (size_t)warp * pitch;
@@ -105,34 +113,34 @@ __global__ void __launch_bounds__(128) norm_rows_kernel(float *__restrict__ out,
                      (!dl || ((reinterpret_cast<uintptr_t>(dl) & 15) == 0 && (reinterpret_cast<uintptr_t>(so) & 15) == 0));
     unsigned key = 0xFFFFFFFFu;
     if (vec) {
-        // eight 128-bit loads per lane in flight: a lone warp has no other warp to hide a load behind
-        for (int j0 = lane * 4; j0 < dm; j0 += 8 * 128) {
-            float4 v[8];
+        // several 128-bit loads per lane in flight: a lone warp has no other warp to hide a load behind
+        for (int j0 = lane * 4; j0 < dm; j0 += AHEAD * 4 * NT) {
+            float4 v[AHEAD];
 #pragma unroll
-            for (int u = 0; u < 8; u++)
-                v[u] = (j0 + u * 128 < dm) ? *reinterpret_cast<const float4 *>(x + j0 + u * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int u = 0; u < AHEAD; u++)
+                v[u] = (j0 + u * 4 * NT < dm) ? *reinterpret_cast<const float4 *>(x + j0 + u * 4 * NT) : make_float4(0.f, 0.f, 0.f, 0.f);
             if (dl) {
-                float4 d[8];
+                float4 d[AHEAD];
 #pragma unroll
-                for (int u = 0; u < 8; u++)
-                    d[u] = (j0 + u * 128 < dm) ? *reinterpret_cast<const float4 *>(dl + j0 + u * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int u = 0; u < AHEAD; u++)
+                    d[u] = (j0 + u * 4 * NT < dm) ? *reinterpret_cast<const float4 *>(dl + j0 + u * 4 * NT) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int u = 0; u < 8; u++) {
+                for (int u = 0; u < AHEAD; u++) {
                     v[u].x = __fadd_rn(ftz_bits(v[u].x), ftz_bits(d[u].x)); v[u].y = __fadd_rn(ftz_bits(v[u].y), ftz_bits(d[u].y));
                     v[u].z = __fadd_rn(ftz_bits(v[u].z), ftz_bits(d[u].z)); v[u].w = __fadd_rn(ftz_bits(v[u].w), ftz_bits(d[u].w));
                 }
             }
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                if (j0 + u * 128 >= dm) break;
+            for (int u = 0; u < AHEAD; u++) {
+                if (j0 + u * 4 * NT >= dm) break;
                 v[u].x = ftz_bits(v[u].x); v[u].y = ftz_bits(v[u].y); v[u].z = ftz_bits(v[u].z); v[u].w = ftz_bits(v[u].w);
                 key = min(min(key, admit_key(v[u].x)), min(admit_key(v[u].y), min(admit_key(v[u].z), admit_key(v[u].w))));
-                *reinterpret_cast<float4 *>(xs + j0 + u * 128) = v[u];
-                if (so) *reinterpret_cast<float4 *>(so + j0 + u * 128) = v[u];
+                *reinterpret_cast<float4 *>(xs + j0 + u * 4 * NT) = v[u];
+                if (so) *reinterpret_cast<float4 *>(so + j0 + u * 4 * NT) = v[u];
             }
         }
     } else {
-        for (int j = lane; j < dm; j += 32) {
+        for (int j = lane; j < dm; j += NT) {
             float v = ftz_bits(x[j]);
             if (dl) v = ftz_bits(__fadd_rn(v, ftz_bits(dl[j])));
             key = min(key, admit_key(v));
@@ -140,21 +148,21 @@ __global__ void __launch_bounds__(128) norm_rows_kernel(float *__restrict__ out,
             if (so) so[j] = v;
         }
     }
-    for (int j = dm + lane; j < pitch; j += 32) xs[j] = 0.f;
-    __syncwarp();
+    for (int j = dm + lane; j < pitch; j += NT) xs[j] = 0.f;
+    row_sync();
     if (kind == NORM_LAYER) {
         const float acc = row_chain(xs, dm, [](float v, float acc) { return add_flushed(acc, v); });
         const float mean = ftz_bits(p_divf(acc, (float)dm));
-        __syncwarp();
+        row_sync();
         key = 0xFFFFFFFFu;
-        for (int j = lane; j < dm; j += 32) {
+        for (int j = lane; j < dm; j += NT) {
             const float v = ftz_bits(__fsub_rn(xs[j], mean));
             key = min(key, admit_key(v));
             xs[j] = v;
         }
-        __syncwarp();
+        row_sync();
     }
-    const bool bare = __all_sync(0xFFFFFFFFu, key >= NORM_ADMIT_MIN);
+    const bool bare = row_all(key >= NORM_ADMIT_MIN);
     const float acc = bare ? row_chain(xs, dm, [](float v, float acc) { return step_bare(v, v, acc); })
                            : row_chain(xs, dm, [](float v, float acc) { return step_flush(v, v, acc); });
     const float var = ftz_bits(p_divf(acc, (float)dm));
@@ -181,29 +189,29 @@ __global__ void __launch_bounds__(128) norm_rows_kernel(float *__restrict__ out,
         const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
         if (w_early && !has_bias) { // the weights are already in registers
 #pragma unroll
-            for (int u = 0; u < NORM_WREG; u++) {
-                const int j = lane * 4 + u * 128;
+            for (int u = 0; u < NORM_WREG / WPR; u++) {
+                const int j = lane * 4 + u * 4 * NT;
                 if (j < dm) finish4(j, wreg[u], zero4);
             }
         } else {
-            for (int j0 = lane * 4; j0 < dm; j0 += 4 * 128) {
+            for (int j0 = lane * 4; j0 < dm; j0 += 4 * 4 * NT) {
                 float4 wv[4], bv[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    const bool in = j0 + u * 128 < dm;
-                    wv[u] = in ? *reinterpret_cast<const float4 *>(w + j0 + u * 128) : zero4;
-                    bv[u] = (in && has_bias) ? *reinterpret_cast<const float4 *>(bias + j0 + u * 128) : zero4;
+                    const bool in = j0 + u * 4 * NT < dm;
+                    wv[u] = in ? *reinterpret_cast<const float4 *>(w + j0 + u * 4 * NT) : zero4;
+                    bv[u] = (in && has_bias) ? *reinterpret_cast<const float4 *>(bias + j0 + u * 4 * NT) : zero4;
                 }
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    const int j = j0 + u * 128;
+                    const int j = j0 + u * 4 * NT;
                     if (j >= dm) break;
                     finish4(j, wv[u], bv[u]);
                 }
             }
         }
     } else {
-        for (int j = lane; j < dm; j += 32) out[row * dm + j] = finish(xs[j], w[j], (kind == NORM_LAYER && bias) ? bias[j] : 0.f);
+        for (int j = lane; j < dm; j += NT) out[row * dm + j] = finish(xs[j], w[j], (kind == NORM_LAYER && bias) ? bias[j] : 0.f);
     }
 }
 
@@ -475,31 +483,42 @@ __global__ void advance_position_kernel(int *pos_dev, int delta) { *pos_dev += d
 // Score seams S12 (scale) and the optional soft cap between it and the mask (transformer_oracle.mojo:2269-2281,
 // Gemma 2's attn_logit_softcapping): cap * tanh(score / cap), one portable division, one portable tanh and one
 // product, each flushed. `softcap` 0 (all bits) = none.
+// The cap is kept out of line: inlined, its tanh and division sat between the stores of every cell of an unrolled tile,
+// 64 skipped copies of it for a call without a cap.
+__device__ __noinline__ float score_cap(float sc, float softcap) {
+    const float cap = ftz_bits(softcap);
+    const float th = ftz_bits(p_tanhf(ftz_bits(p_divf(sc, cap))));
+    return ftz_bits(__fmul_rn(th, cap));
+}
 __device__ __forceinline__ float score_scale_cap(float dot, float scale, float softcap) {
-    float sc = ftz_bits(__fmul_rn(ftz_hw(dot), scale));
-    if (__float_as_uint(softcap) != 0u) {
-        const float cap = ftz_bits(softcap);
-        const float th = ftz_bits(p_tanhf(ftz_bits(p_divf(sc, cap))));
-        sc = ftz_bits(__fmul_rn(th, cap));
-    }
-    return sc;
+    const float sc = ftz_bits(__fmul_rn(ftz_hw(dot), scale));
+    return __float_as_uint(softcap) != 0u ? score_cap(sc, softcap) : sc;
+}
+
+__device__ __forceinline__ unsigned key_of4(float4 v) {
+    return min(min(admit_key(v.x), admit_key(v.y)), min(admit_key(v.z), admit_key(v.w)));
 }
 
 // ---- attention scores -------------------------------------------------------------------------
 // scores[b, h, qi, j] = ftz(ftz(ftz(q . k) * scale) + fill), the dot being one
 // gemm fp32.v1 leaf (k = head_dim <= 128: a single serial chain from +0.0).
-// A CTA owns a 64 x 64 tile of one (batch, head); a thread owns 4 x 4 cells.
-constexpr int ATT_T = 64, ATT_KC = 32;
-__global__ void __launch_bounds__(256) attn_scores_kernel(float *__restrict__ scores, const float *__restrict__ q,
-                                                          const float *__restrict__ kcache, int b, int l, int nh, int nkv, int hd,
-                                                          int cap, int key_lo, int s, int own0, int window,
-                                                          const int *__restrict__ pos_dev, float softcap) {
+// A CTA owns a 128 x 128 tile of one (batch, head), a thread 8 x 8 cells as pairs along the keys: four 128-bit reads and
+// eight doubled words for 32 fma.rn.f32x2, as in the large products. Windows of 16 steps are fetched 16 bytes a lane into
+// registers a window ahead and turned into k-major rows whose 8-word groups are permuted by the step's quad, so neither the
+// turned stores nor the 16-byte reads conflict; one barrier per window publishes it with its admission verdict.
+// 64 heads of 1024 tokens at head_dim 128: 332 us; 613 with 64 x 64 tiles of 4 x 4 scalar cells, turned with four-way
+// conflicts, stored word by word, the soft cap's tanh inlined in every cell and a masked tile's words tested one by one.
+constexpr int ATT_T = 128, ATT_KC = 16;
+__global__ void __launch_bounds__(256, 2) attn_scores_kernel(float *__restrict__ scores, const float *__restrict__ q,
+                                                             const float *__restrict__ kcache, int b, int l, int nh, int nkv, int hd,
+                                                             int cap, int key_lo, int s, int own0, int window,
+                                                             const int *__restrict__ pos_dev, float softcap) {
     attn_geometry(pos_dev, l, cap, window, key_lo, s, own0);
     if ((int)blockIdx.x * ATT_T >= s) return;
     // the attention scale, ftz(rsqrt(head_dim)) in the portable spelling: a pure function of head_dim
     const float scale = ftz_bits(p_rsqrtf((float)hd));
-    __shared__ __align__(16) float qs[ATT_KC][ATT_T + 4]; // pitch 68 words: rows stay 16-byte aligned
-    __shared__ __align__(16) float ks[ATT_KC][ATT_T + 4];
+    __shared__ __align__(16) float qs[2][ATT_KC][ATT_T];
+    __shared__ __align__(16) float ks[2][ATT_KC][ATT_T];
     const int bh = blockIdx.z, bb = bh / nh, h = bh % nh, kv = h / (nh / nkv);
     const int q0 = blockIdx.y * ATT_T, j0 = blockIdx.x * ATT_T;
     const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
@@ -507,6 +526,9 @@ __global__ void __launch_bounds__(256) attn_scores_kernel(float *__restrict__ sc
     const float *qbase = q + ((long long)bb * l) * qw + (long long)h * hd;
     const float *kbase = kcache + (((long long)bb * nkv + kv) * cap + key_lo) * hd;
     const float mfill = __uint_as_float(0xFF7FFFFFu);
+    const bool vec = (hd % 4 == 0) && (((reinterpret_cast<uintptr_t>(qbase) | reinterpret_cast<uintptr_t>(kbase)) & 15u) == 0);
+    float *sbase = scores + (long long)bh * l * s;
+    const bool vec_out = (s % 4 == 0) && ((reinterpret_cast<uintptr_t>(scores) & 15u) == 0);
     // A tile no query of which can see any of its keys: every cell is ftz(score + (-FLT_MAX)). When every
     // operand word of the tile is finite and below 2^40 in magnitude, |score| < 2^88 is under half an ulp of
     // FLT_MAX (2^103), so the sum IS -FLT_MAX and the dot products need not be formed.
@@ -515,103 +537,140 @@ __global__ void __launch_bounds__(256) attn_scores_kernel(float *__restrict__ sc
     const bool tile_masked = __float_as_uint(softcap) == 0u &&
                              (j0 > own0 + q_hi || (window > 0 && j0 + ATT_T - 1 < own0 + q0 - window + 1));
     if (tile_masked) {
-        bool small = true;
+        unsigned big = 0u; // the largest exponent among this thread's words; nothing waits for one load before the next
         const int warp = tid >> 5, lane = tid & 31;
-        const bool vec = (hd % 4 == 0) && (((reinterpret_cast<uintptr_t>(qbase) | reinterpret_cast<uintptr_t>(kbase)) & 15u) == 0);
+        auto exponent = [](float x) { return (__float_as_uint(x) >> 23) & 0xFFu; };
+#pragma unroll 4
         for (int r = warp; r < ATT_T; r += 8) { // a warp per row, lanes along the row: no division by head_dim
-            const float *qr = qbase + (long long)(q0 + r) * qw, *kr = kbase + (long long)(j0 + r) * hd;
             const bool qlive = q0 + r < l, klive = j0 + r < s;
+            const float *qr = qbase + (long long)(qlive ? q0 + r : q0) * qw, *kr = kbase + (long long)(klive ? j0 + r : j0) * hd; // (a row past the end: the first again)
             if (vec) {
                 for (int p = lane * 4; p < hd; p += 128) {
-                    if (qlive) {
-                        const float4 v = *reinterpret_cast<const float4 *>(qr + p);
-                        small = small && ((__float_as_uint(v.x) >> 23) & 0xFFu) < 167u && ((__float_as_uint(v.y) >> 23) & 0xFFu) < 167u &&
-                                ((__float_as_uint(v.z) >> 23) & 0xFFu) < 167u && ((__float_as_uint(v.w) >> 23) & 0xFFu) < 167u;
-                    }
-                    if (klive) {
-                        const float4 v = *reinterpret_cast<const float4 *>(kr + p);
-                        small = small && ((__float_as_uint(v.x) >> 23) & 0xFFu) < 167u && ((__float_as_uint(v.y) >> 23) & 0xFFu) < 167u &&
-                                ((__float_as_uint(v.z) >> 23) & 0xFFu) < 167u && ((__float_as_uint(v.w) >> 23) & 0xFFu) < 167u;
-                    }
+                    const float4 v = *reinterpret_cast<const float4 *>(qr + p), w = *reinterpret_cast<const float4 *>(kr + p);
+                    big = max(big, max(max(exponent(v.x), exponent(v.y)), max(exponent(v.z), exponent(v.w))));
+                    big = max(big, max(max(exponent(w.x), exponent(w.y)), max(exponent(w.z), exponent(w.w))));
                 }
             } else {
-                for (int p = lane; p < hd; p += 32) {
-                    if (qlive) small = small && ((__float_as_uint(qr[p]) >> 23) & 0xFFu) < 167u;
-                    if (klive) small = small && ((__float_as_uint(kr[p]) >> 23) & 0xFFu) < 167u;
-                }
+                for (int p = lane; p < hd; p += 32) big = max(big, max(exponent(qr[p]), exponent(kr[p])));
             }
         }
+        const bool small = big < 167u;
         if (__syncthreads_and(small)) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int qi = q0 + ty * 4 + i;
-                if (qi >= l) continue;
-#pragma unroll
-                for (int jj = 0; jj < 4; jj++) {
-                    const int j = j0 + tx * 4 + jj;
-                    if (j < s) scores[((long long)bh * l + qi) * s + j] = mfill;
-                }
+            for (int r = warp; r < ATT_T && q0 + r < l; r += 8) {
+                float *row = sbase + (long long)(q0 + r) * s + j0;
+                const int j = lane * 4;
+                if (vec_out && j0 + j + 3 < s) *reinterpret_cast<float4 *>(row + j) = make_float4(mfill, mfill, mfill, mfill);
+                else
+                    for (int e = 0; e < 4; e++)
+                        if (j0 + j + e < s) row[j + e] = mfill;
             }
             return;
         }
     }
-    float acc[4][4];
+    // a thread's two quads of each operand's window: rows u * 64 + tid / 4, steps (tid % 4) * 4 .. + 3
+    const int sr = tid >> 2, sq = tid & 3;
+    float4 rq[2], rk[2];
+    auto load4 = [&](const float *row, bool live, int p) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live && p < hd) {
+            if (vec) return *reinterpret_cast<const float4 *>(row + p);
+            v.x = row[p];
+            if (p + 1 < hd) v.y = row[p + 1];
+            if (p + 2 < hd) v.z = row[p + 2];
+            if (p + 3 < hd) v.w = row[p + 3];
+        }
+        return v;
+    };
+    auto fetch = [&](int p0) {
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+        for (int u = 0; u < 2; u++) {
+            const int r = u * 64 + sr;
+            rq[u] = load4(qbase + (long long)(q0 + r) * qw, q0 + r < l, p0 + sq * 4);
+            rk[u] = load4(kbase + (long long)(j0 + r) * hd, j0 + r < s, p0 + sq * 4);
+        }
+    };
+    unsigned key;
+    auto place = [&](int buf) {
+        key = 0xFFFFFFFFu;
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-    bool clean = true; // every chunk so far passed admission: the chains have only taken bare steps
+        for (int u = 0; u < 2; u++) {
+            const int c = (u * 64 + sr) ^ (sq * 8);
+            const float4 a = make_float4(ftz_bits(rq[u].x), ftz_bits(rq[u].y), ftz_bits(rq[u].z), ftz_bits(rq[u].w));
+            const float4 k4 = make_float4(ftz_bits(rk[u].x), ftz_bits(rk[u].y), ftz_bits(rk[u].z), ftz_bits(rk[u].w));
+            key = min(key, min(key_of4(a), key_of4(k4)));
+            qs[buf][sq * 4 + 0][c] = a.x; qs[buf][sq * 4 + 1][c] = a.y; qs[buf][sq * 4 + 2][c] = a.z; qs[buf][sq * 4 + 3][c] = a.w;
+            ks[buf][sq * 4 + 0][c] = k4.x; ks[buf][sq * 4 + 1][c] = k4.y; ks[buf][sq * 4 + 2][c] = k4.z; ks[buf][sq * 4 + 3][c] = k4.w;
+        }
+    };
+    unsigned long long acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
+    auto step = [&](int buf, int p, bool flush) {
+        const int sw = (p >> 2) * 8;
+        float a[8];
+        unsigned long long c2[4];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const float4 v = *reinterpret_cast<const float4 *>(&qs[buf][p][(r * 64 + ty * 4) ^ sw]);
+            a[4 * r] = v.x; a[4 * r + 1] = v.y; a[4 * r + 2] = v.z; a[4 * r + 3] = v.w;
+            const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(&ks[buf][p][(r * 64 + tx * 4) ^ sw]);
+            c2[2 * r] = w.x;
+            c2[2 * r + 1] = w.y;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const unsigned long long a2 = pack2(a[i], a[i]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const unsigned long long d = fma2_bare(a2, c2[j], acc[i][j]);
+                acc[i][j] = flush ? ftz2_hw(d) : d;
+            }
+        }
+    };
+    fetch(0);
+    place(0);
+    bool clean = __syncthreads_and(key >= ADMIT_MIN); // every window so far passed: the chains have only taken bare steps
+    int buf = 0;
     for (int p0 = 0; p0 < hd; p0 += ATT_KC) {
-        unsigned key = 0xFFFFFFFFu;
-        for (int idx = tid; idx < ATT_T * ATT_KC; idx += 256) {
-            const int r = idx / ATT_KC, p = idx % ATT_KC;
-            const bool pk = p0 + p < hd;
-            const float qv = (pk && q0 + r < l) ? ftz_bits(qbase[(long long)(q0 + r) * qw + p0 + p]) : 0.f;
-            const float kvv = (pk && j0 + r < s) ? ftz_bits(kbase[(long long)(j0 + r) * hd + p0 + p]) : 0.f;
-            key = min(key, min(admit_key(qv), admit_key(kvv)));
-            qs[p][r] = qv;
-            ks[p][r] = kvv;
-        }
-        clean = __syncthreads_and(key >= ADMIT_MIN) && clean;
+        const bool more = p0 + ATT_KC < hd;
         const int pn = min(ATT_KC, hd - p0);
-        if (clean) {
-#pragma unroll 8
-            for (int p = 0; p < pn; p++) {
-                const float4 a4 = *reinterpret_cast<const float4 *>(&qs[p][ty * 4]);
-                const float4 c4 = *reinterpret_cast<const float4 *>(&ks[p][tx * 4]);
-                const float a[4] = {a4.x, a4.y, a4.z, a4.w}, c[4] = {c4.x, c4.y, c4.z, c4.w};
+        if (more) fetch(p0 + ATT_KC);
+        if (clean && pn == ATT_KC) {
 #pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) acc[i][j] = step_bare(a[i], c[j], acc[i][j]);
-            }
+            for (int p = 0; p < ATT_KC; p++) step(buf, p, false);
         } else {
-            for (int p = 0; p < pn; p++) {
-                const float4 a4 = *reinterpret_cast<const float4 *>(&qs[p][ty * 4]);
-                const float4 c4 = *reinterpret_cast<const float4 *>(&ks[p][tx * 4]);
-                const float a[4] = {a4.x, a4.y, a4.z, a4.w}, c[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) acc[i][j] = step_flush(a[i], c[j], acc[i][j]);
-            }
+#pragma unroll 1
+            for (int p = 0; p < pn; p++) step(buf, p, true); // exact for any operands
         }
-        __syncthreads();
+        if (more) {
+            place(buf ^ 1);
+            clean = __syncthreads_and(key >= ADMIT_MIN) && clean;
+            buf ^= 1;
+        }
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int qi = q0 + ty * 4 + i;
+    for (int i = 0; i < 8; i++) {
+        const int qi = q0 + (i / 4) * 64 + ty * 4 + (i % 4);
         if (qi >= l) continue;
         int jlo = 0, jhi = own0 + qi;
         if (jhi > s - 1) jhi = s - 1;
         if (window > 0) { jlo = own0 + qi - window + 1; if (jlo < 0) jlo = 0; }
 #pragma unroll
-        for (int jj = 0; jj < 4; jj++) {
-            const int j = j0 + tx * 4 + jj;
-            if (j >= s) continue;
-            const float sc = score_scale_cap(acc[i][jj], scale, softcap);
-            const float fill = (j < jlo || j > jhi) ? mfill : 0.0f;
-            scores[((long long)bh * l + qi) * s + j] = ftz_bits(__fadd_rn(sc, fill));
+        for (int r = 0; r < 2; r++) {
+            const int j = j0 + r * 64 + tx * 4;
+            float v[4];
+            unpack2(acc[i][2 * r], v[0], v[1]);
+            unpack2(acc[i][2 * r + 1], v[2], v[3]);
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                v[e] = ftz_bits(__fadd_rn(score_scale_cap(v[e], scale, softcap), (j + e < jlo || j + e > jhi) ? mfill : 0.0f));
+            float *dst = sbase + (long long)qi * s + j;
+            if (vec_out && j + 3 < s) *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+            else
+                for (int e = 0; e < 4; e++)
+                    if (j + e < s) dst[e] = v[e];
         }
     }
 }
@@ -638,9 +697,6 @@ __device__ __forceinline__ void cp_async_floats(float *dst, const float *src, in
         for (int c = t * 2; c < count; c += nthreads * 2) cp_async8(dst + c, src + c);
     }
 }
-__device__ __forceinline__ unsigned key_of4(float4 v) {
-    return min(min(admit_key(v.x), admit_key(v.y)), min(admit_key(v.z), admit_key(v.w)));
-}
 
 // The same scores for a handful of query rows (a decode step): one lane per key, one
 // serial chain per (query, key) over head_dim. A warp copies the cache rows of its 32
@@ -651,9 +707,11 @@ __device__ __forceinline__ unsigned key_of4(float4 v) {
 // the bare fma while folding the admission key of what it reads; a lane whose row (or
 // the query) fails the product's admission test walks its chain again with the
 // flushed step, which is the contract's spelling for any operands.
+// The rows' pitch is head_dim + 4: at 64 a CTA takes 36 KB and six share an SM (96 heads of 512 keys: one wave, where the
+// pitch of 132 that head_dim 128 needs left 480 CTAs on 444 places).
 constexpr int ATT_SMALL_Q = 8, ATT_KT_PITCH = K_LEAF_MIN + 4;
 template <int LQ>
-constexpr int attn_scores_small_smem() { return (LQ * K_LEAF_MIN + 4 * 32 * ATT_KT_PITCH) * (int)sizeof(float); }
+constexpr int attn_scores_small_smem(int hd) { return (LQ * K_LEAF_MIN + 4 * 32 * ((hd + 7) / 4 * 4)) * (int)sizeof(float); }
 template <int LQ>
 __global__ void __launch_bounds__(128) attn_scores_small_kernel(float *__restrict__ scores, const float *__restrict__ q,
                                                                 const float *__restrict__ kcache, int b, int l, int nh, int nkv,
@@ -665,7 +723,8 @@ __global__ void __launch_bounds__(128) attn_scores_small_kernel(float *__restric
     float (*qs)[K_LEAF_MIN] = reinterpret_cast<float (*)[K_LEAF_MIN]>(att_smem);
     const int bh = blockIdx.y, bb = bh / nh, h = bh % nh, kv = h / (nh / nkv);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float (*kt)[ATT_KT_PITCH] = reinterpret_cast<float (*)[ATT_KT_PITCH]>(att_smem + LQ * K_LEAF_MIN) + warp * 32;
+    const int pitch = (hd + 7) / 4 * 4;
+    float *kt = att_smem + LQ * K_LEAF_MIN + warp * 32 * pitch;
     const int j0 = blockIdx.x * 128 + warp * 32;
     const bool vec16 = (hd % 4) == 0;
     const float *kbase = kcache + (((long long)bb * nkv + kv) * cap + key_lo) * hd;
@@ -673,20 +732,20 @@ __global__ void __launch_bounds__(128) attn_scores_small_kernel(float *__restric
     if (vec16) {
         // one instruction per cache row: lane t moves the 16 bytes at float 4t of the row
         const float *src = kbase + (long long)j0 * hd + lane * 4;
-        float *dst = &kt[0][lane * 4];
+        float *dst = kt + lane * 4;
         if (lane * 4 < hd) {
             if (rows == 32) {
 #pragma unroll
-                for (int r = 0; r < 32; r++) cp_async16(dst + r * ATT_KT_PITCH, src + (long long)r * hd);
+                for (int r = 0; r < 32; r++) cp_async16(dst + r * pitch, src + (long long)r * hd);
             } else {
-                for (int r = 0; r < rows; r++) cp_async16(dst + r * ATT_KT_PITCH, src + (long long)r * hd);
+                for (int r = 0; r < rows; r++) cp_async16(dst + r * pitch, src + (long long)r * hd);
             }
         }
     } else {
-        for (int r = 0; r < rows; r++) cp_async_floats(&kt[r][0], kbase + (long long)(j0 + r) * hd, hd, false, lane, 32);
+        for (int r = 0; r < rows; r++) cp_async_floats(kt + r * pitch, kbase + (long long)(j0 + r) * hd, hd, false, lane, 32);
     }
     for (int r = max(rows, 0); r < 32; r++)
-        for (int c = lane; c < hd; c += 32) kt[r][c] = 0.f;
+        for (int c = lane; c < hd; c += 32) kt[r * pitch + c] = 0.f;
     cp_async_commit();
     __shared__ float scale_s;
     if (threadIdx.x == 0) scale_s = ftz_bits(p_rsqrtf((float)hd)); // a pure function of head_dim: one thread spells it
@@ -702,7 +761,7 @@ __global__ void __launch_bounds__(128) attn_scores_small_kernel(float *__restric
     const float scale = scale_s;
     cp_async_wait<0>();
     __syncwarp();
-    const float *krow = &kt[lane][0];
+    const float *krow = kt + lane * pitch;
     float acc[LQ];
     bool exact = false;
     if (q_ok && vec16) {
@@ -749,7 +808,7 @@ __global__ void __launch_bounds__(128) attn_scores_small_kernel(float *__restric
 
 // ---- softmax and value sum ----------------------------------------------------------------------
 // A CTA owns 32 consecutive query rows of one (batch, head): eight warps of four rows.
-// The masked scores are overwritten in place by exp(s - max) and then by the weights.
+// The masked scores are overwritten in place by exp(s - max); the weights go no further than shared memory.
 // Every chain of the seam stays serial per row; the four rows of a warp are four
 // independent chains walked together, so a value word read from the staged tile serves
 // four rows and a 128-bit broadcast read delivers the four rows' weights of one key.
@@ -899,10 +958,7 @@ __global__ void __launch_bounds__(32 * CTX_WARPS) attn_context_kernel(float *__r
 #pragma unroll
         for (int r = 0; r < CTX_RPW; r++) {
             wgt[r] = 0.f;
-            if (j >= jlo[r] && j <= jhi[r]) {
-                wgt[r] = ftz_bits(p_divf(ftz_bits(row[r][j]), den[r]));
-                row[r][j] = wgt[r];
-            }
+            if (j >= jlo[r] && j <= jhi[r]) wgt[r] = ftz_bits(p_divf(ftz_bits(row[r][j]), den[r]));
             wkey = min(wkey, admit_key(wgt[r]));
             full = full && jlo[r] <= j0 && jhi[r] >= j0 + CTX_KT - 1;
             heads = heads && (jlo[r] <= j0 || jhi[r] < j0);
@@ -991,11 +1047,12 @@ __global__ void __launch_bounds__(32 * CTX_WARPS) attn_context_kernel(float *__r
 // copy needs; those caches go through per-thread cp.async instead.
 // Every wait on an mbarrier is bounded; one that runs out sets the status word read by
 // b200i_decode_status (value 3) and the kernel carries on to its end.
+// 96 rows of 514 keys at head_dim 64 are bound by the instructions of one warp per scheduler: 23 us; see the chain below.
 // Three stages and a 4K-key weight row fit four CTAs on an SM. A call with few CTAs (a head-sharded rank, a small
 // batch) gets up to CTX_ST_MAX stages instead: what bounds it is the bytes one CTA keeps in flight.
 constexpr int CTX_NB = 32, CTX_ST = 3, CTX_ST_MAX = 12;
 inline size_t attn_context_row_smem(int s_grid, int hd, int stages = CTX_ST) {
-    return ((size_t)((s_grid + 3) & ~3) + (size_t)stages * CTX_NB * hd) * sizeof(float);
+    return ((size_t)((s_grid + 3) & ~3) + (size_t)stages * CTX_NB * hd) * sizeof(float) + (size_t)(s_grid + CTX_NB) / CTX_NB;
 }
 __global__ void __launch_bounds__(128) attn_context_row_kernel(float *__restrict__ ctx, float *__restrict__ scores,
                                                                 const float *__restrict__ vcache, int b, int l, int nh, int nkv,
@@ -1006,8 +1063,8 @@ __global__ void __launch_bounds__(128) attn_context_row_kernel(float *__restrict
     float *wrow = ctx_smem;                        // [s] weights of this row
     float *ring = ctx_smem + ((s_grid + 3) & ~3);  // [stages][CTX_NB * hd]
     __shared__ unsigned red[4];
-    __shared__ float den_s;
     __shared__ __align__(8) unsigned long long full[CTX_ST_MAX];
+    unsigned char *wok = reinterpret_cast<unsigned char *>(ring + (size_t)stages * CTX_NB * hd); // per tile of 32 keys: its weights are admitted
     const int r = blockIdx.x; // (bh, qi)
     const int bh = r / l, qi = r % l, bb = bh / nh, h = bh % nh, kv = h / (nh / nkv);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1040,77 +1097,99 @@ __global__ void __launch_bounds__(128) attn_context_row_kernel(float *__restrict
             cp_async_commit();
         }
     };
-    for (int k = 0; k < stages - 1; k++) issue(k);
+    for (int k = 0; k < stages; k++) issue(k);
+    // wrow[i] belongs to key jlo + i, so a tile of 32 keys is one warp's 32 words and starts on a 16-byte boundary
+    const int keys = jhi - jlo + 1;
     unsigned best = 0u;
-    for (int j = tid; j < s; j += 128) best = max(best, order_key(ftz_bits(row[j])));
+    for (int j0 = tid; j0 < s; j0 += 4 * 128) { // S14 over the whole row, four reads in flight; the visible scores stay here
+        float x[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) x[u] = j0 + u * 128 < s ? ftz_bits(row[j0 + u * 128]) : 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int j = j0 + u * 128;
+            if (j < s) best = max(best, order_key(x[u]));
+            if (j >= jlo && j <= jhi) wrow[j - jlo] = x[u];
+        }
+    }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, off));
     if (lane == 0) red[warp] = best;
     __syncthreads();
     best = max(max(red[0], red[1]), max(red[2], red[3]));
     const float fm = ftz_bits(order_unkey(best));
-    for (int j = jlo + tid; j <= jhi; j += 128) wrow[j] = ftz_bits(p_expf(ftz_bits(__fsub_rn(ftz_bits(row[j]), fm))));
+    for (int i = tid; i < keys; i += 128) wrow[i] = ftz_bits(p_expf(ftz_bits(__fsub_rn(wrow[i], fm))));
     __syncthreads();
-    if (warp == 0) { // S17: serial ascending, every value already flushed
-        float den = 0.f;
-        for (int j0 = jlo; j0 <= jhi; j0 += 32) {
-            const float e = (j0 + lane <= jhi) ? wrow[j0 + lane] : 0.f;
-            if (j0 + 31 <= jhi) {
-#pragma unroll
-                for (int t = 0; t < 32; t++) den = add_flushed(den, __shfl_sync(0xFFFFFFFFu, e, t));
-            } else {
-                for (int t = 0; t < jhi - j0 + 1; t++) den = add_flushed(den, __shfl_sync(0xFFFFFFFFu, e, t));
-            }
+    // S17: serial ascending, every value already flushed; every warp walks it, so none waits for another to hand it over
+    const float den = row_chain(wrow, keys, [](float v, float acc) { return add_flushed(acc, v); });
+    __syncthreads(); // all have read the exponentials
+    for (int i0 = warp * 32; i0 < keys; i0 += 128) {
+        const int i = i0 + lane;
+        float wgt = 0.f;
+        if (i < keys) {
+            wgt = ftz_bits(p_divf(wrow[i], den));
+            wrow[i] = wgt;
         }
-        if (lane == 0) den_s = den;
+        const bool ok = __all_sync(0xFFFFFFFFu, admit_key(wgt) >= ADMIT_MIN);
+        if (lane == 0) wok[i0 / CTX_NB] = ok ? 1 : 0;
     }
     __syncthreads();
-    const float den = den_s;
-    for (int j = jlo + tid; j <= jhi; j += 128) {
-        const float wgt = ftz_bits(p_divf(wrow[j], den));
-        wrow[j] = wgt;
-        row[j] = wgt;
-    }
+    // Values: the 32 words of a tile go to registers while the chain of the tile before runs, so a chain step costs its own
+    // latency. When all weights and values of a tile pass the product's admission test and every earlier step of the chain
+    // was admitted too, the bare fma is the contract's step (no result can be subnormal), else the flushed step. The values'
+    // keys are taken 16 bytes at a time by all threads (a tile is hd * 32 words, a chain reads one in hd of them), and the
+    // barrier that frees the tile's slot carries the verdict.
     float acc = 0.f;
-    bool clean = true; // every step of this thread's chain so far was an admitted bare fma
+    bool clean = true, admitted = false;
+    const int d = tid < hd ? tid : 0;
+    float cur[CTX_NB];
+    auto walk = [&](int k, const float (&v)[CTX_NB]) { // tile k, whole
+        const float *w = wrow + k * CTX_NB;
+        clean = clean && admitted;
+        if (clean) {
+#pragma unroll
+            for (int u = 0; u < CTX_NB; u += 4) {
+                const float4 w4 = *reinterpret_cast<const float4 *>(w + u);
+                acc = step_bare(w4.x, v[u], acc);
+                acc = step_bare(w4.y, v[u + 1], acc);
+                acc = step_bare(w4.z, v[u + 2], acc);
+                acc = step_bare(w4.w, v[u + 3], acc);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < CTX_NB; u++) acc = step_flush(w[u], ftz_bits(v[u]), acc);
+        }
+    };
+    int slot = 0;
+    unsigned parity = 0;
+#pragma unroll 2
     for (int k = 0; k < nstages; k++) {
-        issue(k + stages - 1); // refills the slot the previous turn finished with
         if (bulk) {
-            if (!mbar_wait(&full[k % stages], (unsigned)(k / stages) & 1u) && lane == 0) atomicExch(&g_decode_status, 3);
+            if (!mbar_wait(&full[slot], parity) && lane == 0) atomicExch(&g_decode_status, 3);
         } else {
             cp_async_wait<CTX_ST - 1>(); // this thread's copies of stage k have landed
+            __syncthreads();             // and everyone's
         }
-        __syncthreads(); // everyone's copies are visible (the first turn also orders the weights above)
-        if (tid < hd) {
-            const float *vs = ring + (size_t)(k % stages) * CTX_NB * hd + tid;
-            const int first = jlo + k * CTX_NB;
-            if (first + CTX_NB - 1 <= jhi) {
-                // A thread's chain reads its own feature of the 32 values and the 32 weights: when all of them pass
-                // the product's admission test and every earlier step of the chain was admitted too, the bare fma is
-                // the contract's step (no result can be subnormal). The walk runs bare while folding the key and is
-                // redone with the flushed step only when the key fails.
-                const float before = acc;
-                unsigned key = 0xFFFFFFFFu;
-                if (clean) {
+        const float *tile = ring + (size_t)slot * CTX_NB * hd, *vs = tile + d;
+        const int count = min(CTX_NB, keys - k * CTX_NB);
+        float next[CTX_NB];
+        unsigned key = wok[k] ? 0xFFFFFFFFu : 0u;
+        if (count == CTX_NB) {
 #pragma unroll
-                    for (int u = 0; u < CTX_NB; u++) {
-                        const float wj = wrow[first + u], vj = vs[u * hd];
-                        key = min(key, min(admit_key(wj), admit_key(vj)));
-                        acc = step_bare(wj, vj, acc);
-                    }
-                }
-                if (!clean || key < ADMIT_MIN) {
-                    clean = false;
-                    acc = before;
-#pragma unroll
-                    for (int u = 0; u < CTX_NB; u++) acc = step_flush(wrow[first + u], ftz_bits(vs[u * hd]), acc);
-                }
-            } else {
-                clean = false;
-                for (int u = 0; first + u <= jhi; u++) acc = step_flush(wrow[first + u], ftz_bits(vs[u * hd]), acc);
-            }
+            for (int u = 0; u < CTX_NB; u++) next[u] = vs[u * hd];
+            for (int i = tid * 4; i < CTX_NB * hd; i += 4 * 128) key = min(key, key_of4(*reinterpret_cast<const float4 *>(tile + i)));
         }
-        __syncthreads(); // the slot is free for the copy the next turn issues
+        if (k > 0) walk(k - 1, cur);
+        admitted = __syncthreads_and(key >= ADMIT_MIN); // every thread holds its words of the tile: the slot is free
+        if (count < CTX_NB) { // the last tile, ragged
+            for (int u = 0; u < count; u++) acc = step_flush(wrow[k * CTX_NB + u], ftz_bits(vs[u * hd]), acc);
+        } else {
+#pragma unroll
+            for (int u = 0; u < CTX_NB; u++) cur[u] = next[u];
+            if (k == nstages - 1) walk(k, cur);
+        }
+        if (k + stages < nstages || !bulk) issue(k + stages);
+        if (++slot == stages) { slot = 0; parity ^= 1u; }
     }
     if (tid < hd) ctx[((long long)bb * l + qi) * ((long long)nh * hd) + (long long)h * hd + tid] = acc;
 }

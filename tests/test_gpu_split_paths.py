@@ -32,61 +32,6 @@ def test_tall_products(m, n, k):
         assert _same(torch_ops.product(pad[1:].view(k, m), db, op=linalg.OP_TN, plan=torch_ops.PLAN_TALL), want)
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 4), (9, 1024), (8, 1028), (5, 2052), (3, 4096), (2, 8192), (3, 8196), (7, 7), (4, 1001)])
-def test_quantised_rows(rows, cols):
-    rng = np.random.default_rng(cols)
-    x = (rng.standard_normal((rows, cols)) * np.exp2(rng.integers(-140, 120, (rows, 1)))).astype(np.float32)
-    x[0, :3] = [np.nan, 1e-41, -np.inf][:3]
-    x[rows - 1] = 0.0
-    q, e = torch_ops.quantize_int8(torch.from_numpy(x).cuda())
-    qo, eo = oracle.quantize_int8(x)
-    assert _same(q, qo) and _same(e, eo)
-
-
-def test_gated_activation_layouts_agree():
-    """Four outputs a thread on aligned rows against one output a thread on the same values off the 16-byte grid."""
-    import ctypes
-    rng = np.random.default_rng(5)
-    for kind in (0, 4, 5):
-        gu = torch.from_numpy((rng.standard_normal((5, 2 * 72)) * 4).astype(np.float32)).cuda()
-        gu[0, :4] = torch.tensor([float("inf"), float("nan"), 1e-41, -1e-40], device="cuda")
-        off = torch.empty(gu.numel() + 1, device="cuda")
-        off[1:] = gu.reshape(-1)
-        outs = []
-        for src in (gu.data_ptr(), off.data_ptr() + 4):
-            out = torch.empty((5, 72), device="cuda")
-            _native.call("b200i_act_mul", 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(src), None,
-                         5, 72, 144, kind, 1)
-            outs.append(out.view(torch.int32))
-        assert torch.equal(*outs)
-
-
-@pytest.mark.parametrize("m,n,k", [(2304, 2304, 144), (2500, 2060, 272), (130, 38000, 128), (4000, 2600, 16)])
-def test_int8_products_on_sm_pairs(m, n, k):
-    """Whole tiles, the halved last round, rows and columns past the edge, k below and across a stage."""
-    rng = np.random.default_rng(m)
-    qa, qb = rng.integers(-127, 128, (m, k)).astype(np.int8), rng.integers(-127, 128, (n, k)).astype(np.int8)
-    ea, eb = rng.integers(-60, 30, m).astype(np.int32), rng.integers(-60, 30, n).astype(np.int32)
-    got = torch_ops.matmul_int8(*(torch.from_numpy(t).cuda() for t in (qa, ea, qb, eb))).cpu().numpy()
-    rows = np.unique(np.r_[0, 127, 128, 255, 256, m - 1, rng.integers(0, m, 24)] % m)
-    want = oracle.nan_canon(oracle.gemm_int8(np.ascontiguousarray(qa[rows]), ea[rows], qb, eb))
-    assert got[rows].tobytes() == want.tobytes()
-    assert _native.lib().b200i_decode_status(-1) == 0
-
-
-@pytest.mark.parametrize("m,n,k,opname", [(96, 2304, 1500, "NT"), (1100, 1000, 1030, "NN"), (40, 1500, 3000, "NN"), (2000, 70, 900, "TN")])
-def test_host_arrays_through_the_copy_threads(m, n, k, opname):
-    """Megabytes of pageable arrays: both ways of cutting the product, and the plain path."""
-    op = {"NN": linalg.OP_NN, "NT": linalg.OP_NT, "TN": linalg.OP_TN}[opname]
-    rng = np.random.default_rng(k)
-    a = rng.standard_normal((k, m) if opname == "TN" else (m, k)).astype(np.float32)
-    b = rng.standard_normal((n, k) if opname == "NT" else (k, n)).astype(np.float32)
-    want = torch_ops.product(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), op=op).cpu().numpy()
-    for _ in range(2):
-        got = linalg.matmul(a, b, transpose_a=opname == "TN", transpose_b=opname == "NT")
-        assert got.tobytes() == want.tobytes()
-
-
 def _weight(rng, n, k, kind):
     if kind == linalg.W_F32:
         w = rng.standard_normal((n, k)).astype(np.float32)
@@ -126,18 +71,6 @@ def test_rows_plan(m, kind):
         assert _same(torch_ops.product(da, dw, ds, kind, linalg.OP_NT), want), (n, k)
 
 
-@pytest.mark.parametrize("act", [torch_ops.ACT_GELU_ERF, torch_ops.ACT_SILU, torch_ops.ACT_PAIR_SWIGLU, torch_ops.ACT_PAIR_GEGLU_TANH])
-@pytest.mark.parametrize("n,k", [(1000, 768), (48, 5136)])
-def test_rows_plan_store_epilogues(n, k, act):
-    rng = np.random.default_rng(n + act)
-    a, w = torch.from_numpy(rng.standard_normal((7, k)).astype(np.float32)).cuda(), torch.from_numpy(rng.standard_normal((n, k)).astype(np.float32)).cuda()
-    bias = torch.from_numpy(rng.standard_normal(n).astype(np.float32)).cuda()
-    gl = 32 if k > 4096 else 0
-    want = torch_ops.product(a, w, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_SKINNY, bias=bias, act=act)
-    got = torch_ops.product(a, w, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_ROWS, group_leaves=gl, bias=bias, act=act)
-    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
-
-
 @pytest.mark.parametrize("m", [9, 16, 17, 32])
 @pytest.mark.parametrize("n,k", [(24, 128), (770, 784), (255, 16), (1001, 144), (300, 5136)])
 def test_band_plan(m, n, k):
@@ -150,3 +83,70 @@ def test_band_plan(m, n, k):
     for gl in (0, 1, 4):
         if gl <= oracle.leaf_count(k):
             assert _same(torch_ops.product(da, dw, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_BAND, group_leaves=gl), want), gl
+
+
+@pytest.mark.parametrize("act", [torch_ops.ACT_GELU_ERF, torch_ops.ACT_SILU, torch_ops.ACT_PAIR_SWIGLU, torch_ops.ACT_PAIR_GEGLU_TANH])
+@pytest.mark.parametrize("n,k", [(1000, 768), (48, 5136)])
+def test_rows_plan_store_epilogues(n, k, act):
+    rng = np.random.default_rng(n + act)
+    a, w = torch.from_numpy(rng.standard_normal((7, k)).astype(np.float32)).cuda(), torch.from_numpy(rng.standard_normal((n, k)).astype(np.float32)).cuda()
+    bias = torch.from_numpy(rng.standard_normal(n).astype(np.float32)).cuda()
+    gl = 32 if k > 4096 else 0
+    want = torch_ops.product(a, w, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_SKINNY, bias=bias, act=act)
+    got = torch_ops.product(a, w, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_ROWS, group_leaves=gl, bias=bias, act=act)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 4), (9, 1024), (8, 1028), (5, 2052), (3, 4096), (2, 8192), (3, 8196), (7, 7), (4, 1001)])
+def test_quantised_rows(rows, cols):
+    rng = np.random.default_rng(cols)
+    x = (rng.standard_normal((rows, cols)) * np.exp2(rng.integers(-140, 120, (rows, 1)))).astype(np.float32)
+    x[0, :3] = [np.nan, 1e-41, -np.inf][:3]
+    x[rows - 1] = 0.0
+    q, e = torch_ops.quantize_int8(torch.from_numpy(x).cuda())
+    qo, eo = oracle.quantize_int8(x)
+    assert _same(q, qo) and _same(e, eo)
+
+
+@pytest.mark.parametrize("m,n,k", [(2304, 2304, 144), (2500, 2060, 272), (130, 38000, 128), (4000, 2600, 16)])
+def test_int8_products_on_sm_pairs(m, n, k):
+    """Whole tiles, the halved last round, rows and columns past the edge, k below and across a stage."""
+    rng = np.random.default_rng(m)
+    qa, qb = rng.integers(-127, 128, (m, k)).astype(np.int8), rng.integers(-127, 128, (n, k)).astype(np.int8)
+    ea, eb = rng.integers(-60, 30, m).astype(np.int32), rng.integers(-60, 30, n).astype(np.int32)
+    got = torch_ops.matmul_int8(*(torch.from_numpy(t).cuda() for t in (qa, ea, qb, eb))).cpu().numpy()
+    rows = np.unique(np.r_[0, 127, 128, 255, 256, m - 1, rng.integers(0, m, 24)] % m)
+    want = oracle.nan_canon(oracle.gemm_int8(np.ascontiguousarray(qa[rows]), ea[rows], qb, eb))
+    assert got[rows].tobytes() == want.tobytes()
+    assert _native.lib().b200i_decode_status(-1) == 0
+
+
+@pytest.mark.parametrize("m,n,k,opname", [(96, 2304, 1500, "NT"), (1100, 1000, 1030, "NN"), (40, 1500, 3000, "NN"), (2000, 70, 900, "TN")])
+def test_host_arrays_through_the_copy_threads(m, n, k, opname):
+    """Megabytes of pageable arrays: both ways of cutting the product, and the plain path."""
+    op = {"NN": linalg.OP_NN, "NT": linalg.OP_NT, "TN": linalg.OP_TN}[opname]
+    rng = np.random.default_rng(k)
+    a = rng.standard_normal((k, m) if opname == "TN" else (m, k)).astype(np.float32)
+    b = rng.standard_normal((n, k) if opname == "NT" else (k, n)).astype(np.float32)
+    want = torch_ops.product(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), op=op).cpu().numpy()
+    for _ in range(2):
+        got = linalg.matmul(a, b, transpose_a=opname == "TN", transpose_b=opname == "NT")
+        assert got.tobytes() == want.tobytes()
+
+
+def test_gated_activation_layouts_agree():
+    """Four outputs a thread on aligned rows against one output a thread on the same values off the 16-byte grid."""
+    import ctypes
+    rng = np.random.default_rng(5)
+    for kind in (0, 4, 5):
+        gu = torch.from_numpy((rng.standard_normal((5, 2 * 72)) * 4).astype(np.float32)).cuda()
+        gu[0, :4] = torch.tensor([float("inf"), float("nan"), 1e-41, -1e-40], device="cuda")
+        off = torch.empty(gu.numel() + 1, device="cuda")
+        off[1:] = gu.reshape(-1)
+        outs = []
+        for src in (gu.data_ptr(), off.data_ptr() + 4):
+            out = torch.empty((5, 72), device="cuda")
+            _native.call("b200i_act_mul", 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(src), None,
+                         5, 72, 144, kind, 1)
+            outs.append(out.view(torch.int32))
+        assert torch.equal(*outs)
