@@ -1250,7 +1250,8 @@ static int64_t attention_launch(int dev, cudaStream_t st, float *ctx, const floa
     if (l <= ATT_SMALL_Q && (size_t)s_grid * sizeof(float) <= 40 * 1024) {
         static std::atomic<bool> configured[64];
         if (dev >= 0 && dev < 64 && !configured[dev]) {
-            CUDA_TRY(cudaFuncSetAttribute(attn_context_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+            CUDA_TRY(cudaFuncSetAttribute(attn_context_row_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+            CUDA_TRY(cudaFuncSetAttribute(attn_context_row_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
             configured[dev] = true;
         }
         // enough CTAs per SM for one wave (four at most); the shared memory that leaves a CTA becomes ring stages
@@ -1260,9 +1261,13 @@ static int64_t attention_launch(int dev, cudaStream_t st, float *ctx, const floa
         long long stages = ((226ll * 1024 / per_sm - 1664) / 4 - ((s_grid + 3) & ~3)) / (CTX_NB * head_dim);
         if (stages > CTX_ST_MAX) stages = CTX_ST_MAX;
         if (stages < CTX_ST) stages = CTX_ST;
-        attn_context_row_kernel<<<(unsigned)rows, 128, attn_context_row_smem(s_grid, (int)head_dim, (int)stages), st>>>(
-            ctx, scores, vcache, (int)b, (int)l, (int)n_heads, (int)n_kv, (int)head_dim, (int)cap, key_lo, s, own0, (int)window, position,
-            s_grid, (int)stages);
+        const size_t row_smem = attn_context_row_smem(s_grid, (int)head_dim, (int)stages);
+        if (rows <= 2ll * sm_count(dev))
+            attn_context_row_kernel<256><<<(unsigned)rows, 256, row_smem, st>>>(ctx, scores, vcache, (int)b, (int)l, (int)n_heads, (int)n_kv, (int)head_dim, (int)cap,
+                                                                                key_lo, s, own0, (int)window, position, s_grid, (int)stages);
+        else
+            attn_context_row_kernel<128><<<(unsigned)rows, 128, row_smem, st>>>(ctx, scores, vcache, (int)b, (int)l, (int)n_heads, (int)n_kv, (int)head_dim, (int)cap,
+                                                                                key_lo, s, own0, (int)window, position, s_grid, (int)stages);
     } else {
         dim3 g2((unsigned)((l + CTX_ROWS - 1) / CTX_ROWS), (unsigned)(b * n_heads));
 #define CONTEXT_ROWS(DPL)                                                                                                     \

@@ -1047,14 +1047,16 @@ __global__ void __launch_bounds__(32 * CTX_WARPS) attn_context_kernel(float *__r
 // copy needs; those caches go through per-thread cp.async instead.
 // Every wait on an mbarrier is bounded; one that runs out sets the status word read by
 // b200i_decode_status (value 3) and the kernel carries on to its end.
-// 96 rows of 514 keys at head_dim 64 are bound by the instructions of one warp per scheduler: 23 us; see the chain below.
 // Three stages and a 4K-key weight row fit four CTAs on an SM. A call with few CTAs (a head-sharded rank, a small
 // batch) gets up to CTX_ST_MAX stages instead: what bounds it is the bytes one CTA keeps in flight.
 constexpr int CTX_NB = 32, CTX_ST = 3, CTX_ST_MAX = 12;
+// Threads: up to four warps of chains; with 256, where there are too few rows to fill the device, four or more others share
+// what is not a chain.
 inline size_t attn_context_row_smem(int s_grid, int hd, int stages = CTX_ST) {
     return ((size_t)((s_grid + 3) & ~3) + (size_t)stages * CTX_NB * hd) * sizeof(float) + (size_t)(s_grid + CTX_NB) / CTX_NB;
 }
-__global__ void __launch_bounds__(128) attn_context_row_kernel(float *__restrict__ ctx, float *__restrict__ scores,
+template <int CTX_T>
+__global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(float *__restrict__ ctx, float *__restrict__ scores,
                                                                 const float *__restrict__ vcache, int b, int l, int nh, int nkv,
                                                                 int hd, int cap, int key_lo, int s, int own0, int window,
                                                                 const int *__restrict__ pos_dev, int s_grid, int stages) {
@@ -1062,7 +1064,7 @@ __global__ void __launch_bounds__(128) attn_context_row_kernel(float *__restrict
     extern __shared__ __align__(16) float ctx_smem[];
     float *wrow = ctx_smem;                        // [s] weights of this row
     float *ring = ctx_smem + ((s_grid + 3) & ~3);  // [stages][CTX_NB * hd]
-    __shared__ unsigned red[4];
+    __shared__ unsigned red[CTX_T / 32];
     __shared__ __align__(8) unsigned long long full[CTX_ST_MAX];
     unsigned char *wok = reinterpret_cast<unsigned char *>(ring + (size_t)stages * CTX_NB * hd); // per tile of 32 keys: its weights are admitted
     const int r = blockIdx.x; // (bh, qi)
@@ -1092,7 +1094,7 @@ __global__ void __launch_bounds__(128) attn_context_row_kernel(float *__restrict
         } else { // always one commit, so that the groups count stages
             if (k < nstages) {
                 const int first = jlo + k * CTX_NB, keys = min(CTX_NB, jhi - first + 1);
-                cp_async_floats(ring + (size_t)(k % stages) * CTX_NB * hd, vbase + (long long)first * hd, keys * hd, false, tid, 128);
+                cp_async_floats(ring + (size_t)(k % stages) * CTX_NB * hd, vbase + (long long)first * hd, keys * hd, false, tid, CTX_T);
             }
             cp_async_commit();
         }
@@ -1101,13 +1103,13 @@ __global__ void __launch_bounds__(128) attn_context_row_kernel(float *__restrict
     // wrow[i] belongs to key jlo + i, so a tile of 32 keys is one warp's 32 words and starts on a 16-byte boundary
     const int keys = jhi - jlo + 1;
     unsigned best = 0u;
-    for (int j0 = tid; j0 < s; j0 += 4 * 128) { // S14 over the whole row, four reads in flight; the visible scores stay here
+    for (int j0 = tid; j0 < s; j0 += 4 * CTX_T) { // S14 over the whole row, four reads in flight; the visible scores stay here
         float x[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) x[u] = j0 + u * 128 < s ? ftz_bits(row[j0 + u * 128]) : 0.f;
+        for (int u = 0; u < 4; u++) x[u] = j0 + u * CTX_T < s ? ftz_bits(row[j0 + u * CTX_T]) : 0.f;
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const int j = j0 + u * 128;
+            const int j = j0 + u * CTX_T;
             if (j < s) best = max(best, order_key(x[u]));
             if (j >= jlo && j <= jhi) wrow[j - jlo] = x[u];
         }
@@ -1116,14 +1118,15 @@ __global__ void __launch_bounds__(128) attn_context_row_kernel(float *__restrict
     for (int off = 16; off > 0; off >>= 1) best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, off));
     if (lane == 0) red[warp] = best;
     __syncthreads();
-    best = max(max(red[0], red[1]), max(red[2], red[3]));
+#pragma unroll
+    for (int w = 0; w < CTX_T / 32; w++) best = max(best, red[w]);
     const float fm = ftz_bits(order_unkey(best));
-    for (int i = tid; i < keys; i += 128) wrow[i] = ftz_bits(p_expf(ftz_bits(__fsub_rn(wrow[i], fm))));
+    for (int i = tid; i < keys; i += CTX_T) wrow[i] = ftz_bits(p_expf(ftz_bits(__fsub_rn(wrow[i], fm))));
     __syncthreads();
     // S17: serial ascending, every value already flushed; every warp walks it, so none waits for another to hand it over
     const float den = row_chain(wrow, keys, [](float v, float acc) { return add_flushed(acc, v); });
     __syncthreads(); // all have read the exponentials
-    for (int i0 = warp * 32; i0 < keys; i0 += 128) {
+    for (int i0 = warp * 32; i0 < keys; i0 += CTX_T) {
         const int i = i0 + lane;
         float wgt = 0.f;
         if (i < keys) {
@@ -1134,11 +1137,12 @@ __global__ void __launch_bounds__(128) attn_context_row_kernel(float *__restrict
         if (lane == 0) wok[i0 / CTX_NB] = ok ? 1 : 0;
     }
     __syncthreads();
-    // Values: the 32 words of a tile go to registers while the chain of the tile before runs, so a chain step costs its own
-    // latency. When all weights and values of a tile pass the product's admission test and every earlier step of the chain
-    // was admitted too, the bare fma is the contract's step (no result can be subnormal), else the flushed step. The values'
-    // keys are taken 16 bytes at a time by all threads (a tile is hd * 32 words, a chain reads one in hd of them), and the
-    // barrier that frees the tile's slot carries the verdict.
+    // Values: thread d of the first warps walks feature d. The 32 words of a tile go to registers while the chain of the tile
+    // before runs, so a chain step costs its own latency. When all weights and values of a tile pass the product's admission
+    // test and every earlier step of the chain was admitted too, the bare fma is the contract's step (no result can be
+    // subnormal), else the flushed step. The values' keys are taken 16 bytes at a time by the warps that have no feature (by all when every one has), and
+    // the barrier that frees the tile's slot carries the verdict.
+    const int chains = (hd + 31) / 32, helpers = CTX_T / 32 - chains; // warps; head_dim <= 128
     float acc = 0.f;
     bool clean = true, admitted = false;
     const int d = tid < hd ? tid : 0;
@@ -1174,14 +1178,21 @@ __global__ void __launch_bounds__(128) attn_context_row_kernel(float *__restrict
         const int count = min(CTX_NB, keys - k * CTX_NB);
         float next[CTX_NB];
         unsigned key = wok[k] ? 0xFFFFFFFFu : 0u;
-        if (count == CTX_NB) {
+        if (warp < chains) {
+            if (count == CTX_NB) {
 #pragma unroll
-            for (int u = 0; u < CTX_NB; u++) next[u] = vs[u * hd];
-            for (int i = tid * 4; i < CTX_NB * hd; i += 4 * 128) key = min(key, key_of4(*reinterpret_cast<const float4 *>(tile + i)));
+                for (int u = 0; u < CTX_NB; u++) next[u] = vs[u * hd];
+            }
+            if (k > 0) walk(k - 1, cur);
         }
-        if (k > 0) walk(k - 1, cur);
+        if (count == CTX_NB && (helpers == 0 || warp >= chains)) {
+            const int first = helpers == 0 ? tid : tid - chains * 32, step = helpers == 0 ? CTX_T : 32 * helpers;
+            for (int i = first * 4; i < CTX_NB * hd; i += 4 * step) key = min(key, key_of4(*reinterpret_cast<const float4 *>(tile + i)));
+        }
         admitted = __syncthreads_and(key >= ADMIT_MIN); // every thread holds its words of the tile: the slot is free
-        if (count < CTX_NB) { // the last tile, ragged
+        if (warp >= chains) {
+            // nothing to walk
+        } else if (count < CTX_NB) { // the last tile, ragged
             for (int u = 0; u < count; u++) acc = step_flush(wrow[k * CTX_NB + u], ftz_bits(vs[u * hd]), acc);
         } else {
 #pragma unroll
