@@ -15,7 +15,6 @@ always rotates (transformer/block_options.mojo:46-48).
 Activations may be numpy arrays (copied to the device and back, like the
 reference's host surface) or CUDA torch tensors (stay on the device).
 """
-import ctypes
 import os
 
 import numpy as np
@@ -32,12 +31,7 @@ GATED = (0, 4, 5)
 MAX_POSITIONS = 8192
 
 
-def _vp(t):
-    return t.data_ptr() if t is not None else None
-
-
-def _stream(dev):
-    return torch.cuda.current_stream(dev).cuda_stream
+_vp, _stream = torch_ops._vp, torch_ops._stream
 
 
 def _vector(x, name, device):
