@@ -1,10 +1,10 @@
 // The int8i32.v1 product on SM pairs: gemm_int8_tma.cuh with two CTAs of a cluster working on one 256 x 256 tile.
 //
-// The one-CTA kernel is bound by its operand copies: 48 KB of L2 reads per 128 x 256 x 128 block of products, 8.4 TB/s
-// for the device with the tensor pipe 40 % busy. A pair issues tcgen05.mma.cta_group::2 (M 256, N 256, K 32): each CTA
-// brings its own 128 rows of A and HALF of the 256 rows of B, and both tensor cores read both halves, so the same block
-// costs an SM 32 KB, two thirds of the traffic, and six stages fit where four did. With the store taken off the critical path
-// (i8_store_block) 4096^3 takes 60 us = 2.30 POP/s (96 before, 62 with one CTA per tile), 8192^2 x 4096 2.69 POP/s.
+// A pair issues tcgen05.mma.cta_group::2 (M 256, N 256, K 32): each CTA brings its own 128 rows of A and HALF of the 256 rows
+// of B, and both tensor cores read both halves, so a 128 x 256 x 128 block of products costs an SM 32 KB of L2 reads where a
+// lone CTA reads 48, and six stages fit where four did. Both kernels were bound by their store until it was cut to a
+// conversion and two products per cell (i8_store_block): 4096^3 then takes 60 us = 2.30 POP/s (96 before), 62 with one CTA
+// per tile; 8192^2 x 4096 2.69 POP/s against 2.55.
 //
 //   - warp 0, one lane, in both CTAs: the producer of that CTA's rows; its copies complete on the LEADER's mbarrier.
 //   - warp 1, one lane, in the leader (rank 0): the MMA issuer for both; its commits arrive in both CTAs.
