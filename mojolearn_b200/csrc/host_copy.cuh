@@ -14,7 +14,6 @@
 
 #include <atomic>
 #include <cstring>
-#include <system_error>
 #include <thread>
 
 namespace b200i {
@@ -62,7 +61,7 @@ class HostCopier {
             try {
                 workers_[i] = std::thread(&HostCopier::work, this, i);
                 started_++;
-            } catch (const std::system_error &) {
+            } catch (...) { // no thread, no memory for one: the workers there are do the work; nothing leaves a C entry
                 break;
             }
         }
