@@ -79,7 +79,9 @@ int64_t b200i_gemm_w(int64_t device, void *stream, float *c, const float *a, con
  * 6 = the skinny plan (op NT, up to 32 activation rows, k a multiple of 16, 16-byte aligned
  * operands), 7 = the packed plan (operands repacked into tile-major panels in the workspace,
  * then 128x128 tiles fed by bulk copies; needs a 256-byte aligned workspace of
- * b200i_plan_workspace_bytes); `group_leaves` = leaves per group (a power of two, 0 = no split). Every plan returns the same bits; the tests
+ * b200i_plan_workspace_bytes), 8 = the tall plan (op TN, float32, m and n up to 128, every leaf a group of its own), 9 = the
+ * rows plan (op NT, up to 16 activation rows, leaf groups of at most 32, at 9 to 16 rows 16), 10 = the band plan (op NT,
+ * float32 weights, up to 32 rows); `group_leaves` = leaves per group (a power of two, 0 = no split). Every plan returns the same bits; the tests
  * hold them to that (the reference's launch-invariance gate,
  * gemm/checks/gemm_device_check.mojo:1016). */
 int64_t b200i_gemm_w_plan(int64_t device, void *stream, float *c, const float *a, const void *b, const void *bscale,
