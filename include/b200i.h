@@ -80,7 +80,8 @@ int64_t b200i_gemm_w(int64_t device, void *stream, float *c, const float *a, con
  * operands), 7 = the packed plan (operands repacked into tile-major panels in the workspace,
  * then 128x128 tiles fed by bulk copies; needs a 256-byte aligned workspace of
  * b200i_plan_workspace_bytes), 8 = the tall plan (op TN, float32, m and n up to 128, every leaf a group of its own), 9 = the
- * rows plan (op NT, up to 16 activation rows, leaf groups of at most 32, at 9 to 16 rows 16), 10 = the band plan (op NT,
+ * rows plan (op NT, up to 16 activation rows, leaf groups of at most 32, at 9 to 16 rows 16, and a weight for which
+ * b200i_rows_plan_stages is not 0: a CTA holds the int8 factors of its n * groups / SMs columns), 10 = the band plan (op NT,
  * float32 weights, up to 32 rows); `group_leaves` = leaves per group (a power of two, 0 = no split). Every plan returns the same bits; the tests
  * hold them to that (the reference's launch-invariance gate,
  * gemm/checks/gemm_device_check.mojo:1016). */
@@ -125,6 +126,14 @@ int64_t b200i_kernel_timing_read(double *total_ms, int64_t *launches);
 /* Scratch a forced plan needs for the shape (group nodes, and the packed plan's panels and flags);
  * plan -1 is b200i_workspace_bytes. */
 int64_t b200i_plan_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t plan, int64_t group_leaves);
+
+/* The plan (and the leaves per group) that the automatic choice takes on a device of `sms` SMs for 16-byte aligned
+ * operands, a plain store and all the workspace it asks for; -1 for a bad extent. No CUDA call is made. */
+int64_t b200i_auto_plan(int64_t m, int64_t n, int64_t k, int64_t op, int64_t wkind, int64_t sms, int64_t *group_leaves);
+
+/* Stages of the rows plan's shared-memory ring on a device of `sms` SMs (2 or 3), 0 where the plan refuses the shape;
+ * *smem_bytes (may be NULL) = the dynamic shared memory of a CTA. No CUDA call is made. */
+int64_t b200i_rows_plan_stages(int64_t m, int64_t n, int64_t k, int64_t wkind, int64_t group_leaves, int64_t sms, int64_t *smem_bytes);
 
 /* 1 when the row-streaming decode plan accepts the shape (op NT, m <= 8, k a
  * multiple of 16 with 128-element leaves, leaf partials and two ring stages

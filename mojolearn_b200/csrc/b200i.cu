@@ -269,7 +269,8 @@ Plan choose_rows(long long k) {
 // a CTA has one strip of sixteen columns (float32 [2304, 768] 8.9 against 16, [768, 3072] 11.5 against 15.8, but [3072, 768]
 // 16.4 against 15.7).
 inline bool rows_preferred(long long m, long long n, long long k, int wkind, int sms) {
-    if (m < 4 || (leaf_count(k) > 16 && rows_group_leaves(m) < choose_rows(k).group_leaves)) return false;
+    RowsLaunch held;
+    if (m < 4 || !rows_layout(m, n, k, wkind, choose_rows(k).group_leaves, sms, held)) return false;
     if (m <= 8) return wkind == W_F32 || n <= 3072 || (wkind != W_BF16 && m > 4 && k >= 4096);
     return n <= 16ll * sms && (wkind == W_F32 || k <= 1024);
 }
@@ -424,6 +425,41 @@ unsigned grid_for(long long work_items, int block, int sms) {
     return (unsigned)blocks;
 }
 
+size_t plan_need(const Plan &p, long long m, long long n, long long k) { // workspace bytes
+    if (p.kind == PLAN_PACKED) return packed_need(m, n, k, p.groups);
+    if (p.kind == PLAN_TALL) return tall_workspace_bytes(m, n, k);
+    return p.groups > 1 ? (size_t)p.groups * m * n * 4 : 0;
+}
+
+// The automatic choice. `al16`: both operands start on 16 bytes; `pairs`: a gated store; `nodes`: the caller folds.
+// `fits(plan)`: the call's workspace holds what the plan needs; a call whose workspace does not keeps the plan before it.
+struct AutoCall {
+    long long m, n, k;
+    int op, wkind, sms;
+    bool al16, pairs, nodes;
+};
+template <class Fits>
+Plan choose_auto(const AutoCall &x, Fits fits) {
+    const long long m = x.m, n = x.n, k = x.k;
+    Plan plan = choose_plan(m, n, k, x.sms);
+    auto take = [&](const Plan &p) { if (fits(p)) plan = p; };
+    if (packed_candidate(plan.kind, m, n, k)) take(packed_split(plan, m, n, k, x.sms));
+    const bool dec = decode_plan_fits(m, n, k, x.op, x.wkind) && x.al16;
+    const bool skinny = skinny_plan_fits(m, n, k, x.op) && x.al16;
+    const bool wide = n >= DECODE_WIDE_N && (x.wkind == W_BF16 || m == 3);
+    // low-bit weights: the leaf-pair decode kernel wherever it fits (up to four rows), else the rule above
+    const bool pair = x.wkind != W_F32 && decode_pair_fits(m, n, k, x.op, x.wkind, x.sms);
+    const int prefer_m = pair ? DP_MAX_M : ((x.wkind != W_F32 && skinny && !wide) ? DECODE_PREFER_M_LOWBIT : DECODE_PREFER_M);
+    const Plan decode{PLAN_DECODE, (int)leaf_count(k), 1};
+    if (dec && m <= prefer_m && !(skinny && x.pairs)) plan = decode; // (a gated store needs the skinny plan)
+    else if (skinny) plan = choose_skinny(m, n, k, x.sms, x.wkind != W_F32);
+    else if (dec) plan = decode;
+    if (rows_plan_fits(m, n, k, x.op) && x.al16 && rows_preferred(m, n, k, x.wkind, x.sms)) plan = choose_rows(k);
+    if (skinny && m > 8 && band_preferred(n, k, x.wkind)) plan = choose_band(m, n, k, x.sms);
+    if (tall_fits(m, n, k, x.op, x.wkind) && tall_candidate(m, n, k) && !x.nodes && !x.pairs) take(Plan{PLAN_TALL, 1, (int)leaf_count(k)});
+    return plan;
+}
+
 int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const void *b, const void *bscale, int wkind,
                        int64_t m, int64_t n, int64_t k, int op, int plan_kind, int64_t group_leaves, void *ws,
                        int64_t ws_bytes, char *err, int64_t err_cap, Epilogue epi = Epilogue{nullptr, EPI_ACT_NONE},
@@ -455,26 +491,12 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
 
     Plan plan;
     if (plan_kind == PLAN_AUTO) {
-        plan = choose_plan(m, n, k, sm_count(dev));
-        if (packed_candidate(plan.kind, m, n, k)) {
-            const Plan packed = packed_split(plan, m, n, k, sm_count(dev));
-            if (ws && aligned(ws, 256) && (size_t)ws_bytes >= packed_need(m, n, k, packed.groups)) plan = packed;
-        }
-        const bool al16 = aligned(b, 16) && aligned(a, 16);
-        const bool dec = decode_plan_fits(m, n, k, op, wkind) && al16;
-        const bool skinny = skinny_plan_fits(m, n, k, op) && al16;
-        const bool wide = n >= DECODE_WIDE_N && (wkind == W_BF16 || m == 3);
-        // low-bit weights: the leaf-pair decode kernel wherever it fits (up to four rows), else the rule above
-        const bool pair = wkind != W_F32 && decode_pair_fits(m, n, k, op, wkind, sm_count(dev));
-        const int prefer_m = pair ? DP_MAX_M : ((wkind != W_F32 && skinny && !wide) ? DECODE_PREFER_M_LOWBIT : DECODE_PREFER_M);
-        if (dec && m <= prefer_m && !(skinny && epilogue_pairs(g.epi))) plan = Plan{PLAN_DECODE, g.leaves, 1}; // (a gated store needs the skinny plan)
-        else if (skinny) plan = choose_skinny(m, n, k, sm_count(dev), wkind != W_F32);
-        else if (dec) plan = Plan{PLAN_DECODE, g.leaves, 1};
-        if (rows_plan_fits(m, n, k, op) && al16 && rows_preferred(m, n, k, wkind, sm_count(dev))) plan = choose_rows(k);
-        if (skinny && m > 8 && band_preferred(n, k, wkind)) plan = choose_band(m, n, k, sm_count(dev));
-        if (tall_fits(m, n, k, op, wkind) && tall_candidate(m, n, k) && !leave_nodes && !epilogue_pairs(g.epi) && ws && aligned(ws, 4) &&
-            (size_t)ws_bytes >= tall_workspace_bytes(m, n, k))
-            plan = Plan{PLAN_TALL, 1, g.leaves};
+        const bool pairs = epilogue_pairs(g.epi);
+        plan = choose_auto(AutoCall{m, n, k, op, wkind, sm_count(dev), aligned(b, 16) && aligned(a, 16), pairs, leave_nodes != nullptr}, [&](const Plan &p) {
+            const size_t need = plan_need(p, m, n, k);
+            if (need && (!ws || ws_bytes < (int64_t)need || !aligned(ws, p.kind == PLAN_PACKED ? 256 : 4))) return false;
+            return !pairs || p.groups <= 1 || (aligned(ws, 16) && aligned(c, 8)); // the fold of a gated store
+        });
     } else {
         plan.kind = plan_kind;
         int s = group_leaves > 0 ? (int)group_leaves : g.leaves;
@@ -528,10 +550,11 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
             return fail(err, err_cap, "identical gemm: the decode plan needs op NT, m <= %d, k a multiple of 16 and 16-byte aligned weights", DECODE_MAX_M);
         g_launches += launch_decode_plan(g, sm_count(dev), st);
     } else if (plan.kind == PLAN_ROWS) {
-        if (!rows_plan_fits(m, n, k, op) || !aligned(b, 16) || !aligned(a, 16) || plan.group_leaves > rows_group_leaves(m))
-            return fail(err, err_cap, "identical gemm: the rows plan needs op NT, m <= %d, k a multiple of 16, 16-byte aligned operands and leaf groups of at most %d", RW_MAX_ROWS,
-                        rows_group_leaves(m));
-        launch_rows(g, sm_count(dev), st);
+        RowsLaunch rows;
+        if (!rows_plan_fits(m, n, k, op) || !aligned(b, 16) || !aligned(a, 16) || !rows_layout(m, n, k, wkind, plan.group_leaves, sm_count(dev), rows))
+            return fail(err, err_cap, "identical gemm: the rows plan needs op NT, m <= %d, k a multiple of 16, 16-byte aligned operands, leaf groups of at most %d and "
+                        "(int8) a weight whose row factors fit", RW_MAX_ROWS, rows_group_leaves(m));
+        launch_rows(g, rows, st);
         g_launches++;
     } else if (plan.kind == PLAN_BAND) {
         if (!skinny_plan_fits(m, n, k, op) || wkind != W_F32 || !aligned(b, 16) || !aligned(a, 16))
@@ -712,6 +735,22 @@ int64_t b200i_plan_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t plan
     if (plan == PLAN_PACKED) return (int64_t)packed_need(m, n, k, (int)groups);
     if (plan == PLAN_TALL) return (int64_t)tall_workspace_bytes(m, n, k);
     return groups > 1 ? groups * m * n * 4 : 0;
+}
+
+int64_t b200i_auto_plan(int64_t m, int64_t n, int64_t k, int64_t op, int64_t wkind, int64_t sms, int64_t *group_leaves) {
+    if (m <= 0 || n <= 0 || k <= 0 || sms <= 0) return -1;
+    const Plan p = choose_auto(AutoCall{m, n, k, (int)op, (int)wkind, (int)sms, true, false, false}, [](const Plan &) { return true; });
+    if (group_leaves) *group_leaves = p.group_leaves;
+    return p.kind;
+}
+
+int64_t b200i_rows_plan_stages(int64_t m, int64_t n, int64_t k, int64_t wkind, int64_t group_leaves, int64_t sms, int64_t *smem_bytes) {
+    RowsLaunch r;
+    if (m <= 0 || n <= 0 || k <= 0 || sms <= 0 || !rows_plan_fits(m, n, k, OP_NT) ||
+        !rows_layout(m, n, k, (int)wkind, group_leaves > 0 ? (int)group_leaves : (int)leaf_count(k), (int)sms, r))
+        return 0;
+    if (smem_bytes) *smem_bytes = r.smem;
+    return r.p.stages;
 }
 
 int64_t b200i_pair_epilogue_fits(int64_t m, int64_t n, int64_t k, int64_t op) {

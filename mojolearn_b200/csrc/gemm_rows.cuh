@@ -5,8 +5,9 @@
 // groups in a second launch. With eight rows there is too little arithmetic to hide that: 14 us + 4 us of fold for a
 // [2304, 768] float32 product whose bytes take 1 us. Here:
 //
-//   - a CTA owns a contiguous range of weight rows (output columns), about n / SMs of them, so every SM has one CTA and
-//     every CTA the same bytes; it walks them in strips of CB = LC * CPL columns;
+//   - a CTA owns a contiguous range of weight rows (output columns), about n * groups / SMs of them (groups of leaves, below;
+//     one up to sixteen leaves), so nearly every SM has one CTA and every CTA the same bytes; it walks them in strips of
+//     CB = LC * CPL columns;
 //   - the activations of the CTA's leaves are staged ONCE, [k][MT] so that pairs of rows are ready fma.rn.f32x2 operands;
 //   - a warp takes a unit (strip, aligned run of leaves): its own ring of 128-byte row segments by cp.async (16-byte
 //     pieces permuted by the row, so that 32 lanes read 32 rows without a bank conflict), no barrier wider than the warp.
@@ -22,6 +23,8 @@
 // Admission is per leaf: the activations' keys are taken while they are staged, the weights' while they are used; a lane
 // whose leaf fails runs the defining flushed chain again from global memory.
 #pragma once
+#include <algorithm>
+
 #include "gemm_skinny.cuh"
 
 namespace b200i {
@@ -347,9 +350,54 @@ inline int rows_mt(long long m) { return m <= 8 ? 8 : 16; }
 // leaves per CTA whose activations fit: a power of two (32 at eight rows, 16 at sixteen)
 inline int rows_group_leaves(long long m) { return RW_ACT_LIMIT / (rows_mt(m) * RW_LEAF * 4); }
 
+// A launch of the rows plan: the kernel's strip shape, its plan, and its dynamic shared memory.
+struct RowsLaunch {
+    int lc, cpl, smem;
+    RowsPlan p;
+};
+// Lays out a CTA's shared memory; false where it does not hold two stages of a ring for four warps, which is what the kernel's
+// waits need (one stage would be read while its copy is in flight). The factors of int8 weights are what can fill it: four
+// bytes for each of a CTA's n * groups / SMs columns, so about n * k above four billion codes. The rule and the launch
+// both ask here.
+inline bool rows_layout(long long m, long long n, long long k, int wkind, int group_leaves, int sms, RowsLaunch &r) {
+    const int leaves = (int)leaf_count(k), gl = group_leaves < leaves ? group_leaves : leaves, mt = rows_mt(m);
+    if (gl > rows_group_leaves(m)) return false;
+    const int groups = (leaves + gl - 1) / gl, ctas = sms / groups > 0 ? sms / groups : 1;
+    long long cpc = (n + ctas - 1) / ctas;
+    cpc = (cpc + 1) / 2 * 2;
+    r.lc = cpc <= 8 ? 8 : (cpc <= 16 ? 16 : 32);
+    r.cpl = mt > 8 || cpc <= 48 ? 1 : 2;
+    if (cpc <= 16) cpc = r.lc;
+    const int cb = r.lc * r.cpl, stage = cb * RW_SEG;
+    const long long strips = (cpc + cb - 1) / cb, factors = wkind == W_INT8_EXP || wkind == W_INT8_SCALE ? (cpc * 4 + 127) / 128 * 128 : 0;
+    if (factors > RW_SMEM_LIMIT) return false;
+    const long long act = std::min((long long)gl * RW_LEAF, k) * mt * 4;
+    RowsPlan &p = r.p;
+    p.cpc = (int)cpc;
+    // sixteen warps with single leaves, then pairs and fours; eight and four warps when the ring would be shorter than two stages
+    for (int most = RW_MAX_WARPS; most >= 4; most /= 2) {
+        p.run = 1;
+        while (p.run < 4 && (gl + p.run - 1) / p.run > most) p.run *= 2;
+        const int runs = (gl + p.run - 1) / p.run;
+        p.together = 1;
+        while (p.together * 2 <= strips && p.together * runs < 2 * most && (p.together * runs) % most != 0) p.together *= 2;
+        const int total = p.together * runs;
+        p.warps = total < most ? total : most;
+        p.parts_off = (int)((act + 127) / 128 * 128);
+        p.factor_off = p.parts_off + total * mt * cb * 4;
+        p.key_off = p.factor_off + (int)factors;
+        p.ring_off = (p.key_off + gl * 4 + 127) / 128 * 128;
+        p.stages = p.ring_off < RW_SMEM_LIMIT ? (RW_SMEM_LIMIT - p.ring_off) / (p.warps * stage) : 0;
+        if (p.stages < 2) continue;
+        if (p.stages > 3) p.stages = 3;
+        r.smem = p.ring_off + p.warps * p.stages * stage;
+        return true;
+    }
+    return false;
+}
+
 template <int WK, int MT, int LC, int CPL>
-inline void launch_rows_cfg(const GemmArgs &g, int cpc, cudaStream_t st) {
-    constexpr int CB = LC * CPL, STAGE = CB * RW_SEG;
+inline void launch_rows_cfg(const GemmArgs &g, const RowsLaunch &r, cudaStream_t st) {
     static std::atomic<bool> configured[64];
     int dev = 0;
     cudaGetDevice(&dev);
@@ -357,59 +405,28 @@ inline void launch_rows_cfg(const GemmArgs &g, int cpc, cudaStream_t st) {
         cudaFuncSetAttribute(gemm_rows_kernel<WK, MT, LC, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, RW_SMEM_LIMIT);
         configured[dev] = true;
     }
-    const int gl = g.group_leaves < g.leaves ? g.group_leaves : g.leaves;
-    const int strips = (cpc + CB - 1) / CB;
-    RowsPlan p;
-    p.cpc = cpc;
-    const int act = gl * RW_LEAF * MT * 4 < g.k * MT * 4 ? gl * RW_LEAF * MT * 4 : g.k * MT * 4;
-    // sixteen warps with single leaves, then pairs and fours; eight warps when the ring would be shorter than two stages
-    p.warps = RW_MAX_WARPS;
-    for (;;) {
-        p.run = 1;
-        while (p.run < 4 && (gl + p.run - 1) / p.run > p.warps) p.run *= 2;
-        const int runs = (gl + p.run - 1) / p.run;
-        p.together = 1;
-        while (p.together * 2 <= strips && p.together * runs < 2 * p.warps && (p.together * runs) % p.warps != 0) p.together *= 2;
-        const int total = p.together * runs;
-        const int warps = total < p.warps ? total : p.warps;
-        p.parts_off = (act + 127) / 128 * 128;
-        p.factor_off = p.parts_off + total * MT * CB * 4;
-        p.key_off = p.factor_off + (WK == W_INT8_EXP || WK == W_INT8_SCALE ? (cpc * 4 + 127) / 128 * 128 : 0);
-        p.ring_off = (p.key_off + gl * 4 + 127) / 128 * 128;
-        p.stages = (RW_SMEM_LIMIT - p.ring_off) / (warps * STAGE);
-        if (p.stages >= 2 || p.warps == 4) {
-            p.warps = warps;
-            break;
-        }
-        p.warps /= 2;
-    }
-    if (p.stages > 3) p.stages = 3;
-    const int smem = p.ring_off + p.warps * p.stages * STAGE;
-    const dim3 grid((unsigned)((g.n + cpc - 1) / cpc), (unsigned)g.groups);
-    gemm_rows_kernel<WK, MT, LC, CPL><<<grid, 32 * p.warps, smem, st>>>(g, p);
+    const dim3 grid((unsigned)((g.n + r.p.cpc - 1) / r.p.cpc), (unsigned)g.groups);
+    gemm_rows_kernel<WK, MT, LC, CPL><<<grid, 32 * r.p.warps, r.smem, st>>>(g, r.p);
 }
 
 template <int WK, int MT>
-inline void launch_rows_mt(const GemmArgs &g, int sms, cudaStream_t st) {
-    const int ctas = sms / g.groups > 0 ? sms / g.groups : 1;
-    int cpc = (g.n + ctas - 1) / ctas;
-    cpc = (cpc + 1) / 2 * 2;
-    if (cpc <= 8) launch_rows_cfg<WK, MT, 8, 1>(g, 8, st);
-    else if (cpc <= 16) launch_rows_cfg<WK, MT, 16, 1>(g, 16, st);
-    else if (MT > 8 || cpc <= 48) launch_rows_cfg<WK, MT, 32, 1>(g, cpc, st);
-    else launch_rows_cfg<WK, 8, 32, 2>(g, cpc, st);
+inline void launch_rows_mt(const GemmArgs &g, const RowsLaunch &r, cudaStream_t st) {
+    if (r.lc == 8) launch_rows_cfg<WK, MT, 8, 1>(g, r, st);
+    else if (r.lc == 16) launch_rows_cfg<WK, MT, 16, 1>(g, r, st);
+    else if (r.cpl == 1) launch_rows_cfg<WK, MT, 32, 1>(g, r, st);
+    else launch_rows_cfg<WK, 8, 32, 2>(g, r, st);
 }
 template <int WK>
-inline void launch_rows_wk(const GemmArgs &g, int sms, cudaStream_t st) {
-    if (g.m <= 8) launch_rows_mt<WK, 8>(g, sms, st);
-    else launch_rows_mt<WK, 16>(g, sms, st);
+inline void launch_rows_wk(const GemmArgs &g, const RowsLaunch &r, cudaStream_t st) {
+    if (g.m <= 8) launch_rows_mt<WK, 8>(g, r, st);
+    else launch_rows_mt<WK, 16>(g, r, st);
 }
-inline void launch_rows(const GemmArgs &g, int sms, cudaStream_t st) {
+inline void launch_rows(const GemmArgs &g, const RowsLaunch &r, cudaStream_t st) {
     switch (g.wkind) {
-    case W_F32: launch_rows_wk<W_F32>(g, sms, st); break;
-    case W_BF16: launch_rows_wk<W_BF16>(g, sms, st); break;
-    case W_INT8_EXP: launch_rows_wk<W_INT8_EXP>(g, sms, st); break;
-    default: launch_rows_wk<W_INT8_SCALE>(g, sms, st); break;
+    case W_F32: launch_rows_wk<W_F32>(g, r, st); break;
+    case W_BF16: launch_rows_wk<W_BF16>(g, r, st); break;
+    case W_INT8_EXP: launch_rows_wk<W_INT8_EXP>(g, r, st); break;
+    default: launch_rows_wk<W_INT8_SCALE>(g, r, st); break;
     }
 }
 

@@ -1,0 +1,53 @@
+"""The host arithmetic of the product's plans, without a GPU: what the automatic choice takes, and the shared memory that the
+rows plan lays out for it."""
+import ctypes
+
+import pytest
+
+from mojolearn_b200 import _native
+from mojolearn_b200.linalg import OP_NT, W_BF16, W_F32, W_INT8_EXP, W_INT8_SCALE, leaf_count
+from mojolearn_b200.torch_ops import PLAN_ROWS, PLAN_SKINNY
+
+SMEM_LIMIT = 225 * 1024  # of a CTA of the rows plan; the device's own limit is 227 KB
+KINDS = [W_F32, W_BF16, W_INT8_EXP, W_INT8_SCALE]
+
+
+def auto_plan(m, n, k, op=OP_NT, wkind=W_F32, sms=148):
+    leaves = ctypes.c_int64()
+    return _native.lib().b200i_auto_plan(m, n, k, op, wkind, sms, ctypes.byref(leaves)), leaves.value
+
+
+def rows_stages(m, n, k, wkind, group_leaves, sms=148):
+    smem = ctypes.c_int64()
+    return _native.lib().b200i_rows_plan_stages(m, n, k, wkind, group_leaves, sms, ctypes.byref(smem)), smem.value
+
+
+@pytest.mark.parametrize("kind", [W_INT8_EXP, W_INT8_SCALE])
+@pytest.mark.parametrize("n,k", [(1144930, 4096), (278498, 16384), (61890, 65536), (65536, 50304), (151936, 32768), (300000, 16384), (100000, 65536),
+                                 (131072, 65536), (2000000000, 4096)])
+def test_weights_whose_factors_leave_no_ring_keep_the_skinny_plan(n, k, kind):
+    for m in (5, 8):
+        assert auto_plan(m, n, k, wkind=kind)[0] == PLAN_SKINNY
+        run = 8
+        while -(-leaf_count(k) // run) > 64:
+            run *= 2
+        assert rows_stages(m, n, k, kind, run)[0] == 0
+
+
+@pytest.mark.parametrize("sms", [148, 132, 16, 1])
+@pytest.mark.parametrize("kind", KINDS)
+def test_the_rows_plan_always_has_two_stages(kind, sms):
+    """Whatever the rule takes and whatever may be asked for by hand: a ring of two or three stages inside the limit, or a refusal."""
+    taken = 0
+    for m in (4, 5, 8, 9, 16):
+        for k in (16, 128, 144, 768, 2048, 2064, 3072, 4096, 8192, 16384, 32768, 50304, 65536, 131072):
+            for n in (1, 2, 24, 305, 768, 2304, 2369, 3072, 11008, 50304, 61890, 278498, 1144929, 1144930, 30000000, 2000000000):
+                plan, leaves = auto_plan(m, n, k, wkind=kind, sms=sms)
+                if plan == PLAN_ROWS:
+                    taken += 1
+                    stages, smem = rows_stages(m, n, k, kind, leaves, sms)
+                    assert stages in (2, 3) and smem <= SMEM_LIMIT, (m, n, k, stages, smem)
+                for run in (1, 2, 4, 8, 16, 32):
+                    stages, smem = rows_stages(m, n, k, kind, run, sms)
+                    assert stages in (0, 2, 3) and (stages == 0 or smem <= SMEM_LIMIT), (m, n, k, run, stages, smem)
+    assert taken > 50
