@@ -1224,11 +1224,8 @@ static int64_t attention_launch(int dev, cudaStream_t st, float *ctx, const floa
         // scores kernel's split over key tiles is what keeps all SMs loading.
         const int lq = l == 1 ? 1 : (l == 2 ? 2 : (l <= 4 ? 4 : 8));
         const long long ctas = b * n_heads;
-        const int sms = sm_count(dev);
-        long long per_sm = (ctas + sms - 1) / sms; // CTAs an SM must hold for the call to be one wave
-        if (per_sm > 6) per_sm = 6;
         const long long fixed = (long long)lq * K_LEAF_MIN + (long long)lq * ((s_grid + 3) & ~3);
-        const long long room = (226ll * 1024 / per_sm - 1280) / 4 - fixed; // floats for the key tiles / the value ring
+        const long long room = att_cta_bytes(ctas, sm_count(dev), 6) / 4 - fixed; // floats for the key tiles / the value ring
         int kkeys = 32, nkb = (int)(room / (ATD_WARPS * 32 * ATT_KT_PITCH));
         if (nkb > 3) nkb = 3;
         if (nkb < 1) { // not even one full tile per warp: fewer keys per tile
@@ -1244,7 +1241,7 @@ static int64_t attention_launch(int dev, cudaStream_t st, float *ctx, const floa
     do {                                                                                                                          \
         static std::atomic<bool> configured[64];                                                                                  \
         if (dev >= 0 && dev < 64 && !configured[dev]) {                                                                           \
-            CUDA_TRY(cudaFuncSetAttribute(attn_decode_kernel<LQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));      \
+            CUDA_TRY(cudaFuncSetAttribute(attn_decode_kernel<LQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM_LIMIT));  \
             configured[dev] = true;                                                                                               \
         }                                                                                                                         \
         attn_decode_kernel<LQ><<<(unsigned)ctas, ATD_THREADS, smem, st>>>(ctx, q, kcache, vcache, (int)b, (int)l, (int)n_heads,   \
@@ -1289,24 +1286,20 @@ static int64_t attention_launch(int dev, cudaStream_t st, float *ctx, const floa
     if (l <= ATT_SMALL_Q && (size_t)s_grid * sizeof(float) <= 40 * 1024) {
         static std::atomic<bool> configured[64];
         if (dev >= 0 && dev < 64 && !configured[dev]) {
-            CUDA_TRY(cudaFuncSetAttribute(attn_context_row_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-            CUDA_TRY(cudaFuncSetAttribute(attn_context_row_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+            CUDA_TRY(cudaFuncSetAttribute(attn_context_row_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM_LIMIT));
+            CUDA_TRY(cudaFuncSetAttribute(attn_context_row_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM_LIMIT));
             configured[dev] = true;
         }
         // enough CTAs per SM for one wave (four at most); the shared memory that leaves a CTA becomes ring stages
         const long long rows = b * n_heads * l;
-        long long per_sm = (rows + sm_count(dev) - 1) / sm_count(dev);
-        if (per_sm > 4) per_sm = 4;
-        long long stages = ((226ll * 1024 / per_sm - 1664) / 4 - ((s_grid + 3) & ~3)) / (CTX_NB * head_dim);
-        if (stages > CTX_ST_MAX) stages = CTX_ST_MAX;
-        if (stages < CTX_ST) stages = CTX_ST;
-        const size_t row_smem = attn_context_row_smem(s_grid, (int)head_dim, (int)stages);
+        const int stages = attn_context_row_stages(rows, s_grid, (int)head_dim, sm_count(dev));
+        const size_t row_smem = attn_context_row_smem(s_grid, (int)head_dim, stages);
         if (rows <= 2ll * sm_count(dev))
             attn_context_row_kernel<256><<<(unsigned)rows, 256, row_smem, st>>>(ctx, scores, vcache, (int)b, (int)l, (int)n_heads, (int)n_kv, (int)head_dim, (int)cap,
-                                                                                key_lo, s, own0, (int)window, position, s_grid, (int)stages);
+                                                                                key_lo, s, own0, (int)window, position, s_grid, stages);
         else
             attn_context_row_kernel<128><<<(unsigned)rows, 128, row_smem, st>>>(ctx, scores, vcache, (int)b, (int)l, (int)n_heads, (int)n_kv, (int)head_dim, (int)cap,
-                                                                                key_lo, s, own0, (int)window, position, s_grid, (int)stages);
+                                                                                key_lo, s, own0, (int)window, position, s_grid, stages);
     } else {
         dim3 g2((unsigned)((l + CTX_ROWS - 1) / CTX_ROWS), (unsigned)(b * n_heads));
 #define CONTEXT_ROWS(DPL)                                                                                                     \

@@ -19,6 +19,8 @@
 // 128-byte row segments, one warp per row or one thread per element, grids sized
 // from the row count.
 #pragma once
+#include <algorithm>
+
 #include "decode.cuh" // mbarrier and bulk-copy primitives, the status word of the bounded waits
 #include "seams_math.cuh"
 
@@ -1054,6 +1056,19 @@ constexpr int CTX_NB = 32, CTX_ST = 3, CTX_ST_MAX = 12;
 // what is not a chain.
 inline size_t attn_context_row_smem(int s_grid, int hd, int stages = CTX_ST) {
     return ((size_t)((s_grid + 3) & ~3) + (size_t)stages * CTX_NB * hd) * sizeof(float) + (size_t)(s_grid + CTX_NB) / CTX_NB;
+}
+// What the decode attention kernels divide among the CTAs of an SM, and what a CTA has of it beside its dynamic part (its
+// static arrays and the system's 1 KB; 2 KB of the SM stay over for what that leaves out). A launch spends the rest of its
+// share on bytes in flight, and the kernels' attribute is the share of a CTA alone, so no launch asks for more than it.
+constexpr long long ATT_SM_BYTES = 226 * 1024, ATT_CTA_BYTES = 1280;
+constexpr int ATT_SMEM_LIMIT = (int)(ATT_SM_BYTES - ATT_CTA_BYTES);
+inline long long att_cta_bytes(long long ctas, int sms, long long most) { // enough CTAs per SM for one wave, `most` at the most
+    const long long per_sm = std::min((ctas + sms - 1) / sms, most);
+    return ATT_SM_BYTES / per_sm - ATT_CTA_BYTES;
+}
+inline int attn_context_row_stages(long long rows, int s_grid, int hd, int sms) {
+    const long long ring = att_cta_bytes(rows, sms, 4) - (long long)attn_context_row_smem(s_grid, hd, 0);
+    return (int)std::min<long long>(std::max<long long>(ring / (CTX_NB * hd * (long long)sizeof(float)), CTX_ST), CTX_ST_MAX);
 }
 template <int CTX_T>
 __global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(float *__restrict__ ctx, float *__restrict__ scores,

@@ -119,3 +119,15 @@ def test_prefill_attention_against_the_oracle_at_head_dim_128_and_64():
         want = oracle.attention(q, kc, vc, l, used, window)
         got = _run(q, kc, vc, l, used, window, False)
         assert got.tobytes() == want.tobytes(), (hd, l, used, window)
+
+
+@pytest.mark.parametrize("l,hd,cap,used", [(1, 128, 8192, 8192), (1, 128, 7150, 7140), (1, 128, 10240, 8288), (2, 64, 2700, 2690), (2, 128, 8192, 8100),
+                                           (4, 128, 1300, 1285), (4, 64, 8192, 6000), (8, 64, 600, 580), (8, 128, 4096, 3200)])
+def test_few_rows_on_a_long_cache(l, hd, cap, used):
+    """A lone sequence on a long cache: the launch spends an SM's whole shared memory on its score rows and its ring."""
+    rng = np.random.default_rng(cap + l)
+    q, kc, vc = _operands(rng, 1, l, 2, 1, hd, cap, 0.3)
+    want = oracle.attention(q, kc, vc, l, used)
+    for at in (False, True):
+        got = _run(q, kc, vc, l, used, 0, at)
+        assert got.tobytes() == want.tobytes(), at
