@@ -128,8 +128,9 @@ int64_t b200i_kernel_timing_read(double *total_ms, int64_t *launches);
 int64_t b200i_plan_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t plan, int64_t group_leaves);
 
 /* The plan (and the leaves per group) that the automatic choice takes on a device of `sms` SMs for 16-byte aligned
- * operands, a plain store and all the workspace it asks for; -1 for a bad extent. No CUDA call is made. */
-int64_t b200i_auto_plan(int64_t m, int64_t n, int64_t k, int64_t op, int64_t wkind, int64_t sms, int64_t *group_leaves);
+ * operands, a plain store and `ws_bytes` of workspace (-1 = all it asks for; a plan that the workspace does not hold is passed
+ * over for the one before it); -1 for a bad extent. No CUDA call is made. */
+int64_t b200i_auto_plan(int64_t m, int64_t n, int64_t k, int64_t op, int64_t wkind, int64_t sms, int64_t ws_bytes, int64_t *group_leaves);
 
 /* Stages of the rows plan's shared-memory ring on a device of `sms` SMs (2 or 3), 0 where the plan refuses the shape;
  * *smem_bytes (may be NULL) = the dynamic shared memory of a CTA. No CUDA call is made. */

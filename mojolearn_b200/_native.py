@@ -45,7 +45,7 @@ SIGNATURES = {
     "b200i_launch_count": [],
     "b200i_workspace_bytes": [I64, I64, I64],
     "b200i_plan_workspace_bytes": [I64, I64, I64, I64, I64],
-    "b200i_auto_plan": [I64, I64, I64, I64, I64, I64, VP],
+    "b200i_auto_plan": [I64, I64, I64, I64, I64, I64, I64, VP],
     "b200i_rows_plan_stages": [I64, I64, I64, I64, I64, I64, VP],
     "b200i_kernel_timing": [I64],
     "b200i_kernel_timing_read": [VP, VP],

@@ -454,8 +454,8 @@ Plan choose_auto(const AutoCall &x, Fits fits) {
     if (dec && m <= prefer_m && !(skinny && x.pairs)) plan = decode; // (a gated store needs the skinny plan)
     else if (skinny) plan = choose_skinny(m, n, k, x.sms, x.wkind != W_F32);
     else if (dec) plan = decode;
-    if (rows_plan_fits(m, n, k, x.op) && x.al16 && rows_preferred(m, n, k, x.wkind, x.sms)) plan = choose_rows(k);
-    if (skinny && m > 8 && band_preferred(n, k, x.wkind)) plan = choose_band(m, n, k, x.sms);
+    if (rows_plan_fits(m, n, k, x.op) && x.al16 && rows_preferred(m, n, k, x.wkind, x.sms)) take(choose_rows(k));
+    if (skinny && m > 8 && band_preferred(n, k, x.wkind)) take(choose_band(m, n, k, x.sms));
     if (tall_fits(m, n, k, x.op, x.wkind) && tall_candidate(m, n, k) && !x.nodes && !x.pairs) take(Plan{PLAN_TALL, 1, (int)leaf_count(k)});
     return plan;
 }
@@ -737,9 +737,10 @@ int64_t b200i_plan_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t plan
     return groups > 1 ? groups * m * n * 4 : 0;
 }
 
-int64_t b200i_auto_plan(int64_t m, int64_t n, int64_t k, int64_t op, int64_t wkind, int64_t sms, int64_t *group_leaves) {
+int64_t b200i_auto_plan(int64_t m, int64_t n, int64_t k, int64_t op, int64_t wkind, int64_t sms, int64_t ws_bytes, int64_t *group_leaves) {
     if (m <= 0 || n <= 0 || k <= 0 || sms <= 0) return -1;
-    const Plan p = choose_auto(AutoCall{m, n, k, (int)op, (int)wkind, (int)sms, true, false, false}, [](const Plan &) { return true; });
+    const Plan p = choose_auto(AutoCall{m, n, k, (int)op, (int)wkind, (int)sms, true, false, false},
+                               [&](const Plan &q) { return ws_bytes < 0 || (int64_t)plan_need(q, m, n, k) <= ws_bytes; });
     if (group_leaves) *group_leaves = p.group_leaves;
     return p.kind;
 }

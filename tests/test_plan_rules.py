@@ -6,15 +6,15 @@ import pytest
 
 from mojolearn_b200 import _native
 from mojolearn_b200.linalg import OP_NT, W_BF16, W_F32, W_INT8_EXP, W_INT8_SCALE, leaf_count
-from mojolearn_b200.torch_ops import PLAN_ROWS, PLAN_SKINNY
+from mojolearn_b200.torch_ops import PLAN_BAND, PLAN_ROWS, PLAN_SKINNY
 
 SMEM_LIMIT = 225 * 1024  # of a CTA of the rows plan; the device's own limit is 227 KB
 KINDS = [W_F32, W_BF16, W_INT8_EXP, W_INT8_SCALE]
 
 
-def auto_plan(m, n, k, op=OP_NT, wkind=W_F32, sms=148):
+def auto_plan(m, n, k, op=OP_NT, wkind=W_F32, sms=148, ws=-1):
     leaves = ctypes.c_int64()
-    return _native.lib().b200i_auto_plan(m, n, k, op, wkind, sms, ctypes.byref(leaves)), leaves.value
+    return _native.lib().b200i_auto_plan(m, n, k, op, wkind, sms, ws, ctypes.byref(leaves)), leaves.value
 
 
 def rows_stages(m, n, k, wkind, group_leaves, sms=148):
@@ -51,3 +51,15 @@ def test_the_rows_plan_always_has_two_stages(kind, sms):
                     stages, smem = rows_stages(m, n, k, kind, run, sms)
                     assert stages in (0, 2, 3) and (stages == 0 or smem <= SMEM_LIMIT), (m, n, k, run, stages, smem)
     assert taken > 50
+
+
+@pytest.mark.parametrize("m,n,k,plan", [(8, 220000, 2064, PLAN_ROWS), (4, 400000, 4096, PLAN_ROWS), (14, 178374, 12208, PLAN_BAND), (31, 165405, 1536, PLAN_BAND)])
+def test_a_workspace_that_holds_the_skinny_plan_only_gets_the_skinny_plan(m, n, k, plan):
+    """These sizes are unsplit in the skinny plan, which needs no workspace, and split in the plan that the rule prefers."""
+    got, leaves = auto_plan(m, n, k)
+    assert got == plan and leaves < leaf_count(k)
+    need = -(-leaf_count(k) // leaves) * m * n * 4
+    assert auto_plan(m, n, k, ws=need)[0] == plan
+    for ws in (0, need - 1):
+        got, leaves = auto_plan(m, n, k, ws=ws)
+        assert got != plan and leaves >= leaf_count(k)
