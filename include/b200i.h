@@ -170,10 +170,13 @@ int64_t b200i_gemm_f32_noalloc(int64_t device, void *stream, float *c, const flo
                                int64_t k, int64_t op, char *err, int64_t err_cap);
 int64_t b200i_noalloc_scratch_bytes(int64_t m, int64_t n, int64_t k);
 
-/* Scratch bytes the product needs for this shape. The answer depends on the SM count of the
- * device that is CURRENT when this is called: call it with the device current that the product
+/* Scratch bytes the product needs for this shape, whatever its op and weight storage. The answer depends on the SM count of
+ * the device that is CURRENT when this is called: call it with the device current that the product
  * will later be given. */
 int64_t b200i_workspace_bytes(int64_t m, int64_t n, int64_t k);
+/* The same for one op and weight storage: less where only another op's plan needs much (a tall A^T B product of 128 x 128
+ * over 131072 rows keeps a node per leaf, 67 MB; the same extents as NT or NN take at most 4 MB). */
+int64_t b200i_product_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t op, int64_t wkind);
 
 /* --- conversions, device pointers ----------------------------------------------------------
  * Replace to_bf16 / from_bf16 / quantize_int8 / dequantize_int8

@@ -44,6 +44,7 @@ SIGNATURES = {
     "b200i_device_count": [],
     "b200i_launch_count": [],
     "b200i_workspace_bytes": [I64, I64, I64],
+    "b200i_product_workspace_bytes": [I64, I64, I64, I64, I64],
     "b200i_plan_workspace_bytes": [I64, I64, I64, I64, I64],
     "b200i_auto_plan": [I64, I64, I64, I64, I64, I64, I64, VP],
     "b200i_rows_plan_stages": [I64, I64, I64, I64, I64, I64, VP],

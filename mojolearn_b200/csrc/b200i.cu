@@ -700,6 +700,19 @@ int64_t b200i_workspace_bytes(int64_t m, int64_t n, int64_t k) {
     return groups > 1 ? (int64_t)groups * m * n * 4 : 0;
 }
 
+int64_t b200i_product_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t op, int64_t wkind) {
+    if (m <= 0 || n <= 0 || k <= 0) return 0;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); dev = -1; }
+    size_t most = 0; // of what the choice comes to over operand alignments and stores, and of what it falls back to
+    for (const bool al16 : {true, false})
+        for (const bool pairs : {false, true})
+            for (const bool all : {true, false})
+                most = std::max(most, plan_need(choose_auto(AutoCall{m, n, k, (int)op, (int)wkind, sm_count(dev), al16, pairs, false},
+                                                            [&](const Plan &p) { return all || p.kind == PLAN_PACKED; }), m, n, k));
+    return (int64_t)most;
+}
+
 int64_t b200i_kernel_timing(int64_t enable) {
     std::lock_guard<std::mutex> lock(g_timing_mu);
     g_timing.on = enable != 0;
@@ -1840,7 +1853,7 @@ int64_t b200i_host_gemm_w(int64_t device, float *c, const float *a, const void *
     }
     const size_t abytes = (size_t)m * k * 4, bbytes = (size_t)n * k * wkind_elem_bytes((int)wkind), cbytes = (size_t)m * n * 4;
     const size_t sbytes = (wkind >= W_INT8_EXP) ? (size_t)n * 4 : 0;
-    const int64_t wsbytes = b200i_workspace_bytes(m, n, k);
+    const int64_t wsbytes = b200i_product_workspace_bytes(m, n, k, op, wkind);
     void *da, *db, *dc, *ds = nullptr, *dw = nullptr;
     CUDA_TRY(pool_get(dev, 0, abytes, &da));
     CUDA_TRY(pool_get(dev, 1, bbytes, &db));

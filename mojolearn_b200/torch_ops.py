@@ -48,8 +48,10 @@ def _stream(device):
 
 
 @functools.lru_cache(maxsize=4096)
-def _workspace_bytes(device_index, m, n, k, plan, group_leaves):
-    """A pure function of the shape, the plan and the device's SM count (the device is current when this is called)."""
+def _workspace_bytes(device_index, m, n, k, op, wkind, plan, group_leaves):
+    """A pure function of the call's form, the plan and the device's SM count (the device is current when this is called)."""
+    if plan == PLAN_AUTO:
+        return int(_native.lib().b200i_product_workspace_bytes(m, n, k, op, wkind))
     return int(_native.lib().b200i_plan_workspace_bytes(m, n, k, plan, group_leaves))
 
 
@@ -117,7 +119,7 @@ def product(a, b, bscale=None, wkind=W_F32, op=OP_NN, out=None, plan=PLAN_AUTO, 
         if tuple(out.shape) != (m, n_out):
             raise ValueError("out must be (%d, %d)" % (m, n_out))
     with _on(dev):
-        ws_bytes = _workspace_bytes(dev.index, m, n, k, plan, group_leaves)
+        ws_bytes = _workspace_bytes(dev.index, m, n, k, op, wkind, plan, group_leaves)
         ws = torch.empty((max(ws_bytes, 16),), dtype=torch.uint8, device=dev) if ws_bytes else None
         if bias is None and act == ACT_NONE:
             _native.call("b200i_gemm_w_plan", dev.index, _stream(dev), _vp(out), _vp(a), _vp(b), _vp(bscale), wkind, m, n, k,
@@ -152,10 +154,9 @@ def product_nodes(a, b, bscale=None, wkind=W_F32, bias=None, act=ACT_NONE):
     dev = a.device
     n_out = n // 2 if act >= ACT_PAIR_SWIGLU else n
     out = torch.empty((m, n_out), dtype=torch.float32, device=dev)
-    lib = _native.lib()
     nodes = ctypes.c_int64(1)
     with _on(dev):
-        ws_bytes = int(lib.b200i_plan_workspace_bytes(m, n, k, PLAN_AUTO, 0))
+        ws_bytes = _workspace_bytes(dev.index, m, n, k, OP_NT, wkind, PLAN_AUTO, 0)
         ws = torch.empty((max(ws_bytes, 16),), dtype=torch.uint8, device=dev) if ws_bytes else None
         _native.call("b200i_gemm_w_nodes", dev.index, _stream(dev), _vp(out), _vp(a), _vp(b), _vp(bscale), wkind, m, n, k, OP_NT,
                      _vp(bias), act, _vp(ws), ws_bytes, ctypes.byref(nodes))

@@ -5,7 +5,7 @@ import ctypes
 import pytest
 
 from mojolearn_b200 import _native
-from mojolearn_b200.linalg import OP_NT, W_BF16, W_F32, W_INT8_EXP, W_INT8_SCALE, leaf_count
+from mojolearn_b200.linalg import OP_NN, OP_NT, OP_TN, W_BF16, W_F32, W_INT8_EXP, W_INT8_SCALE, leaf_count
 from mojolearn_b200.torch_ops import PLAN_BAND, PLAN_ROWS, PLAN_SKINNY
 
 SMEM_LIMIT = 225 * 1024  # of a CTA of the rows plan; the device's own limit is 227 KB
@@ -63,3 +63,20 @@ def test_a_workspace_that_holds_the_skinny_plan_only_gets_the_skinny_plan(m, n, 
     for ws in (0, need - 1):
         got, leaves = auto_plan(m, n, k, ws=ws)
         assert got != plan and leaves >= leaf_count(k)
+
+
+def test_workspace_by_op_and_storage():
+    """Enough for the automatic plan, never more than the answer that knows neither op nor storage, and no node per leaf for an
+    op that the tall plan does not take."""
+    lib = _native.lib()
+    for m, n, k in [(128, 128, 131072), (32, 32, 1000000), (27, 27, 3001), (8, 768, 3072), (8, 11008, 4096), (32, 16384, 2048), (300, 5136, 4096),
+                    (128, 11008, 4096), (1000, 1000, 1000), (1, 64, 2048), (5, 7, 50), (31, 165405, 1536)]:
+        for op in (OP_NN, OP_NT, OP_TN):
+            for kind in KINDS if op == OP_NT else (W_F32, W_BF16):
+                plan, leaves = auto_plan(m, n, k, op=op, wkind=kind)
+                need = int(lib.b200i_product_workspace_bytes(m, n, k, op, kind))
+                assert auto_plan(m, n, k, op=op, wkind=kind, ws=need) == (plan, leaves)
+                assert need <= int(lib.b200i_workspace_bytes(m, n, k))
+    assert int(lib.b200i_product_workspace_bytes(128, 128, 131072, OP_TN, W_F32)) == 1024 * 128 * 128 * 4
+    for op, kind in ((OP_NN, W_F32), (OP_NT, W_F32), (OP_NT, W_BF16), (OP_TN, W_BF16)):
+        assert int(lib.b200i_product_workspace_bytes(128, 128, 131072, op, kind)) <= 64 * 128 * 128 * 4
