@@ -878,21 +878,22 @@ int64_t b200i_gemm_int8(int64_t device, void *stream, float *c, const int8_t *qa
     int dev;
     if (select_device(device, err, err_cap, &dev)) return 1;
     const long long cells = m * n;
-    // the tensor-core kernel wherever its 16-byte copies are aligned (k a multiple of 16); one thread per cell otherwise
-    if (gemm_int8_mma_fits(qa, qb, m, n, k)) {
-        const signed char *sa = reinterpret_cast<const signed char *>(qa), *sb = reinterpret_cast<const signed char *>(qb);
+    // the tensor-core kernels wherever their 16-byte copies are aligned (k a multiple of 16) and tensor maps can be made; one
+    // thread per cell otherwise
+    const signed char *sa = reinterpret_cast<const signed char *>(qa), *sb = reinterpret_cast<const signed char *>(qb);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    bool launched = false;
+    if (gemm_int8_mma_fits(qa, qb, k)) {
         const int sms = sm_count(dev);
-        // SM pairs at every size (1024 x 4096 x 4096: 23 us against 100 for the per-tile kernel, 4096^3 60 against 62 for one CTA
-        // per tile), except where the contraction is so short that the store is all there is and the one-CTA kernel's wider
-        // spread of it wins (2048 x 50304 x 768: 157 against 174 us); the per-tile kernel where no tensor map can be made
+        // SM pairs at every size (1024 x 4096 x 4096 in 23 us, 4096^3 60 against 62 for one CTA per tile), except where the
+        // contraction is so short that the store is all there is and the one-CTA kernel's wider spread of it wins
+        // (2048 x 50304 x 768: 157 against 174 us)
         const long long wide = ((m + T8_BM - 1) / T8_BM) * ((n + T8_BN - 1) / T8_BN);
         const bool single = wide >= 4ll * sms && k < 1024;
-        if ((single || !launch_gemm_int8_pair(c, sa, ea, sb, eb, (int)m, (int)n, (int)k, static_cast<cudaStream_t>(stream))) &&
-            !launch_gemm_int8_tma(c, sa, ea, sb, eb, (int)m, (int)n, (int)k, sms, static_cast<cudaStream_t>(stream)))
-            launch_gemm_int8_mma(c, sa, ea, sb, eb, (int)m, (int)n, (int)k, sms, static_cast<cudaStream_t>(stream));
+        launched = (!single && launch_gemm_int8_pair(c, sa, ea, sb, eb, (int)m, (int)n, (int)k, st)) ||
+                   launch_gemm_int8_tma(c, sa, ea, sb, eb, (int)m, (int)n, (int)k, sms, st);
     }
-    else
-        gemm_int8_flat_kernel<<<(unsigned)((cells + 127) / 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(c, reinterpret_cast<const signed char *>(qa), ea, reinterpret_cast<const signed char *>(qb), eb, (int)m, (int)n, (int)k);
+    if (!launched) gemm_int8_flat_kernel<<<(unsigned)((cells + 127) / 128), 128, 0, st>>>(c, sa, ea, sb, eb, (int)m, (int)n, (int)k);
     g_launches++;
     CUDA_TRY(cudaGetLastError());
     return 0;

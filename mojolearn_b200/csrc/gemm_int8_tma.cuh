@@ -1,15 +1,15 @@
 // The int8i32.v1 product as a persistent, warp-specialised tensor-core kernel.
 //
-// gemm_int8_mma.cuh moves its operand tiles with per-thread cp.async copies and a CTA barrier per 128 bytes of k, and
-// that is what bounds it (tensor pipe 12 % busy, long-scoreboard stalls). Here the tile traffic is taken off the threads:
+// Operand tiles moved by per-thread cp.async copies with a CTA barrier per 128 bytes of k kept the tensor pipe 12 % busy
+// (464 TOP/s on 4096^3). Here the tile traffic is taken off the threads:
 //   - warp 0, one lane: the producer. Two tensor-map bulk copies (cp.async.bulk.tensor.2d; every CTA fetches its own tiles) per k-block bring
 //     128 rows of A and 256 rows of B, 128 bytes of k each, into a ring of four 48 KB stages in the 128-byte swizzled
 //     K-major layout; edges and the k tail are zero-filled by the copy engine; completion is counted on the stage's mbarrier;
 //   - warp 1, one lane: the MMA issuer. Four tcgen05.mma.kind::i8 (M 128, N 256, K 32) per stage, the shared-memory
 //     descriptor stepped 32 bytes along k inside the swizzle atom; a tcgen05.commit hands the stage back to the producer and,
 //     after a tile's last k-block, hands the accumulator to the store warps;
-//   - warps 2 to 9: the store (two warps per quarter of the accumulator's lanes, half the columns each). Two accumulators of 256 columns fill the 512 columns of tensor memory, so a tile's conversion
-//     and store (the same turned, coalesced store as gemm_int8_mma_kernel's) run under the next tile's MMAs.
+//   - warps 2 to 9: the store (two warps per quarter of the accumulator's lanes, half the columns each). Two accumulators of 256 columns
+//     fill the 512 columns of tensor memory, so a tile's conversion and store run under the next tile's MMAs.
 // One CTA per SM walks tiles blockIdx.x, blockIdx.x + gridDim.x, ... Every wait is bounded (status 9).
 #pragma once
 #include <cuda.h>
@@ -229,7 +229,7 @@ inline bool t8_make_map(CUtensorMap *map, const void *base, long long rows, long
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Returns false when the tensor maps cannot be made (the caller then takes gemm_int8_mma_kernel).
+// Returns false when the tensor maps cannot be made (the caller then takes gemm_int8_flat_kernel).
 inline bool launch_gemm_int8_tma(float *c, const signed char *qa, const int *ea, const signed char *qb, const int *eb, int m, int n, int k,
                                  int sms, cudaStream_t st) {
     alignas(64) CUtensorMap map_a, map_b;

@@ -121,6 +121,22 @@ def test_int8_products_on_sm_pairs(m, n, k):
     assert _native.lib().b200i_decode_status(-1) == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(1100, 17000, 144), (1030, 17003, 16), (40, 151600, 1008), (2056, 8960, 512)])
+def test_int8_products_with_a_short_contraction(m, n, k):
+    """One CTA a tile: at least four 128 x 256 tiles per SM and k below 1024; whole and ragged rows of 16-byte stores, exponents
+    inside and outside the short conversion's range."""
+    assert -(-m // 128) * -(-n // 256) >= 4 * torch.cuda.get_device_properties(0).multi_processor_count and k < 1024
+    rng = np.random.default_rng(n)
+    qa, qb = rng.integers(-127, 128, (m, k)).astype(np.int8), rng.integers(-127, 128, (n, k)).astype(np.int8)
+    ea, eb = rng.integers(-60, 30, m).astype(np.int32), rng.integers(-60, 30, n).astype(np.int32)
+    eb[n // 2 :] += 40
+    got = torch_ops.matmul_int8(*(torch.from_numpy(t).cuda() for t in (qa, ea, qb, eb))).cpu().numpy()
+    rows = np.unique(np.r_[0, 31, 127, 128, m - 1, rng.integers(0, m, 12)] % m)
+    want = oracle.nan_canon(oracle.gemm_int8(np.ascontiguousarray(qa[rows]), ea[rows], qb, eb))
+    assert got[rows].tobytes() == want.tobytes()
+    assert _native.lib().b200i_decode_status(-1) == 0
+
+
 @pytest.mark.parametrize("m,n,k,opname", [(96, 2304, 1500, "NT"), (1100, 1000, 1030, "NN"), (40, 1500, 3000, "NN"), (2000, 70, 900, "TN")])
 def test_host_arrays_through_the_copy_threads(m, n, k, opname):
     """Megabytes of pageable arrays: both ways of cutting the product, and the plain path."""
