@@ -166,3 +166,98 @@ def test_gated_activation_layouts_agree():
                          5, 72, 144, kind, 1)
             outs.append(out.view(torch.int32))
         assert torch.equal(*outs)
+
+
+ACTS = [torch_ops.ACT_NONE, torch_ops.ACT_GELU_ERF, torch_ops.ACT_SILU]
+
+
+@pytest.mark.parametrize("m", [9, 16, 17, 32])
+@pytest.mark.parametrize("n,k", [(1001, 144), (770, 2064), (516, 1040)])
+def test_band_plan_store_epilogues(m, n, k):
+    """Bias, activations and (whole quads of columns) gated stores, in the kernel's own store and in the fold of its groups."""
+    rng = np.random.default_rng(m + n + k)
+    a, w = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda(), torch.from_numpy(rng.standard_normal((n, k)).astype(np.float32)).cuda()
+    bias = torch.from_numpy(rng.standard_normal(n).astype(np.float32)).cuda()
+    for act in ACTS + ([torch_ops.ACT_PAIR_SWIGLU, torch_ops.ACT_PAIR_GEGLU_TANH] if n % 4 == 0 else []):
+        want = torch_ops.product(a, w, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_SKINNY, bias=bias, act=act)
+        for gl in (0, 4):
+            if gl < oracle.leaf_count(k):
+                got = torch_ops.product(a, w, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_BAND, group_leaves=gl, bias=bias, act=act)
+                assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (act, gl)
+
+
+@pytest.mark.parametrize("m,n,k", [(33, 40, 20000), (27, 5, 140000)])
+def test_tall_plan_store_epilogues(m, n, k):
+    """Both depths of the node fold (up to 256 nodes, and more), which is where the tall plan applies them."""
+    rng = np.random.default_rng(k)
+    a, b = torch.from_numpy(rng.standard_normal((k, m)).astype(np.float32)).cuda(), torch.from_numpy(rng.standard_normal((k, n)).astype(np.float32)).cuda()
+    bias = torch.from_numpy(rng.standard_normal(n).astype(np.float32)).cuda()
+    for act in ACTS:
+        got, want = (torch_ops.product(a, b, op=linalg.OP_TN, plan=p, bias=bias, act=act) for p in (torch_ops.PLAN_TALL, torch_ops.PLAN_FLAT))
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32)), act
+
+
+@pytest.mark.parametrize("m", [9, 16, 17, 32])
+def test_band_plan_by_the_rule(m):
+    """Just above ten million float32 weights, ragged columns: the automatic split and its workspace."""
+    n, k = 4901, 2048
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert _native.lib().b200i_auto_plan(m, n, k, linalg.OP_NT, linalg.W_F32, sms, -1, None) == torch_ops.PLAN_BAND
+    rng = np.random.default_rng(m)
+    a, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    a[m - 1, k // 3], w[n - 1, 5] = 1e-41, 3e-39
+    rows = np.unique([0, m // 2, m - 1])
+    want = oracle.nan_canon(oracle.gemm_rows(np.ascontiguousarray(a[rows]), w, oracle.OP_NT))
+    got = torch_ops.matmul(torch.from_numpy(a).cuda(), torch.from_numpy(w).cuda(), transpose_b=True).cpu().numpy()
+    assert got[rows].tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("kind", [linalg.W_F32, linalg.W_INT8_EXP])
+def test_rows_plan_with_many_columns_and_several_leaf_groups(kind):
+    """Hundreds of columns in a CTA beside five groups of eight leaves, the last one ragged."""
+    m, n, k = 7, 30001, 4112
+    rng = np.random.default_rng(kind)
+    w, scale, dense = _weight(rng, n, k, kind)
+    a = rng.standard_normal((m, k)).astype(np.float32)
+    want = oracle.nan_canon(oracle.gemm_rows(a, dense, oracle.OP_NT))
+    ds = torch.from_numpy(scale).cuda() if scale is not None else None
+    got = torch_ops.product(torch.from_numpy(a).cuda(), torch.from_numpy(w).cuda(), ds, kind, linalg.OP_NT, plan=torch_ops.PLAN_ROWS, group_leaves=8)
+    assert _same(got, want)
+
+
+SPECIALS = [1e-41, -3e-39, 2.0**-64, -(2.0**-63), np.inf, np.nan]
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 300, 1044), (37, 130, 396), (1, 129, 20), (65, 256, 2048)])
+def test_packed_plan_reading_b_in_place_takes_the_flushed_step_where_a_word_needs_it(m, n, k):
+    """One row of tiles over float32 rows of whole quads: words that fail admission only in B (first, a middle and the last
+    stage of 32 steps), only in A, and in both; ragged last stages, split and unsplit."""
+    rng = np.random.default_rng(m + n + k)
+    a0, b0 = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    a0[m - 1] *= np.float32(2.0**-70)  # products that a bare step would leave subnormal
+    places = [0, (k // 2) // 32 * 32 + 7, k - 1]
+    for where in ("b", "a", "both"):
+        for p in (places if where == "b" else [places[1]]):
+            a, b = a0.copy(), b0.copy()
+            for i, v in enumerate(SPECIALS):
+                if where != "a":
+                    b[(i * 37 + 3) % n, min(p + (i & 3) if p + 3 < k else p - (i & 3), k - 1)] = v
+                if where != "b":
+                    a[(i * 11) % m, (p + i) % k] = v
+            want = oracle.nan_canon(oracle.gemm_rows(a, b, oracle.OP_NT))
+            da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+            for gl in (0, 2):
+                if gl < oracle.leaf_count(k):
+                    got = torch_ops.product(da, db, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_PACKED, group_leaves=gl)
+                    assert _same(got, want), (where, p, gl)
+
+
+@pytest.mark.parametrize("m", [2176, 2500, 3970])
+def test_packed_plan_walks_a_whole_band_of_tiles_and_a_part_of_one(m):
+    """17, 20 and 32 rows of tiles: bands of sixteen, the last one short or whole."""
+    n, k = 300, 200
+    rng = np.random.default_rng(m)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    want = oracle.nan_canon(oracle.gemm_rows(a, b, oracle.OP_NN))
+    got = torch_ops.product(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), op=linalg.OP_NN, plan=torch_ops.PLAN_PACKED)
+    assert _same(got, want)
