@@ -9,21 +9,28 @@
 // have left) its stream. Workers live for one call: nothing runs between calls, no descriptor is inherited by a fork.
 // The pinned buffers (16 MB) are kept with the device's pool under the pool's lock. A worker that cannot be started, and
 // a piece whose transfer fails, is reported by finish(); fewer workers than asked for do the same work.
+//
+// Nobody spins for long: a worker without a segment, and the caller that waits for one, sleep on a condition variable after
+// HC_SPIN_US, and the workers of a device-to-host segment sleep on an event of the work before it (a product may run for
+// much longer than its copies). Only the wait for a piece's own transfer is the driver's usual one.
 #pragma once
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <chrono>
+#include <condition_variable>
 #include <cstring>
+#include <mutex>
 #include <thread>
 
 namespace b200i {
 
 constexpr size_t HC_PIECE = 1u << 20;
-constexpr int HC_WORKERS = 8, HC_SEGMENTS = 24;
+constexpr int HC_WORKERS = 8, HC_SEGMENTS = 24, HC_SPIN_US = 2000;
 
-struct HostStage { // per device, kept: two pinned pieces and their events per worker
+struct HostStage { // per device, kept: two pinned pieces and their events per worker, and an event per segment to sleep on
     unsigned char *pinned = nullptr;
-    cudaEvent_t ev[2 * HC_WORKERS] = {};
+    cudaEvent_t ev[2 * HC_WORKERS] = {}, before[HC_SEGMENTS] = {};
     bool ready = false;
 };
 
@@ -36,6 +43,8 @@ inline cudaError_t host_stage_prepare(HostStage &s) {
     }
     for (auto &x : s.ev)
         if (!x && (e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming)) != cudaSuccess) return e;
+    for (auto &x : s.before)
+        if (!x && (e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming | cudaEventBlockingSync)) != cudaSuccess) return e;
     s.ready = true;
     return cudaSuccess;
 }
@@ -76,7 +85,7 @@ class HostCopier {
     int add(bool to_device, void *device, void *host, size_t width, size_t pitch, size_t rows, cudaStream_t st) {
         const int i = published_.load(std::memory_order_relaxed);
         if (i >= HC_SEGMENTS) { // never more than the caller's chunks; refused rather than overrun
-            failed_.store((int)cudaErrorInvalidValue);
+            fail(cudaErrorInvalidValue);
             return -1;
         }
         Segment &s = seg_[i];
@@ -96,21 +105,51 @@ class HostCopier {
         s.stream = st;
         s.next.store(0);
         s.done.store(0);
+        if (!to_device) { // what the stream holds now, the product among it, comes before this segment
+            const cudaError_t e = cudaEventRecord(stage_.before[i], st);
+            if (e != cudaSuccess) {
+                fail(e);
+                return -1;
+            }
+        }
         published_.store(i + 1, std::memory_order_release);
+        wake(more_);
         return i;
     }
     void wait(int i) { // all pieces of segment i are queued (to the device) or home (from it)
         if (i < 0) return;
-        while (seg_[i].done.load(std::memory_order_acquire) < seg_[i].pieces && failed_.load() == 0) std::this_thread::yield();
+        sleep_until(whole_, [&] { return seg_[i].done.load(std::memory_order_acquire) >= seg_[i].pieces || failed_.load() != 0; });
     }
     cudaError_t finish() {
         closed_.store(true, std::memory_order_release);
+        wake(more_);
         for (int i = 0; i < started_; i++)
             if (workers_[i].joinable()) workers_[i].join();
         return (cudaError_t)failed_.load();
     }
 
   private:
+    void wake(std::condition_variable &cv) { // after the change itself: a sleeper that missed it holds the mutex until it sleeps
+        { std::lock_guard<std::mutex> lock(mu_); }
+        cv.notify_all();
+    }
+    void fail(cudaError_t e) {
+        failed_.store((int)e);
+        wake(more_);
+        wake(whole_);
+    }
+    template <class Ready>
+    void sleep_until(std::condition_variable &cv, Ready ready) {
+        const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(HC_SPIN_US);
+        while (!ready()) {
+            if (std::chrono::steady_clock::now() >= until) {
+                std::unique_lock<std::mutex> lock(mu_);
+                cv.wait(lock, ready);
+                return;
+            }
+            std::this_thread::yield();
+        }
+    }
     struct Segment {
         bool to_device;
         unsigned char *device, *host;
@@ -118,6 +157,15 @@ class HostCopier {
         cudaStream_t stream;
         std::atomic<size_t> next{0}, done{0};
     };
+    static cudaError_t past(cudaEvent_t ev) { // the work before the event is over
+        const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(HC_SPIN_US);
+        for (;;) {
+            const cudaError_t e = cudaEventQuery(ev);
+            if (e != cudaErrorNotReady) return e;
+            if (std::chrono::steady_clock::now() >= until) return cudaEventSynchronize(ev);
+            std::this_thread::yield();
+        }
+    }
     void piece(Segment &s, size_t i, int slot) {
         unsigned char *buf = stage_.pinned + (size_t)slot * HC_PIECE;
         cudaEvent_t ev = stage_.ev[slot];
@@ -140,16 +188,17 @@ class HostCopier {
         } else if (e == cudaSuccess) {
             e = cudaMemcpyAsync(buf, dp, count * len, cudaMemcpyDeviceToHost, s.stream);
             if (e == cudaSuccess) e = cudaEventRecord(ev, s.stream);
+            if (e == cudaSuccess) e = past(stage_.before[&s - seg_]); // the transfer is queued, and sleeps behind the product
             if (e == cudaSuccess) e = cudaEventSynchronize(ev);
             if (e == cudaSuccess)
                 for (size_t r = 0; r < count; r++) std::memcpy(hp + r * s.pitch, buf + r * len, len);
         }
-        if (e != cudaSuccess) failed_.store((int)e);
+        if (e != cudaSuccess) fail(e);
     }
     void work(int id) {
         cudaError_t e = cudaSetDevice(dev_);
         if (e != cudaSuccess) {
-            failed_.store((int)e);
+            fail(e);
             return;
         }
         int turn = 0;
@@ -157,7 +206,7 @@ class HostCopier {
             if (failed_.load() != 0) return;
             if (i >= published_.load(std::memory_order_acquire)) {
                 if (closed_.load(std::memory_order_acquire) && i >= published_.load(std::memory_order_acquire)) return;
-                std::this_thread::yield();
+                sleep_until(more_, [&] { return i < published_.load(std::memory_order_acquire) || closed_.load(std::memory_order_acquire) || failed_.load() != 0; });
                 continue;
             }
             Segment &s = seg_[i];
@@ -167,13 +216,15 @@ class HostCopier {
                 continue;
             }
             piece(s, p, 2 * id + (turn ^= 1));
-            s.done.fetch_add(1, std::memory_order_release);
+            if (s.done.fetch_add(1, std::memory_order_acq_rel) + 1 == s.pieces) wake(whole_);
         }
     }
     HostStage &stage_;
     int dev_, started_ = 0;
     std::thread workers_[HC_WORKERS];
     Segment seg_[HC_SEGMENTS];
+    std::mutex mu_;
+    std::condition_variable more_, whole_; // segments to take; a segment done
     std::atomic<int> published_{0}, failed_{0};
     std::atomic<bool> closed_{false};
 };
