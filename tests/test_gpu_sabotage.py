@@ -88,3 +88,23 @@ def test_admit_always_build_fails_the_subnormal_forcing_cases():
         assert not bad["plans"][plan], "plan %s passed the subnormal-forcing product with admission sabotaged" % plan
     assert not bad["skinny_int8"], "the register skinny plan passed with admission sabotaged"
     assert not bad["attention"], "the subnormal-forcing attention call passed with admission sabotaged"
+
+
+SPLIT_CHILD = r"""
+import json, sys
+sys.path[:0] = [%(root)r, %(root)r + "/tests"]
+import test_gpu_split_paths as t
+print("RESULT " + json.dumps({name: t._same(run(), want) for name, run, want in t.forcing_cases()}))
+"""
+
+
+def test_admit_always_build_fails_every_forcing_case_of_the_split_paths():
+    """One forcing window in one operand, on the rows, band and tall plans and the packed plan that reads B in place."""
+    from mojolearn_b200.csrc import build as cuda_build
+    run = subprocess.run([sys.executable, "-c", SPLIT_CHILD % {"root": ROOT}], env=dict(os.environ, MOJOLEARN_B200_LIB=cuda_build.build(sabotage=True)),
+                         capture_output=True, text=True, timeout=600)
+    assert run.returncode == 0, run.stderr[-3000:]
+    line = [ln for ln in run.stdout.splitlines() if ln.startswith("RESULT ")][-1]
+    right = json.loads(line[len("RESULT "):])
+    whole = {name: ok for name, ok in right.items() if "ragged" not in name}
+    assert len(whole) > 100 and not any(whole.values()), [name for name, ok in whole.items() if ok]

@@ -229,27 +229,78 @@ SPECIALS = [1e-41, -3e-39, 2.0**-64, -(2.0**-63), np.inf, np.nan]
 
 
 @pytest.mark.parametrize("m,n,k", [(128, 300, 1044), (37, 130, 396), (1, 129, 20), (65, 256, 2048)])
-def test_packed_plan_reading_b_in_place_takes_the_flushed_step_where_a_word_needs_it(m, n, k):
-    """One row of tiles over float32 rows of whole quads: words that fail admission only in B (first, a middle and the last
-    stage of 32 steps), only in A, and in both; ragged last stages, split and unsplit."""
+def test_packed_plan_reading_b_in_place(m, n, k):
+    """One row of tiles over float32 rows of whole quads, ragged last stages, split and unsplit: subnormal, tiny and non-finite
+    words in the first, a middle and the last stage of 32 steps."""
     rng = np.random.default_rng(m + n + k)
-    a0, b0 = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
-    a0[m - 1] *= np.float32(2.0**-70)  # products that a bare step would leave subnormal
-    places = [0, (k // 2) // 32 * 32 + 7, k - 1]
-    for where in ("b", "a", "both"):
-        for p in (places if where == "b" else [places[1]]):
-            a, b = a0.copy(), b0.copy()
-            for i, v in enumerate(SPECIALS):
-                if where != "a":
-                    b[(i * 37 + 3) % n, min(p + (i & 3) if p + 3 < k else p - (i & 3), k - 1)] = v
-                if where != "b":
-                    a[(i * 11) % m, (p + i) % k] = v
-            want = oracle.nan_canon(oracle.gemm_rows(a, b, oracle.OP_NT))
-            da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
-            for gl in (0, 2):
-                if gl < oracle.leaf_count(k):
-                    got = torch_ops.product(da, db, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_PACKED, group_leaves=gl)
-                    assert _same(got, want), (where, p, gl)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    for p in (0, (k // 2) // 32 * 32 + 7, k - 4):
+        for i, v in enumerate(SPECIALS):
+            b[(i * 37 + p) % n, p + (i & 3)] = v
+            a[(i * 11) % m, p + (i & 3)] = SPECIALS[i - 1] if i < 4 else v
+    want = oracle.nan_canon(oracle.gemm_rows(a, b, oracle.OP_NT))
+    da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    for gl in (0, 2):
+        if gl < oracle.leaf_count(k):
+            assert _same(torch_ops.product(da, db, None, linalg.W_F32, linalg.OP_NT, plan=torch_ops.PLAN_PACKED, group_leaves=gl), want), gl
+
+
+def forcing_cases():
+    """(name, product, oracle's words): products with ONE window in which bare steps give another word than flushed ones, the words
+    that force it in the weight only, in the activations only, or in both; in the first, a middle and the last window.
+    The last row is zero but for two steps, whose products are 2^-127 (flushed away) and 2^-126. `ragged` in a name: the steps lie
+    in a window that is not whole, which every kernel walks flushed."""
+    def build(m, n, k, where, p, exps=False):
+        rng = np.random.default_rng(m * 7 + n + k + p)
+        a, w = rng.standard_normal((m, k)).astype(np.float32), rng.integers(-127, 128, (n, k)).astype(np.float32) / 64
+        a[m - 1] = 0.0
+        small, large = {"w": (2.0**-120, 2.0**-7), "a": (2.0**-120, 2.0**-7), "both": (2.0**-64, 2.0**-63)}[where]
+        if where == "w":
+            a[m - 1, p], a[m - 1, p + 1], w[n - 1, p], w[n - 1, p + 1] = large, 2 * large, small, small
+        else:
+            a[m - 1, p], a[m - 1, p + 1], w[n - 1, p], w[n - 1, p + 1] = small, small, large, 2 * large
+        e = np.full(n, -6, np.int32)
+        if exps:  # a row of codes has one exponent: the whole column is as small as its two words
+            e[n - 1] = int(np.log2(small if where == "w" else large))
+            w[n - 1] = np.where(np.arange(k) < p, 3, 5) * np.exp2(e[n - 1].astype(np.float64))
+            w[n - 1, p] = np.exp2(float(e[n - 1]))
+            w[n - 1, p + 1] = w[n - 1, p] * (1 if where == "w" else 2)
+        return a, w, e
+
+    def case(name, a, w, e, kind, op, plan, gl):
+        stored, scale = w, None
+        if kind == linalg.W_BF16:
+            stored = oracle.to_bf16(w)
+        elif kind in (linalg.W_INT8_EXP, linalg.W_INT8_SCALE):
+            stored = np.rint(w / np.exp2(e.astype(np.float64))[:, None]).astype(np.int8)
+            scale = e if kind == linalg.W_INT8_EXP else np.exp2(e.astype(np.float64)).astype(np.float32)
+        want = oracle.nan_canon(oracle.gemm_rows(a, w, op))
+
+        def run():
+            up = lambda t: torch.from_numpy(t).cuda() if t is not None else None  # noqa: E731
+            return torch_ops.product(up(a), up(stored), up(scale), kind, op, plan=plan, group_leaves=gl)
+        return name, run, want
+
+    for where in ("w", "a", "both"):
+        for m, n, k, plan, gls in ((128, 300, 1044, torch_ops.PLAN_PACKED, (0, 2)), (37, 130, 396, torch_ops.PLAN_PACKED, (0,)), (16, 770, 784, torch_ops.PLAN_BAND, (0, 4)),
+                                   (32, 300, 528, torch_ops.PLAN_BAND, (0,)), (8, 305, 784, torch_ops.PLAN_ROWS, (0, 4)), (16, 40, 256, torch_ops.PLAN_ROWS, (0,))):
+            kinds = [linalg.W_F32, linalg.W_BF16, linalg.W_INT8_EXP, linalg.W_INT8_SCALE] if plan == torch_ops.PLAN_ROWS else [linalg.W_F32]
+            for p in (0, k // 2 + 3, k // 32 * 32 - 2, k - 2):
+                for kind in kinds:
+                    a, w, e = build(m, n, k, where, p, kind in (linalg.W_INT8_EXP, linalg.W_INT8_SCALE))
+                    for gl in gls:
+                        ragged = " ragged" if p == k - 2 and k % 32 else ""
+                        yield case("%s %s %s %s %s%s" % (plan, (m, n, k, gl), where, p, kind, ragged), a, w, e, kind, linalg.OP_NT, plan, gl)
+        for m, n, k in ((32, 64, 2100), (27, 33, 20001)):
+            for p in (0, k // 2 + 3, k // 128 * 128 - 19, k - 2):
+                a, w, e = build(m, n, k, where, p)
+                yield case("tall %s %s %s%s" % ((m, n, k), where, p, " ragged" if p == k - 2 else ""), np.ascontiguousarray(a.T), np.ascontiguousarray(w.T), e, linalg.W_F32, linalg.OP_TN,
+                           torch_ops.PLAN_TALL, 0)
+
+
+def test_windows_that_need_the_flushed_step_get_it():
+    for name, run, want in forcing_cases():
+        assert _same(run(), want), name
 
 
 @pytest.mark.parametrize("m", [2176, 2500, 3970])
