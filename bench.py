@@ -44,7 +44,7 @@ DECODE_N, DECODE_K = 11008, 4096
 CONFIG1 = (1024, 1024, 1024)
 # DRAM bytes of one launch from the committed ncu captures (profiles/): the bench cannot read counters itself
 DECODE_INT8_M1_DRAM_BYTES = 45202944  # profiles/decode_pair_kernel_int8_m1_11008x4096.md
-PACKED_4096_DRAM_BYTES = 1060e6 + 940.4e6  # dram__bytes_read + dram__bytes_write of one 4096-cubed launch (profiles/gemm_packed_kernel_4096cubed.md)
+PACKED_4096_DRAM_BYTES = 438.0e6 + 273.4e6  # dram__bytes_read + dram__bytes_write of one 4096-cubed launch (profiles/gemm_packed_kernel_4096cubed.md)
 
 
 def sweep_flops(shapes):
@@ -358,7 +358,7 @@ def main():
         i8_ms.append(e0.elapsed_time(e1))
     i8_us = statistics.median(i8_ms) * 1e3
     i8_tops = 2.0 * 4096 ** 3 / (i8_us * 1e-6) / 1e12
-    int8_product = {"kernel": "gemm_int8_tma_kernel (tensor-map copies, tcgen05.mma kind::i8, two int32 accumulators in tensor memory)", "shape": [4096, 4096, 4096],
+    int8_product = {"kernel": "gemm_int8_pair_kernel (SM pairs: tensor-map copies, tcgen05.mma.cta_group::2 kind::i8, two int32 accumulators in tensor memory)", "shape": [4096, 4096, 4096],
                     "us": i8_us, "tops": i8_tops, "bound": "tensor", "peak": 4500.0, "unit": "TOP/s", "frac": i8_tops / 4500.0,
                     "peak_source": "nominal dense int8 rate of the part (twice the nominal bf16 rate; no measured int8 figure exists)",
                     "l2": "a 160 MB buffer is written between timed launches", "launches_timed": 10,

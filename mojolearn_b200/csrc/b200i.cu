@@ -100,10 +100,11 @@ int64_t check_wait_status(char *err, int64_t err_cap, const char *who) {
 // ---- plans -----------------------------------------------------------------------------
 enum { PLAN_AUTO = -1, PLAN_FLAT = 0, PLAN_T128 = 1, PLAN_T64 = 2, PLAN_DECODE = 3, PLAN_T32 = 4, PLAN_T128X64 = 5, PLAN_SKINNY = 6, PLAN_PACKED = 7, PLAN_TALL = 8, PLAN_ROWS = 9, PLAN_BAND = 10 };
 
-// Up to this many rows the weight-streaming decode plan wins; above, the skinny plan. Low-bit weights
-// switch earlier: at three and four rows the decode kernel's serial chains cost more than the register
-// skinny kernel's eight-row tile (int8 [11008, 4096]: 44 us against 37 us at four rows, 40 against 36 at
-// three), except on a very wide weight, where the decode kernel's row streams run at their best
+// Up to this many rows the weight-streaming decode plan is preferred to the skinny plan; float32 weights at four rows then take
+// the rows plan where their call's workspace holds its nodes (rows_preferred: [11008, 4096] 55 us). Low-bit weights switch
+// earlier unless the leaf-pair kernel fits (up to four rows): at three and four rows decode_kernel's serial chains cost more
+// than the register skinny kernel's eight-row tile (int8 [11008, 4096]: 44 us against 37 us at four rows, 40 against 36 at
+// three), except on a very wide weight, where its row streams run at their best
 // ([50304, 2048]: bf16 79 us against 98 at four rows, int8 60 against 69 at three).
 constexpr int DECODE_PREFER_M = 4;
 constexpr long long DECODE_WIDE_N = 32768;
