@@ -263,27 +263,71 @@ Plan choose_rows(long long k) {
     while ((leaves + run - 1) / run > MAX_GROUPS) run *= 2;
     return Plan{PLAN_ROWS, run, (leaves + run - 1) / run};
 }
-// Where it wins (graph replay, folds included): float32 at 4 to 8 rows ([2304, 768] 6.5 against 14 us, [768, 3072] 8.6 against
-// 13.9, [50304, 768] 54 against 66, [11008, 4096] 57 against 80); low-bit weights while they are small enough to be bound by
-// latency, int8 ones also where they are deep (int8 [2304, 768] 5.3 against 9.4, [768, 3072] 7.3 against 8.9, [4096, 8192] 29
-// against 31, but [6144, 2048] 17.2 against 15.8 and bf16 [11008, 4096] no faster), and not at four rows where the leaf-pair kernel streams a large weight; 9 to 16 rows while
-// a CTA has one strip of sixteen columns (float32 [2304, 768] 8.9 against 16, [768, 3072] 11.5 against 15.8, but [3072, 768]
-// 16.4 against 15.7).
-inline bool rows_preferred(long long m, long long n, long long k, int wkind, int sms) {
-    RowsLaunch held;
-    if (m < 4 || !rows_layout(m, n, k, wkind, choose_rows(k).group_leaves, sms, held)) return false;
-    if (m <= 8) return wkind == W_F32 || n <= 3072 || (wkind != W_BF16 && m > 4 && k >= 4096);
-    return n <= 16ll * sms && (wkind == W_F32 || k <= 1024);
+// Modelled microseconds of a rows launch, its fold included: what a warp walks one leaf after the other at the rate of its strip
+// shape, slower while more than eight warps share the SM, plus staging and start. Fitted to 6600 launches of 300 to 50304
+// columns by 768 to 8192 steps (nine in ten within 10 %; ragged depths and strips are where the plan's time jumps).
+double rows_us(const RowsLaunch &r, long long m, long long n, int wkind) {
+    static const double leaf_us[3][5][2] = { // [float32, bf16, int8][8 rows: 8 or 16, 32, 64 columns; 16 rows: 8 or 16, 32][to 8 warps, at 16]
+        {{2.2, 4.2}, {4.9, 8.8}, {10.2, 13.2}, {4.0, 6.7}, {12.4, 16.4}},
+        {{1.8, 3.4}, {3.6, 7.1}, {7.5, 10.7}, {3.3, 5.5}, {9.6, 14.1}},
+        {{1.3, 2.6}, {2.7, 5.6}, {5.4, 7.7}, {2.6, 4.8}, {5.8, 10.6}}};
+    const int columns = r.lc * r.cpl, shape = (columns <= 16 ? 0 : (columns == 32 ? 1 : 2)) + (m <= 8 ? 0 : 3);
+    const double *rate = leaf_us[wkind == W_F32 ? 0 : (wkind == W_BF16 ? 1 : 2)][shape];
+    const double crowd = std::max(0, r.p.warps - 8) / 8.0;
+    double t = 2.95 + 0.72 * r.act_bytes / 32768.0 + r.rounds * (rate[0] + (rate[1] - rate[0]) * crowd);
+    if (r.groups > 1) t += 2.4 + (double)r.groups * m * n * 8.0 / 7.5e6;
+    return t;
+}
+// The same for the plan that the call would take otherwise (`before`: decode or skinny), fitted to the same sizes.
+double before_rows_us(const Plan &before, long long m, long long n, long long k, int wkind, int sms) {
+    const double words = (double)n * k / 1e6, steps = k / 1000.0;
+    if (before.kind == PLAN_DECODE && wkind == W_F32) { // a warp walks 32 rows: to 32 rows an SM, to 64, above
+        if (n <= 32ll * sms) return 3.6 + 3.73 * steps + 0.6 * words + 0.27 * n / 1000.0;
+        return n <= 64ll * sms ? 4.3 + 6.0 * steps + 0.74 * words : 4.5 + 3.5 * steps + 1.27 * words;
+    }
+    if (before.kind == PLAN_DECODE) { // the leaf-pair kernel, eight leaves of a row at a time (bf16 past 2048 and int8 past 4096
+        const double turns = (double)((k + 1023) / 1024); // steps: more than one copy a row, too short a ring)
+        return wkind == W_BF16 ? 4.6 + 1.8 * turns + 0.56 * words + (k > 2048 ? 2.0 : 0.0) : 5.4 + (1.78 * turns + 0.28 * words) * (k > 4096 ? 1.5 : 1.0);
+    }
+    // leaves that an SM walks, a few CTAs beyond a whole number per SM not showing; a CTA alone takes longer over its own
+    const long long ctas = (n + 255) / 256 * before.groups - sms / 20;
+    const int own = std::min(before.group_leaves, (int)leaf_count(k));
+    const double walk = (double)std::max<long long>((ctas + sms - 1) / sms, 1) * own;
+    if (wkind == W_F32)
+        return m <= 8 ? 9.1 + std::max(4.08 * walk, 9.5 * own - 5.0) + 0.68 * words : 8.7 + std::max(6.4 * walk, 12.0 * own - 6.0) + 0.59 * words;
+    return wkind == W_BF16 ? 6.2 + std::max(2.38 * walk, 5.2 * own - 3.0) + 0.3 * words : 6.1 + std::max(2.34 * walk, 4.4 * own - 2.5) + 0.135 * words;
+}
+// Float32 weights at 4 to 8 rows and, while a CTA has one strip of sixteen columns, at 9 to 16; int8 ones at 4 rows to 3072
+// columns, at 5 to 8 rows also where they are deep; bf16 ones to 3072 columns; low-bit ones at 9 to 16 rows while small enough to
+// be bound by latency. Inside these lines the modelled times decide: float32 [2304, 768] at eight rows 6.5 against 14 us,
+// [11008, 4096] 57 against 80, but [32000, 1792] 138 against 96 and [1536, 6160] 28 against 21 (a strip of 64 columns for ten).
+inline bool rows_preferred(const Plan &before, long long m, long long n, long long k, int wkind, int sms) {
+    RowsLaunch r;
+    if (m < 4 || !rows_layout(m, n, k, wkind, choose_rows(k).group_leaves, sms, r)) return false;
+    if (m > 8 && (n > 16ll * sms || (wkind != W_F32 && k > 1024))) return false;
+    if (m <= 8 && wkind != W_F32 && n > 3072 && (wkind == W_BF16 || m <= 4 || k < 4096)) return false;
+    if (m > 8 && wkind != W_F32) return true;
+    if (before.kind != PLAN_DECODE && before.kind != PLAN_SKINNY) return true;
+    return rows_us(r, m, n, wkind) < before_rows_us(before, m, n, k, wkind, sms);
 }
 
-// 9 to 32 rows: the leaf split of the band kernel. Modelled time in microseconds: waves of CTAs over two slots per SM
-// (leaves per CTA at the kernel's rate, a last wave that fills at most half the slots counting 0.55 because its CTAs are
-// alone on their SMs, + 1 us to start), plus the second launch and the L2-resident node traffic of the fold.
+// 9 to 16 rows: modelled microseconds of the band kernel (fitted like rows_us, within 5 % from two million words up). Up to one CTA
+// an SM a leaf takes 8.4 us, above that two share an SM and every round of 2 * SMs takes 13 a leaf, however few CTAs the last
+// one has (they start beside the others). Ragged groups count by their leaves.
+double band_us(long long m, long long n, long long k, int group_leaves, int sms) {
+    const int leaves = (int)leaf_count(k), sl = std::min(group_leaves, leaves), groups = (leaves + sl - 1) / sl;
+    const long long ctas = ((n + BD_BN - 1) / BD_BN * leaves + sl - 1) / sl;
+    double t = 2.9 + (ctas <= sms ? 2.0 + 8.37 * sl : (double)((ctas + 2 * sms - 1) / (2 * sms)) * (2.73 + 13.0 * sl));
+    if (groups > 1) t += 2.1 + (double)groups * m * n * 8.0 / 7.5e6;
+    return t;
+}
+// 9 to 32 rows: the leaf split of the band kernel. Modelled time in microseconds: band_us up to sixteen rows; above, waves of
+// CTAs over two slots per SM (leaves per CTA at the kernel's rate, a last wave that fills at most half the slots counting 0.55
+// because its CTAs are alone on their SMs, + 1 us to start), plus the second launch and the L2-resident node traffic of the fold.
 Plan choose_band(long long m, long long n, long long k, int sms) {
     const int leaves = (int)leaf_count(k) > 0 ? (int)leaf_count(k) : 1;
     const int max_s = pow2_floor(leaves) * ((leaves & (leaves - 1)) ? 2 : 1);
     const long long tiles = (n + BD_BN - 1) / BD_BN, slots = 2ll * sms;
-    const double leaf_us = m <= 16 ? 5.5 : 9.5;
     int min_s = 1;
     while ((leaves + min_s - 1) / min_s > MAX_GROUPS) min_s *= 2;
     int best = max_s;
@@ -292,16 +336,21 @@ Plan choose_band(long long m, long long n, long long k, int sms) {
         const int groups = (leaves + sl - 1) / sl;
         const long long ctas = tiles * groups, whole = ctas / slots, rest = ctas % slots;
         const double waves = (double)whole + (rest == 0 ? 0.0 : (2 * rest <= slots ? 0.55 : 1.0));
-        double t = waves * (std::min(sl, leaves) * leaf_us + 1.0);
+        double t = waves * (std::min(sl, leaves) * 9.5 + 1.0);
         if (groups > 1) t += 2.5 + (double)groups * m * n * 8.0 / 7.5e6;
+        if (m <= 16) t = band_us(m, n, k, sl, sms);
         if (t < best_t) { best_t = t; best = sl; }
     }
     Plan p{PLAN_BAND, best, (leaves + best - 1) / best};
     if (p.groups <= 1) p.group_leaves = leaves;
     return p;
 }
-// Float32 weights from ten million words up (the sizes on both sides of the line stand in gemm_band.cuh).
-inline bool band_preferred(long long n, long long k, int wkind) { return wkind == W_F32 && (double)n * (double)k >= 1.0e7; }
+// Float32 weights from ten million words up (the sizes on both sides of the line stand in gemm_band.cuh); up to sixteen rows also
+// by the modelled times ([8192, 1792] 35 against 41 us, but [5120, 4096] 55 against 51).
+inline bool band_size(long long n, long long k, int wkind) { return wkind == W_F32 && (double)n * (double)k >= 1.0e7; }
+inline bool band_preferred(const Plan &skinny, const Plan &band, long long m, long long n, long long k, int sms) {
+    return m > 16 || band_us(m, n, k, band.group_leaves, sms) < 0.97 * before_rows_us(skinny, m, n, k, W_F32, sms);
+}
 
 // A^T B of few cells over many rows: every leaf of every 32 x 32 tile as a warp of its own (gemm_tall.cuh).
 constexpr long long TALL_MIN_LEAVES = 16;
@@ -455,8 +504,12 @@ Plan choose_auto(const AutoCall &x, Fits fits) {
     if (dec && m <= prefer_m && !(skinny && x.pairs)) plan = decode; // (a gated store needs the skinny plan)
     else if (skinny) plan = choose_skinny(m, n, k, x.sms, x.wkind != W_F32);
     else if (dec) plan = decode;
-    if (rows_plan_fits(m, n, k, x.op) && x.al16 && rows_preferred(m, n, k, x.wkind, x.sms)) take(choose_rows(k));
-    if (skinny && m > 8 && band_preferred(n, k, x.wkind)) take(choose_band(m, n, k, x.sms));
+    if (skinny && m > 8 && band_size(n, k, x.wkind)) {
+        const Plan band = choose_band(m, n, k, x.sms);
+        if (band_preferred(plan, band, m, n, k, x.sms)) take(band);
+    } else if (rows_plan_fits(m, n, k, x.op) && x.al16 && rows_preferred(plan, m, n, k, x.wkind, x.sms)) {
+        take(choose_rows(k));
+    }
     if (tall_fits(m, n, k, x.op, x.wkind) && tall_candidate(m, n, k) && !x.nodes && !x.pairs) take(Plan{PLAN_TALL, 1, (int)leaf_count(k)});
     return plan;
 }

@@ -352,7 +352,9 @@ inline int rows_group_leaves(long long m) { return RW_ACT_LIMIT / (rows_mt(m) * 
 
 // A launch of the rows plan: the kernel's strip shape, its plan, and its dynamic shared memory.
 struct RowsLaunch {
-    int lc, cpl, smem;
+    int lc, cpl, smem, groups;
+    int rounds;  // leaves that a CTA's busiest warp walks one after the other
+    int act_bytes;
     RowsPlan p;
 };
 // Lays out a CTA's shared memory; false where it does not hold two stages of a ring for four warps, which is what the kernel's
@@ -391,6 +393,10 @@ inline bool rows_layout(long long m, long long n, long long k, int wkind, int gr
         if (p.stages < 2) continue;
         if (p.stages > 3) p.stages = 3;
         r.smem = p.ring_off + p.warps * p.stages * stage;
+        r.groups = groups;
+        r.act_bytes = (int)act;
+        const int rest = (int)(strips % p.together);
+        r.rounds = (int)std::min<long long>((strips / p.together * ((total + p.warps - 1) / p.warps) + (rest * runs + p.warps - 1) / p.warps) * p.run, 1 << 30);
         return true;
     }
     return false;

@@ -53,7 +53,7 @@ def test_the_rows_plan_always_has_two_stages(kind, sms):
     assert taken > 50
 
 
-@pytest.mark.parametrize("m,n,k,plan", [(8, 220000, 2064, PLAN_ROWS), (4, 400000, 4096, PLAN_ROWS), (14, 178374, 12208, PLAN_BAND), (31, 165405, 1536, PLAN_BAND)])
+@pytest.mark.parametrize("m,n,k,plan", [(8, 220000, 4096, PLAN_ROWS), (4, 400000, 4096, PLAN_ROWS), (14, 178374, 12208, PLAN_BAND), (31, 165405, 1536, PLAN_BAND)])
 def test_a_workspace_that_holds_the_skinny_plan_only_gets_the_skinny_plan(m, n, k, plan):
     """These sizes are unsplit in the skinny plan, which needs no workspace, and split in the plan that the rule prefers."""
     got, leaves = auto_plan(m, n, k)
@@ -80,3 +80,13 @@ def test_workspace_by_op_and_storage():
     assert int(lib.b200i_product_workspace_bytes(128, 128, 131072, OP_TN, W_F32)) == 1024 * 128 * 128 * 4
     for op, kind in ((OP_NN, W_F32), (OP_NT, W_F32), (OP_NT, W_BF16), (OP_TN, W_BF16)):
         assert int(lib.b200i_product_workspace_bytes(128, 128, 131072, op, kind)) <= 64 * 128 * 128 * 4
+
+
+@pytest.mark.parametrize("m,n,k,kind,plan", [
+    (8, 2304, 768, W_F32, PLAN_ROWS), (8, 11008, 4096, W_F32, PLAN_ROWS), (4, 11008, 4096, W_F32, PLAN_ROWS), (8, 2304, 768, W_INT8_EXP, PLAN_ROWS),
+    (8, 11008, 4096, W_INT8_EXP, PLAN_ROWS), (12, 2304, 768, W_F32, PLAN_ROWS), (8, 1536, 6160, W_F32, PLAN_SKINNY), (8, 32000, 1792, W_F32, PLAN_SKINNY),
+    (8, 1536, 6160, W_BF16, PLAN_SKINNY), (8, 1536, 6160, W_INT8_EXP, PLAN_SKINNY), (16, 1536, 6160, W_F32, PLAN_SKINNY), (16, 5120, 4096, W_F32, PLAN_SKINNY),
+    (16, 8192, 1792, W_F32, PLAN_BAND), (16, 16384, 2048, W_F32, PLAN_BAND), (32, 16384, 2048, W_F32, PLAN_BAND)])
+def test_small_batches_take_the_plan_that_measured_faster(m, n, k, kind, plan):
+    """Both sides of the rules' lines: depths whose last group or strip is nearly empty keep the skinny plan."""
+    assert auto_plan(m, n, k, wkind=kind)[0] == plan
