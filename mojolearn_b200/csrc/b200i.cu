@@ -1710,18 +1710,20 @@ int64_t b200i_comm_destroy(void *comm) {
 // ---- host-pointer twins -------------------------------------------------------------------
 
 // The copies of one host-pointer call: through the worker threads for pageable arrays when there are megabytes of them
-// (see host_copy.cuh), else plain asynchronous copies.
-constexpr size_t HOST_STAGED_MIN = 4u << 20;
+// (see host_copy.cuh), else plain asynchronous copies: below 8 MB starting the threads costs what they save (256 x 1024 x 1024
+// 440 us plain, 480 with them), and without a pipeline to overlap, below 16 MB unless one operand has 8 (1000 cubed 755 us
+// plain, 800 to 870 with them; 1 x 4096 x 512 603 against 521).
+constexpr size_t HOST_STAGED_MIN = 8u << 20;
 struct HostTransfers {
     struct Span {
         const void *p;
         size_t bytes;
     };
-    HostTransfers(HostPool &pool, int dev, std::initializer_list<Span> spans) {
+    HostTransfers(HostPool &pool, int dev, size_t least, std::initializer_list<Span> spans) {
         size_t total = 0;
         for (const Span &s : spans)
             if (host_is_pageable(s.p)) total += s.bytes;
-        if (total < HOST_STAGED_MIN) return;
+        if (total < least) return;
         if (host_stage_prepare(pool.stage) != cudaSuccess) {
             cudaGetLastError();
             return;
@@ -1820,7 +1822,7 @@ static int64_t host_gemm_pipelined(int dev, HostPool &pool, float *c, const floa
     CUDA_TRY(cudaStreamWaitEvent(pool.s_in, pool.ev[0], 0));
     CUDA_TRY(cudaStreamWaitEvent(pool.s_out, pool.ev[0], 0));
     // the operand that is not cut crosses first and is packed once
-    HostTransfers io(pool, dev, {{a, abytes}, {b, bbytes}, {c, cbytes}});
+    HostTransfers io(pool, dev, HOST_STAGED_MIN, {{a, abytes}, {b, bbytes}, {c, cbytes}});
     const void *first = by_rows ? b : static_cast<const void *>(a);
     int seg_first = -1, seg_in[HOST_CHUNKS + 1];
     CUDA_TRY(io.to_device(by_rows ? db : da, first, by_rows ? bbytes : abytes, pool.s_in, &seg_first));
@@ -1915,7 +1917,7 @@ int64_t b200i_host_gemm_w(int64_t device, float *c, const float *a, const void *
     CUDA_TRY(pool_get(dev, 2, cbytes, &dc));
     if (sbytes) CUDA_TRY(pool_get(dev, 3, sbytes, &ds));
     if (wsbytes) CUDA_TRY(pool_get(dev, 4, (size_t)wsbytes, &dw));
-    HostTransfers io(pool, dev, {{a, abytes}, {b, bbytes}, {c, cbytes}});
+    HostTransfers io(pool, dev, std::max(abytes, bbytes) >= HOST_STAGED_MIN ? HOST_STAGED_MIN : 2 * HOST_STAGED_MIN, {{a, abytes}, {b, bbytes}, {c, cbytes}});
     int seg_a, seg_b;
     CUDA_TRY(io.to_device(da, a, abytes, pool.stream, &seg_a));
     CUDA_TRY(io.to_device(db, b, bbytes, pool.stream, &seg_b));
