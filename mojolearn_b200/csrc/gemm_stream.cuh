@@ -1,0 +1,335 @@
+// C[m, n] = A[m, k] . W[n, k]^T for a decode batch (5 to 32 rows), any weight storage: warps that walk the weight on their own.
+//
+// The register skinny kernel (gemm_skinny_reg.cuh) reads a weight 16 bytes of 64 rows at a time, which DRAM serves far below its
+// streaming rate, stages activations behind CTA barriers and comes in whole waves of CTAs; it stays at half of the fma pipe at
+// 32 rows and at a third of HBM at eight. Here:
+//
+//   - one CTA per SM, its warps independent after one barrier. The work is cut into items (leaf group, unit of CB columns),
+//     numbered leaf group by leaf group, and every CTA takes an equal run of them, so it meets at most two leaf groups, whose
+//     activations are staged once, [k][MT] with the row quads permuted by k so that the turning stores are free of bank conflicts;
+//   - a warp owns an item and brings its weights itself: one tensor-map copy (cp.async.bulk.tensor.2d, 64 bytes of CB rows,
+//     64-byte swizzle) per stage of its own ring, completion on its own mbarriers, refilled by the warp when it has read a slot.
+//     No other warp is waited for. Edges of the weight and the k tail are zero-filled by the copy engine;
+//   - a lane owns RL rows (MT rows over RG row groups) by CPL columns, the rows in pairs: one 16-byte read of the activations
+//     serves 2 * CPL packed fmas, one 16-byte read of a column serves 4 to 16 k-steps.
+//
+// Admission is per leaf and lane: the activations' keys are taken while they are staged, the weights' while they are widened
+// (bf16: two words an instruction, zero passing as 0xFFFF after the subtraction); a lane whose leaf fails runs the defining
+// flushed chain again from global memory. Every wait is bounded (status 10).
+#pragma once
+#include <cuda.h>
+
+#include <algorithm>
+
+#include "gemm_int8_tma.cuh"
+#include "gemm_skinny.cuh"
+
+namespace b200i {
+
+constexpr int SM_SEG = 64;  // bytes of a weight row per ring stage
+constexpr int SM_LEAF = 128;
+constexpr int SM_SMEM_LIMIT = 225 * 1024;
+constexpr int SM_SLABS = 2; // leaf groups whose activations a CTA holds
+
+struct StreamPlan {
+    int units;  // column units
+    int items;  // units * groups
+    int stages; // of a warp's ring
+    int key_off, bar_off, ring_off; // bytes into shared memory
+};
+
+template <int WK>
+struct StreamKind {
+    static constexpr int ES = WK == W_F32 ? 4 : (WK == W_BF16 ? 2 : 1);
+    static constexpr int KC = SM_SEG / ES; // k-steps per stage
+    static constexpr int EPQ = 16 / ES;    // k-steps per 16-byte piece
+    static constexpr int PPW = KS / EPQ;   // pieces per sixteen k-steps
+};
+
+template <int MT>
+__host__ __device__ constexpr bool sm_pow2() { return (MT & (MT - 1)) == 0; }
+// What row quad numbers of k-step k are permuted by (exclusive or): 32 / MT k-steps fill the banks once.
+template <int MT>
+__device__ __forceinline__ int sm_turn(int k) { return sm_pow2<MT>() ? (k / (32 / MT)) & (MT / 4 - 1) : 0; }
+
+template <int WK, int MT, int RG, int CPL, int NW>
+__global__ void __launch_bounds__(32 * NW, 1) gemm_stream_kernel(const __grid_constant__ CUtensorMap wmap, const GemmArgs g, const StreamPlan p) {
+    using K = StreamKind<WK>;
+    constexpr int LC = 32 / RG, CB = LC * CPL, RL = MT / RG, PAIRS = RL / 2, QUADS = RL / 4, CELLS = RL * CPL;
+    constexpr int STAGE = CB * SM_SEG;
+    constexpr bool INT8 = WK == W_INT8_EXP || WK == W_INT8_SCALE;
+    extern __shared__ __align__(1024) unsigned char sm_smem[];
+    float *act = reinterpret_cast<float *>(sm_smem);
+    unsigned *lkey = reinterpret_cast<unsigned *>(sm_smem + p.key_off);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, stages = p.stages;
+    unsigned long long *full = reinterpret_cast<unsigned long long *>(sm_smem + p.bar_off) + warp * stages;
+    unsigned char *ring = sm_smem + p.ring_off + (size_t)warp * stages * STAGE;
+
+    const int lo = (int)((long long)p.items * blockIdx.x / gridDim.x), hi = (int)((long long)p.items * (blockIdx.x + 1) / gridDim.x);
+    const int slab0 = lo / p.units, gl = g.group_leaves;
+
+    if (lane == 0) {
+        for (int s = 0; s < stages; s++) mbar_init(&full[s], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+
+    // ---- the copy stream of this warp: (item, chunk of its leaves) ----
+    int p_item = lo + warp, p_k = 0, p_slot = 0, p_row = 0, p_end = 0;
+    auto p_enter = [&]() {
+        if (p_item < hi) {
+            const int slab = p_item / p.units;
+            p_row = (p_item - slab * p.units) * CB;
+            p_k = slab * gl * SM_LEAF;
+            p_end = min(p_k + gl * SM_LEAF, g.k);
+        }
+    };
+    auto issue = [&]() {
+        if (p_item >= hi) return;
+        if (lane == 0) {
+            mbar_expect_tx(&full[p_slot], STAGE);
+            t8_tma_load(ring + (size_t)p_slot * STAGE, &wmap, &full[p_slot], p_k, p_row);
+        }
+        if (++p_slot == stages) p_slot = 0;
+        p_k += K::KC;
+        if (p_k >= p_end) {
+            p_item += NW;
+            p_enter();
+        }
+    };
+    p_enter();
+    for (int s = 0; s < stages; s++) issue();
+
+    // ---- activations of the CTA's leaf groups, rows past m zero; one key per leaf ----
+    const int k_first = slab0 * gl * SM_LEAF, k_last = min(min((hi - 1) / p.units + 1, g.groups) * gl * SM_LEAF, g.k), klen = k_last - k_first;
+    for (int i = tid; i < SM_SLABS * gl; i += 32 * NW) lkey[i] = 0xFFFFFFFFu;
+    __syncthreads();
+    for (int k0 = warp * 32; k0 < klen; k0 += 32 * NW) {
+        const int kk = k0 + lane;
+        float x[MT];
+#pragma unroll
+        for (int r = 0; r < MT; r++) x[r] = (kk < klen && r < g.m) ? __ldg(g.a + (size_t)r * g.k + k_first + kk) : 0.f;
+        unsigned key = 0xFFFFFFFFu;
+#pragma unroll
+        for (int r = 0; r < MT; r++) key = min(key, admit_key(x[r]));
+        if (kk < klen) {
+#pragma unroll
+            for (int q = 0; q < MT / 4; q++)
+                *reinterpret_cast<float4 *>(act + (size_t)kk * MT + (q ^ sm_turn<MT>(kk)) * 4) = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+        }
+        key = __reduce_min_sync(0xFFFFFFFFu, key);
+        if (lane == 0) atomicMin(&lkey[k0 / SM_LEAF], key);
+    }
+    __syncthreads();
+
+    const int lc = lane % LC, rg = lane / LC;
+    const int wswz = (lc >> 1) & 3; // the copy's swizzle: 16-byte pieces of row r lie at piece ^ (r / 2 % 4)
+    unsigned long long acc[PAIRS][CPL];
+    float stack[2][CELLS];
+    int slot = 0;
+    unsigned phase = 0;
+    bool alive = true;
+
+    for (int item = lo + warp; item < hi; item += NW) {
+        const int slab = item / p.units, col0 = (item - slab * p.units) * CB;
+        const int t0 = slab * gl, t1 = min(t0 + gl, g.leaves);
+        float f[CPL], nbias[CPL];
+        unsigned fkey = 0xFFFFFFFFu;
+        if (INT8) {
+#pragma unroll
+            for (int j = 0; j < CPL; j++) {
+                const int c = col0 + lc + j * LC;
+                f[j] = 1.f;
+                if (c < g.n) f[j] = WK == W_INT8_EXP ? pow2_f32(__ldg(static_cast<const int *>(g.bscale) + c)) : __ldg(static_cast<const float *>(g.bscale) + c);
+                const unsigned fexp = (__float_as_uint(f[j]) >> 23) & 0xFFu;
+                if (fexp < ADMIT_EXP || fexp < 27u || fexp > 227u) fkey = 0u; // the short spellings below would not be exact, or not admitted
+                nbias[j] = -8388736.0f * f[j];
+            }
+        }
+        for (int t = t0; t < t1; t++) {
+            const int leaf_len = min(SM_LEAF, g.k - t * SM_LEAF);
+            const float *ak = act + (size_t)(t * SM_LEAF - k_first) * MT;
+            unsigned key = fkey, key2 = 0xFFFFFFFFu;
+#pragma unroll
+            for (int i = 0; i < PAIRS; i++)
+#pragma unroll
+                for (int j = 0; j < CPL; j++) acc[i][j] = 0ull;
+            for (int koff = 0; koff < leaf_len; koff += K::KC) {
+                if (alive && !mbar_wait(&full[slot], phase)) {
+                    if (lane == 0) atomicExch(&g_decode_status, 10);
+                    alive = false;
+                }
+                const unsigned char *st = ring + (size_t)slot * STAGE + lc * SM_SEG;
+                const int len = min(K::KC, leaf_len - koff);
+#pragma unroll 1
+                for (int s = 0; s * KS < len; s++) { // sixteen k-steps
+                    const float *arow = ak + (size_t)(koff + s * KS) * MT;
+#pragma unroll
+                    for (int pp = 0; pp < K::PPW; pp++) {
+                        float v[CPL][K::EPQ];
+                        const int place = ((s * K::PPW + pp) ^ wswz) * 16;
+#pragma unroll
+                        for (int j = 0; j < CPL; j++) {
+                            const uint4 w4 = *reinterpret_cast<const uint4 *>(st + j * LC * SM_SEG + place);
+                            const unsigned word[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                if (WK == W_F32) {
+                                    v[j][e] = __uint_as_float(word[e]);
+                                    key = min(key, admit_key(v[j][e]));
+                                } else if (WK == W_BF16) {
+                                    v[j][(2 * e) % K::EPQ] = __uint_as_float(word[e] << 16);
+                                    v[j][(2 * e + 1) % K::EPQ] = __uint_as_float(word[e] & 0xFFFF0000u);
+                                    key2 = __viaddmin_u16x2(word[e] & 0x7FFF7FFFu, 0xFFFFFFFFu, key2);
+                                } else {
+                                    const unsigned x = word[e] ^ 0x80808080u;
+                                    const float b[4] = {biased_code<0>(x), biased_code<1>(x), biased_code<2>(x), biased_code<3>(x)};
+#pragma unroll
+                                    for (int z = 0; z < 4; z++)
+                                        v[j][(4 * e + z) % K::EPQ] = WK == W_INT8_EXP ? __fmaf_rn(b[z], f[j], nbias[j]) : __fmul_rn(__fsub_rn(b[z], 8388736.0f), f[j]);
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int e = 0; e < K::EPQ; e++) {
+                            const int kk = pp * K::EPQ + e, turn = sm_turn<MT>(kk), low = turn & (QUADS - 1), high = turn - low; // 0 unless MT and RL are powers of two
+                            const float *row = arow + kk * MT + ((rg * QUADS) ^ high) * 4;
+                            unsigned long long a2[PAIRS];
+#pragma unroll
+                            for (int i = 0; i < QUADS; i++) {
+                                const ulonglong2 tt = *reinterpret_cast<const ulonglong2 *>(row + (i ^ low) * 4);
+                                a2[2 * i] = tt.x;
+                                a2[2 * i + 1] = tt.y;
+                            }
+#pragma unroll
+                            for (int j = 0; j < CPL; j++) {
+                                const unsigned long long w2 = pack2(v[j][e], v[j][e]);
+#pragma unroll
+                                for (int i = 0; i < PAIRS; i++) acc[i][j] = fma2_bare(a2[i], w2, acc[i][j]);
+                            }
+                        }
+                    }
+                }
+                __syncwarp(); // every lane has read the slot
+                issue();
+                if (++slot == stages) { slot = 0; phase ^= 1u; }
+            }
+            // ---- the leaf's nodes ----
+            float v[CELLS];
+#pragma unroll
+            for (int i = 0; i < PAIRS; i++)
+#pragma unroll
+                for (int j = 0; j < CPL; j++) unpack2(ftz2_hw(acc[i][j]), v[2 * i * CPL + j], v[(2 * i + 1) * CPL + j]);
+            bool ok = min(key, lkey[t - slab0 * gl]) >= ADMIT_MIN;
+            if (WK == W_BF16) {
+                constexpr unsigned least = ADMIT_EXP ? (ADMIT_EXP << 7) - 1u : 0u;
+                ok = ok && (key2 & 0xFFFFu) >= least && (key2 >> 16) >= least;
+            }
+            if (!ok) { // this lane's columns again, by the defining step, from global memory
+#pragma unroll 1
+                for (int j = 0; j < CPL; j++) {
+                    const int c = col0 + lc + j * LC;
+                    if (c >= g.n) continue;
+                    float fj = 1.f;
+                    if (WK == W_INT8_EXP) fj = pow2_f32(__ldg(static_cast<const int *>(g.bscale) + c));
+                    if (WK == W_INT8_SCALE) fj = __ldg(static_cast<const float *>(g.bscale) + c);
+                    float slow[RL];
+#pragma unroll
+                    for (int r = 0; r < RL; r++) slow[r] = 0.f;
+#pragma unroll 1
+                    for (int kk = 0; kk < leaf_len; kk++) {
+                        const size_t off = (size_t)c * g.k + (size_t)t * SM_LEAF + kk;
+                        float w;
+                        if (WK == W_F32) w = ftz_bits(__ldg(static_cast<const float *>(g.b) + off));
+                        else if (WK == W_BF16) w = ftz_bits(bf16_bits_to_f32(__ldg(static_cast<const unsigned short *>(g.b) + off)));
+                        else w = dequant_int8_pow2((int)__ldg(static_cast<const signed char *>(g.b) + off), fj);
+#pragma unroll
+                        for (int r = 0; r < RL; r++) {
+                            const int q = (rg * QUADS + r / 4) ^ sm_turn<MT>(kk);
+                            slow[r] = step_flush(ftz_bits(ak[(size_t)kk * MT + q * 4 + (r & 3)]), w, slow[r]);
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < RL; r++)
+#pragma unroll
+                        for (int jj = 0; jj < CPL; jj++)
+                            if (jj == j) v[r * CPL + jj] = ftz_hw(slow[r]);
+                }
+            }
+            // the fold of the group's leaves: the binary counter's stack, in local memory
+            const int i_leaf = t - t0, last = t1 - t0 - 1;
+            if (i_leaf != last) {
+                int lvl = 0;
+                for (int bits = i_leaf; bits & 1; bits >>= 1, lvl++)
+#pragma unroll
+                    for (int c = 0; c < CELLS; c++) v[c] = fold_add(stack[lvl][c], v[c]);
+#pragma unroll
+                for (int c = 0; c < CELLS; c++) stack[lvl][c] = v[c];
+            } else {
+#pragma unroll 1
+                for (int lvl = 0; (last >> lvl) != 0; lvl++)
+                    if ((last >> lvl) & 1) {
+#pragma unroll
+                        for (int c = 0; c < CELLS; c++) v[c] = fold_add(stack[lvl][c], v[c]);
+                    }
+                float *out = g.groups > 1 ? g.ws + (size_t)slab * (size_t)g.m * (size_t)g.n : g.c;
+                const bool pairs = g.groups == 1 && epilogue_pairs(g.epi), on = g.groups == 1 && epilogue_on(g.epi);
+#pragma unroll
+                for (int r = 0; r < RL; r++) {
+                    const int row = rg * RL + r;
+#pragma unroll
+                    for (int j = 0; j < CPL; j++) {
+                        const int c = col0 + lc + j * LC;
+                        const float x = nan_canon(v[r * CPL + j]);
+                        if (pairs) { // gate and up of a pair are neighbouring lanes
+                            const float other = __shfl_xor_sync(0xFFFFFFFFu, x, 1);
+                            if (!(lane & 1) && row < g.m && c + 1 < g.n) g.c[(size_t)row * (g.n / 2) + c / 2] = epilogue_pair_apply(x, other, g.epi.bias, g.epi.act, c / 2);
+                        } else if (row < g.m && c < g.n) {
+                            out[(size_t)row * g.n + c] = on ? epilogue_apply(x, g.epi.bias, g.epi.act, c) : x;
+                        }
+                    }
+                }
+            }
+        }
+    }
+}
+
+inline bool sm_make_map(CUtensorMap *map, const void *base, long long rows, long long k, int wkind, int box_rows) {
+    T8EncodeFn fn = t8_encode_fn();
+    if (!fn) return false;
+    const int es = wkind == W_F32 ? 4 : (wkind == W_BF16 ? 2 : 1);
+    const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)k * es};
+    const cuuint32_t box[2] = {(cuuint32_t)(SM_SEG / es), (cuuint32_t)box_rows}, estr[2] = {1u, 1u};
+    const CUtensorMapDataType type = wkind == W_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : (wkind == W_BF16 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8);
+    return fn(map, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int WK, int MT, int RG, int CPL, int NW>
+inline bool launch_stream_cfg(const GemmArgs &g, int sms, cudaStream_t st) {
+    constexpr int CB = 32 / RG * CPL;
+    alignas(64) CUtensorMap map;
+    if (!sm_make_map(&map, g.b, g.n, g.k, WK, CB)) return false;
+    StreamPlan p;
+    p.units = (g.n + CB - 1) / CB;
+    p.items = p.units * g.groups;
+    p.key_off = std::min(g.groups, SM_SLABS) * g.group_leaves * SM_LEAF * MT * 4;
+    p.bar_off = (p.key_off + SM_SLABS * g.group_leaves * 4 + 15) / 16 * 16;
+    p.stages = 8;
+    auto ring = [&](int s) { return (p.bar_off + NW * s * 8 + 1023) / 1024 * 1024; };
+    while (p.stages > 1 && ring(p.stages) + NW * p.stages * CB * SM_SEG > SM_SMEM_LIMIT) p.stages--;
+    p.ring_off = ring(p.stages);
+    const int smem = p.ring_off + NW * p.stages * CB * SM_SEG;
+    if (smem > SM_SMEM_LIMIT || g.groups > sms) return false;
+    static std::atomic<bool> configured[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !configured[dev]) {
+        cudaFuncSetAttribute(gemm_stream_kernel<WK, MT, RG, CPL, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_SMEM_LIMIT);
+        configured[dev] = true;
+    }
+    gemm_stream_kernel<WK, MT, RG, CPL, NW><<<std::min(p.items, sms), 32 * NW, smem, st>>>(map, g, p);
+    return true;
+}
+
+} // namespace b200i
