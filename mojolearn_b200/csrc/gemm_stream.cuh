@@ -30,6 +30,7 @@ constexpr int SM_SEG = 64;  // bytes of a weight row per ring stage
 constexpr int SM_LEAF = 128;
 constexpr int SM_SMEM_LIMIT = 225 * 1024;
 constexpr int SM_SLABS = 2; // leaf groups whose activations a CTA holds
+constexpr int SM_LEVELS = 2, SM_MAX_RUN = 1 << SM_LEVELS; // levels of a lane's fold stack, and the leaves of a group that they hold
 
 struct StreamPlan {
     int units;  // column units
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(32 * NW, 1) gemm_stream_kernel(const __grid_co
     const int lc = lane % LC, rg = lane / LC;
     const int wswz = (lc >> 1) & 3; // the copy's swizzle: 16-byte pieces of row r lie at piece ^ (r / 2 % 4)
     unsigned long long acc[PAIRS][CPL];
-    float stack[2][CELLS];
+    float stack[SM_LEVELS][CELLS];
     int slot = 0;
     unsigned phase = 0;
     bool alive = true;
@@ -308,6 +309,7 @@ inline bool sm_make_map(CUtensorMap *map, const void *base, long long rows, long
 template <int WK, int MT, int RG, int CPL, int NW>
 inline bool launch_stream_cfg(const GemmArgs &g, int sms, cudaStream_t st) {
     constexpr int CB = 32 / RG * CPL;
+    if (g.group_leaves > SM_MAX_RUN || g.groups > sms) return false;
     alignas(64) CUtensorMap map;
     if (!sm_make_map(&map, g.b, g.n, g.k, WK, CB)) return false;
     StreamPlan p;
@@ -320,7 +322,7 @@ inline bool launch_stream_cfg(const GemmArgs &g, int sms, cudaStream_t st) {
     while (p.stages > 1 && ring(p.stages) + NW * p.stages * CB * SM_SEG > SM_SMEM_LIMIT) p.stages--;
     p.ring_off = ring(p.stages);
     const int smem = p.ring_off + NW * p.stages * CB * SM_SEG;
-    if (smem > SM_SMEM_LIMIT || g.groups > sms) return false;
+    if (smem > SM_SMEM_LIMIT) return false;
     static std::atomic<bool> configured[64];
     int dev = 0;
     cudaGetDevice(&dev);
