@@ -82,7 +82,9 @@ int64_t b200i_gemm_w(int64_t device, void *stream, float *c, const float *a, con
  * b200i_plan_workspace_bytes), 8 = the tall plan (op TN, float32, m and n up to 128, every leaf a group of its own), 9 = the
  * rows plan (op NT, up to 16 activation rows, leaf groups of at most 32, at 9 to 16 rows 16, and a weight for which
  * b200i_rows_plan_stages is not 0: a CTA holds the int8 factors of its n * groups / SMs columns), 10 = the band plan (op NT,
- * float32 weights, up to 32 rows); `group_leaves` = leaves per group (a power of two, 0 = no split). Every plan returns the same bits; the tests
+ * float32 weights, up to 32 rows), 11 = the stream plan (op NT, float32 or bf16 weights, up to 16 rows, leaf groups of at most
+ * four; a call of 5 to 16 rows over a large weight takes it in the place of the plan that b200i_auto_plan names, where its
+ * workspace holds the nodes); `group_leaves` = leaves per group (a power of two, 0 = no split). Every plan returns the same bits; the tests
  * hold them to that (the reference's launch-invariance gate,
  * gemm/checks/gemm_device_check.mojo:1016). */
 int64_t b200i_gemm_w_plan(int64_t device, void *stream, float *c, const float *a, const void *b, const void *bscale,

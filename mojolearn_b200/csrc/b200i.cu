@@ -27,6 +27,7 @@
 #include "gemm_skinny_reg.cuh"
 #include "gemm_rows.cuh"
 #include "gemm_band.cuh"
+#include "gemm_stream.cuh"
 #include "lowbit.cuh"
 
 using namespace b200i;
@@ -98,7 +99,7 @@ int64_t check_wait_status(char *err, int64_t err_cap, const char *who) {
 }
 
 // ---- plans -----------------------------------------------------------------------------
-enum { PLAN_AUTO = -1, PLAN_FLAT = 0, PLAN_T128 = 1, PLAN_T64 = 2, PLAN_DECODE = 3, PLAN_T32 = 4, PLAN_T128X64 = 5, PLAN_SKINNY = 6, PLAN_PACKED = 7, PLAN_TALL = 8, PLAN_ROWS = 9, PLAN_BAND = 10 };
+enum { PLAN_AUTO = -1, PLAN_FLAT = 0, PLAN_T128 = 1, PLAN_T64 = 2, PLAN_DECODE = 3, PLAN_T32 = 4, PLAN_T128X64 = 5, PLAN_SKINNY = 6, PLAN_PACKED = 7, PLAN_TALL = 8, PLAN_ROWS = 9, PLAN_BAND = 10, PLAN_STREAM = 11 };
 
 // Up to this many rows the weight-streaming decode plan is preferred to the skinny plan; float32 weights at four rows then take
 // the rows plan where their call's workspace holds its nodes (rows_preferred: [11008, 4096] 55 us). Low-bit weights switch
@@ -352,6 +353,30 @@ inline bool band_preferred(const Plan &skinny, const Plan &band, long long m, lo
     return m > 16 || band_us(m, n, k, band.group_leaves, sms) < 0.97 * before_rows_us(skinny, m, n, k, W_F32, sms);
 }
 
+// 5 to 16 rows over large weights: the streaming kernel (gemm_stream.cuh) in the place of what choose_auto comes to. Lines from
+// 57 sizes of 768 to 50304 columns by 768 to 8192 steps at 5, 8, 11 and 16 rows, the plan before -> this one, in microseconds:
+// float32 from nine million words (8 rows [4935, 1840] 21.4 -> 16.8, 16 rows 32.7 -> 22.2; below, [1376, 5824] 17.4 -> 16.6 but
+// [3776, 1600] 12.5 -> 15.9); bf16 from 30 million at 5 to 8 rows ([7632, 4192] 35.6 -> 30.7; below, [2800, 7472] 23.8 -> 25.3)
+// and from 42 million at 9 to 16 ([11008, 4096] 67.9 -> 62.8; below, [18880, 2064] 58.1 -> 62.2).
+inline bool stream_preferred(long long m, long long n, long long k, int wkind) {
+    const double words = (double)n * (double)k;
+    if (m < 5) return false;
+    return wkind == W_F32 ? words >= 9.0e6 : (wkind == W_BF16 && words >= (m <= 8 ? 30.0e6 : 42.0e6));
+}
+// Leaves per group: single ones while every warp has an item or two, more where the items are many, so that fewer nodes pass
+// through L2 (float32, 8 rows, groups of one / two / four leaves: [5536, 2208] 20.2 / 23 / 31 us, [10512, 2256] 32.6 / 28.9 / 36,
+// [11008, 4096] 49.9 / 53.7 / 45.1). Groups of four want eight leaves at least.
+Plan choose_stream(long long n, long long k) {
+    const int leaves = (int)leaf_count(k) > 0 ? (int)leaf_count(k) : 1;
+    const double words = (double)n * (double)k;
+    int run = words < 16.0e6 ? 1 : (words < 42.0e6 || leaves < 8 ? 2 : 4);
+    while (run < SM_MAX_RUN && (leaves + run - 1) / run > MAX_GROUPS) run *= 2;
+    return Plan{PLAN_STREAM, run, (leaves + run - 1) / run};
+}
+inline bool stream_takes(const Plan &p, long long m, long long n, long long k, int op, int wkind, int sms) {
+    return stream_preferred(m, n, k, wkind) && stream_plan_fits(m, n, k, op, wkind, p.group_leaves, sms) && p.groups <= MAX_GROUPS;
+}
+
 // A^T B of few cells over many rows: every leaf of every 32 x 32 tile as a warp of its own (gemm_tall.cuh).
 constexpr long long TALL_MIN_LEAVES = 16;
 inline bool tall_fits(long long m, long long n, long long k, int op, int wkind) {
@@ -546,11 +571,15 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
     Plan plan;
     if (plan_kind == PLAN_AUTO) {
         const bool pairs = epilogue_pairs(g.epi);
-        plan = choose_auto(AutoCall{m, n, k, op, wkind, sm_count(dev), aligned(b, 16) && aligned(a, 16), pairs, leave_nodes != nullptr}, [&](const Plan &p) {
+        const bool al16 = aligned(b, 16) && aligned(a, 16);
+        auto fits = [&](const Plan &p) {
             const size_t need = plan_need(p, m, n, k);
             if (need && (!ws || ws_bytes < (int64_t)need || !aligned(ws, p.kind == PLAN_PACKED ? 256 : 4))) return false;
             return !pairs || p.groups <= 1 || (aligned(ws, 16) && aligned(c, 8)); // the fold of a gated store
-        });
+        };
+        plan = choose_auto(AutoCall{m, n, k, op, wkind, sm_count(dev), al16, pairs, leave_nodes != nullptr}, fits);
+        const Plan stream = choose_stream(n, k);
+        if (al16 && stream_takes(stream, m, n, k, op, wkind, sm_count(dev)) && fits(stream) && t8_encode_fn() != nullptr) plan = stream;
     } else {
         plan.kind = plan_kind;
         int s = group_leaves > 0 ? (int)group_leaves : g.leaves;
@@ -590,7 +619,7 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         // a gated activation needs both columns of a pair in one thread: the skinny plans, whose threads own adjacent
         // columns, apply it in their own store or in the group fold; no other plan spells it
         const bool fold_ok = plan.groups == 1 || (((long long)m * n) % 4 == 0 && aligned(ws, 16) && aligned(c, 8));
-        if ((plan.kind != PLAN_SKINNY && plan.kind != PLAN_ROWS && plan.kind != PLAN_BAND) || n % 4 != 0 || !fold_ok)
+        if ((plan.kind != PLAN_SKINNY && plan.kind != PLAN_ROWS && plan.kind != PLAN_BAND && plan.kind != PLAN_STREAM) || n % 4 != 0 || !fold_ok)
             return fail(err, err_cap, "identical gemm: the gated store activation needs the skinny plan (up to 32 rows, op NT, k a multiple of 16) and n a multiple of 4");
     }
     int tslot = -1;
@@ -614,6 +643,11 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         if (!skinny_plan_fits(m, n, k, op) || wkind != W_F32 || !aligned(b, 16) || !aligned(a, 16))
             return fail(err, err_cap, "identical gemm: the band plan needs op NT, m <= 32, float32 weights, k a multiple of 16 and 16-byte aligned operands");
         launch_band(g, st);
+        g_launches++;
+    } else if (plan.kind == PLAN_STREAM) {
+        if (!stream_plan_fits(m, n, k, op, wkind, plan.group_leaves, sm_count(dev)) || !aligned(b, 16) || !aligned(a, 16) || !launch_stream(g, sm_count(dev), st))
+            return fail(err, err_cap, "identical gemm: the stream plan needs op NT, m <= %d, float32 or bf16 weights, k a multiple of 16, 16-byte aligned operands, leaf "
+                        "groups of at most %d and tensor maps", SM_MAX_ROWS, SM_MAX_RUN);
         g_launches++;
     } else if (plan.kind == PLAN_TALL) {
         launch_tall(g, st); // its own fold, the store epilogue included
@@ -655,7 +689,7 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
         launch_fold_groups(g.ws, c, cells, plan.groups, st, g.epi, g.n);
         g_launches++;
     } else if (epilogue_on(g.epi) && plan.kind != PLAN_SKINNY && plan.kind != PLAN_DECODE && plan.kind != PLAN_TALL &&
-               plan.kind != PLAN_ROWS && plan.kind != PLAN_BAND) {
+               plan.kind != PLAN_ROWS && plan.kind != PLAN_BAND && plan.kind != PLAN_STREAM) {
         // the tiled, packed and flat plans store plain product words; their epilogue is a pass of its own
         const long long cells = (long long)m * n;
         if (n % 4 == 0 && aligned(c, 16))
@@ -750,6 +784,9 @@ int64_t b200i_workspace_bytes(int64_t m, int64_t n, int64_t k) {
         }
         if (rows_plan_fits(m, n, k, OP_NT)) groups = std::max(groups, choose_rows(k).groups);
         groups = std::max(groups, choose_band(m, n, k, sm_count(dev)).groups);
+        const Plan stream = choose_stream(n, k);
+        for (const int wkind : {W_F32, W_BF16})
+            if (stream_takes(stream, m, n, k, OP_NT, wkind, sm_count(dev))) groups = std::max(groups, stream.groups);
     }
     return groups > 1 ? (int64_t)groups * m * n * 4 : 0;
 }
@@ -764,6 +801,8 @@ int64_t b200i_product_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t o
             for (const bool all : {true, false})
                 most = std::max(most, plan_need(choose_auto(AutoCall{m, n, k, (int)op, (int)wkind, sm_count(dev), al16, pairs, false},
                                                             [&](const Plan &p) { return all || p.kind == PLAN_PACKED; }), m, n, k));
+    const Plan stream = choose_stream(n, k);
+    if (stream_takes(stream, m, n, k, (int)op, (int)wkind, sm_count(dev))) most = std::max(most, plan_need(stream, m, n, k));
     return (int64_t)most;
 }
 

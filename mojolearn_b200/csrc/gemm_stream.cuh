@@ -1,20 +1,29 @@
-// C[m, n] = A[m, k] . W[n, k]^T for a decode batch (5 to 32 rows), any weight storage: warps that walk the weight on their own.
+// C[m, n] = A[m, k] . W[n, k]^T for 5 to 16 rows over a large float32 or bf16 weight: warps that stream the weight on their own.
 //
-// The register skinny kernel (gemm_skinny_reg.cuh) reads a weight 16 bytes of 64 rows at a time, which DRAM serves far below its
-// streaming rate, stages activations behind CTA barriers and comes in whole waves of CTAs; it stays at half of the fma pipe at
-// 32 rows and at a third of HBM at eight. Here:
+// The rows, band and skinny kernels bring a weight by 16-byte pieces that a CTA's or a warp's threads ask for one window ahead,
+// and walk it between barriers or on short per-warp rings; on float32 weights of tens of millions of words they stay at half of
+// the HBM rate ([11008, 4096] at eight rows 57 us for 28 of bytes). Here:
 //
-//   - one CTA per SM, its warps independent after one barrier. The work is cut into items (leaf group, unit of CB columns),
-//     numbered leaf group by leaf group, and every CTA takes an equal run of them, so it meets at most two leaf groups, whose
-//     activations are staged once, [k][MT] with the row quads permuted by k so that the turning stores are free of bank conflicts;
-//   - a warp owns an item and brings its weights itself: one tensor-map copy (cp.async.bulk.tensor.2d, 64 bytes of CB rows,
+//   - one CTA of sixteen warps per SM, the warps independent after one barrier. The work is cut into items (leaf group, unit of
+//     64 columns), numbered leaf group by leaf group, and every CTA takes an equal run of them, so it meets at most two leaf
+//     groups, whose activations are staged once, [k][MT] with the row quads permuted by k so that the turning stores are free of
+//     bank conflicts;
+//   - a warp owns an item and brings its weights itself: one tensor-map copy (cp.async.bulk.tensor.2d, 64 bytes of 64 rows,
 //     64-byte swizzle) per stage of its own ring, completion on its own mbarriers, refilled by the warp when it has read a slot.
-//     No other warp is waited for. Edges of the weight and the k tail are zero-filled by the copy engine;
-//   - a lane owns RL rows (MT rows over RG row groups) by CPL columns, the rows in pairs: one 16-byte read of the activations
-//     serves 2 * CPL packed fmas, one 16-byte read of a column serves 4 to 16 k-steps.
+//     No other warp is waited for, and an SM has up to 192 KB in flight. Edges of the weight and the k tail are zero-filled;
+//   - a lane owns eight rows (MT rows over RG row groups) by CPL columns, the rows in pairs: one 16-byte read of the activations
+//     serves 2 * CPL packed fmas, one 16-byte read of a column serves 4 or 8 k-steps. Bodies of 4, 8 and 16 k-steps, eight and
+//     twelve warps and twice the cells per lane measured the same or slower.
+//
+// Measured (graph replay, several weights in turn, fold included), the plan before -> this: float32 at eight rows [11008, 4096]
+// 57 -> 45 us, [50304, 768] 54 -> 43, [10512, 2256] 48 -> 29; at sixteen [16384, 2048] 62 -> 50, [39296, 6416] 393 -> 270; bf16 at
+// eight [11008, 4096] 43.7 -> 38.6, at sixteen 67.9 -> 62.8. Bound: float32 at eight rows HBM (63 % of the measured copy rate at
+// [11008, 4096], 75 % at [39296, 6416]); otherwise the warps' own instructions. Int8 weights measured no faster than the rows and
+// register skinny kernels (36 against 34 us at eight rows, 87 against 86 at 32), nor did float32 ones at 32 rows (79 to 114
+// against 85 to 108), so those keep theirs.
 //
 // Admission is per leaf and lane: the activations' keys are taken while they are staged, the weights' while they are widened
-// (bf16: two words an instruction, zero passing as 0xFFFF after the subtraction); a lane whose leaf fails runs the defining
+// (bf16: two words an instruction, a zero passing as 0xFFFF after the subtraction); a lane whose leaf fails runs the defining
 // flushed chain again from global memory. Every wait is bounded (status 10).
 #pragma once
 #include <cuda.h>
@@ -27,7 +36,11 @@
 namespace b200i {
 
 constexpr int SM_SEG = 64;  // bytes of a weight row per ring stage
+constexpr int SM_CB = 64;   // columns of an item
+constexpr int SM_WARPS = 16;
+constexpr int SM_STEPS = 8; // k-steps of an unrolled body
 constexpr int SM_LEAF = 128;
+constexpr int SM_MAX_ROWS = 16;
 constexpr int SM_SMEM_LIMIT = 225 * 1024;
 constexpr int SM_SLABS = 2; // leaf groups whose activations a CTA holds
 constexpr int SM_LEVELS = 2, SM_MAX_RUN = 1 << SM_LEVELS; // levels of a lane's fold stack, and the leaves of a group that they hold
@@ -41,24 +54,22 @@ struct StreamPlan {
 
 template <int WK>
 struct StreamKind {
-    static constexpr int ES = WK == W_F32 ? 4 : (WK == W_BF16 ? 2 : 1);
+    static constexpr int ES = WK == W_F32 ? 4 : 2;
     static constexpr int KC = SM_SEG / ES; // k-steps per stage
     static constexpr int EPQ = 16 / ES;    // k-steps per 16-byte piece
-    static constexpr int PPW = KS / EPQ;   // pieces per sixteen k-steps
 };
 
+// What the row quad numbers of k-step k are permuted by (exclusive or): 32 / MT k-steps fill the banks once.
 template <int MT>
-__host__ __device__ constexpr bool sm_pow2() { return (MT & (MT - 1)) == 0; }
-// What row quad numbers of k-step k are permuted by (exclusive or): 32 / MT k-steps fill the banks once.
-template <int MT>
-__device__ __forceinline__ int sm_turn(int k) { return sm_pow2<MT>() ? (k / (32 / MT)) & (MT / 4 - 1) : 0; }
+__host__ __device__ constexpr int sm_turn(int k) { return (k / (32 / MT)) & (MT / 4 - 1); }
 
-template <int WK, int MT, int RG, int CPL, int NW>
-__global__ void __launch_bounds__(32 * NW, 1) gemm_stream_kernel(const __grid_constant__ CUtensorMap wmap, const GemmArgs g, const StreamPlan p) {
+template <int WK, int MT, int RG, int CPL>
+__global__ void __launch_bounds__(32 * SM_WARPS, 1) gemm_stream_kernel(const __grid_constant__ CUtensorMap wmap, const GemmArgs g, const StreamPlan p) {
+    static_assert(WK == W_F32 || WK == W_BF16, "int8 weights keep their kernels");
     using K = StreamKind<WK>;
-    constexpr int LC = 32 / RG, CB = LC * CPL, RL = MT / RG, PAIRS = RL / 2, QUADS = RL / 4, CELLS = RL * CPL;
+    constexpr int LC = 32 / RG, CB = LC * CPL, RL = MT / RG, PAIRS = RL / 2, QUADS = RL / 4, CELLS = RL * CPL, NW = SM_WARPS, UN = SM_STEPS;
     constexpr int STAGE = CB * SM_SEG;
-    constexpr bool INT8 = WK == W_INT8_EXP || WK == W_INT8_SCALE;
+    static_assert(CB == SM_CB && sm_turn<MT>(UN) == 0, "the quads' places inside a body are constants");
     extern __shared__ __align__(1024) unsigned char sm_smem[];
     float *act = reinterpret_cast<float *>(sm_smem);
     unsigned *lkey = reinterpret_cast<unsigned *>(sm_smem + p.key_off);
@@ -134,23 +145,10 @@ __global__ void __launch_bounds__(32 * NW, 1) gemm_stream_kernel(const __grid_co
     for (int item = lo + warp; item < hi; item += NW) {
         const int slab = item / p.units, col0 = (item - slab * p.units) * CB;
         const int t0 = slab * gl, t1 = min(t0 + gl, g.leaves);
-        float f[CPL], nbias[CPL];
-        unsigned fkey = 0xFFFFFFFFu;
-        if (INT8) {
-#pragma unroll
-            for (int j = 0; j < CPL; j++) {
-                const int c = col0 + lc + j * LC;
-                f[j] = 1.f;
-                if (c < g.n) f[j] = WK == W_INT8_EXP ? pow2_f32(__ldg(static_cast<const int *>(g.bscale) + c)) : __ldg(static_cast<const float *>(g.bscale) + c);
-                const unsigned fexp = (__float_as_uint(f[j]) >> 23) & 0xFFu;
-                if (fexp < ADMIT_EXP || fexp < 27u || fexp > 227u) fkey = 0u; // the short spellings below would not be exact, or not admitted
-                nbias[j] = -8388736.0f * f[j];
-            }
-        }
         for (int t = t0; t < t1; t++) {
             const int leaf_len = min(SM_LEAF, g.k - t * SM_LEAF);
             const float *ak = act + (size_t)(t * SM_LEAF - k_first) * MT;
-            unsigned key = fkey, key2 = 0xFFFFFFFFu;
+            unsigned key = 0xFFFFFFFFu; // bf16: of two words at a time
 #pragma unroll
             for (int i = 0; i < PAIRS; i++)
 #pragma unroll
@@ -163,12 +161,12 @@ __global__ void __launch_bounds__(32 * NW, 1) gemm_stream_kernel(const __grid_co
                 const unsigned char *st = ring + (size_t)slot * STAGE + lc * SM_SEG;
                 const int len = min(K::KC, leaf_len - koff);
 #pragma unroll 1
-                for (int s = 0; s * KS < len; s++) { // sixteen k-steps
-                    const float *arow = ak + (size_t)(koff + s * KS) * MT;
+                for (int s = 0; s * UN < len; s++) { // len is a multiple of sixteen
+                    const float *arow = ak + (size_t)(koff + s * UN) * MT;
 #pragma unroll
-                    for (int pp = 0; pp < K::PPW; pp++) {
+                    for (int pp = 0; pp < UN / K::EPQ; pp++) {
                         float v[CPL][K::EPQ];
-                        const int place = ((s * K::PPW + pp) ^ wswz) * 16;
+                        const int place = ((s * (UN / K::EPQ) + pp) ^ wswz) * 16;
 #pragma unroll
                         for (int j = 0; j < CPL; j++) {
                             const uint4 w4 = *reinterpret_cast<const uint4 *>(st + j * LC * SM_SEG + place);
@@ -178,22 +176,16 @@ __global__ void __launch_bounds__(32 * NW, 1) gemm_stream_kernel(const __grid_co
                                 if (WK == W_F32) {
                                     v[j][e] = __uint_as_float(word[e]);
                                     key = min(key, admit_key(v[j][e]));
-                                } else if (WK == W_BF16) {
+                                } else {
                                     v[j][(2 * e) % K::EPQ] = __uint_as_float(word[e] << 16);
                                     v[j][(2 * e + 1) % K::EPQ] = __uint_as_float(word[e] & 0xFFFF0000u);
-                                    key2 = __viaddmin_u16x2(word[e] & 0x7FFF7FFFu, 0xFFFFFFFFu, key2);
-                                } else {
-                                    const unsigned x = word[e] ^ 0x80808080u;
-                                    const float b[4] = {biased_code<0>(x), biased_code<1>(x), biased_code<2>(x), biased_code<3>(x)};
-#pragma unroll
-                                    for (int z = 0; z < 4; z++)
-                                        v[j][(4 * e + z) % K::EPQ] = WK == W_INT8_EXP ? __fmaf_rn(b[z], f[j], nbias[j]) : __fmul_rn(__fsub_rn(b[z], 8388736.0f), f[j]);
+                                    key = __viaddmin_u16x2(word[e] & 0x7FFF7FFFu, 0xFFFFFFFFu, key);
                                 }
                             }
                         }
 #pragma unroll
                         for (int e = 0; e < K::EPQ; e++) {
-                            const int kk = pp * K::EPQ + e, turn = sm_turn<MT>(kk), low = turn & (QUADS - 1), high = turn - low; // 0 unless MT and RL are powers of two
+                            const int kk = pp * K::EPQ + e, turn = sm_turn<MT>(kk), low = turn & (QUADS - 1), high = turn - low;
                             const float *row = arow + kk * MT + ((rg * QUADS) ^ high) * 4;
                             unsigned long long a2[PAIRS];
 #pragma unroll
@@ -221,29 +213,26 @@ __global__ void __launch_bounds__(32 * NW, 1) gemm_stream_kernel(const __grid_co
             for (int i = 0; i < PAIRS; i++)
 #pragma unroll
                 for (int j = 0; j < CPL; j++) unpack2(ftz2_hw(acc[i][j]), v[2 * i * CPL + j], v[(2 * i + 1) * CPL + j]);
-            bool ok = min(key, lkey[t - slab0 * gl]) >= ADMIT_MIN;
-            if (WK == W_BF16) {
+            bool ok = lkey[t - slab0 * gl] >= ADMIT_MIN;
+            if (WK == W_F32) {
+                ok = ok && key >= ADMIT_MIN;
+            } else {
                 constexpr unsigned least = ADMIT_EXP ? (ADMIT_EXP << 7) - 1u : 0u;
-                ok = ok && (key2 & 0xFFFFu) >= least && (key2 >> 16) >= least;
+                ok = ok && (key & 0xFFFFu) >= least && (key >> 16) >= least;
             }
             if (!ok) { // this lane's columns again, by the defining step, from global memory
 #pragma unroll 1
                 for (int j = 0; j < CPL; j++) {
                     const int c = col0 + lc + j * LC;
                     if (c >= g.n) continue;
-                    float fj = 1.f;
-                    if (WK == W_INT8_EXP) fj = pow2_f32(__ldg(static_cast<const int *>(g.bscale) + c));
-                    if (WK == W_INT8_SCALE) fj = __ldg(static_cast<const float *>(g.bscale) + c);
                     float slow[RL];
 #pragma unroll
                     for (int r = 0; r < RL; r++) slow[r] = 0.f;
 #pragma unroll 1
                     for (int kk = 0; kk < leaf_len; kk++) {
                         const size_t off = (size_t)c * g.k + (size_t)t * SM_LEAF + kk;
-                        float w;
-                        if (WK == W_F32) w = ftz_bits(__ldg(static_cast<const float *>(g.b) + off));
-                        else if (WK == W_BF16) w = ftz_bits(bf16_bits_to_f32(__ldg(static_cast<const unsigned short *>(g.b) + off)));
-                        else w = dequant_int8_pow2((int)__ldg(static_cast<const signed char *>(g.b) + off), fj);
+                        const float w = WK == W_F32 ? ftz_bits(__ldg(static_cast<const float *>(g.b) + off))
+                                                    : ftz_bits(bf16_bits_to_f32(__ldg(static_cast<const unsigned short *>(g.b) + off)));
 #pragma unroll
                         for (int r = 0; r < RL; r++) {
                             const int q = (rg * QUADS + r / 4) ^ sm_turn<MT>(kk);
@@ -284,8 +273,8 @@ __global__ void __launch_bounds__(32 * NW, 1) gemm_stream_kernel(const __grid_co
                         const float x = nan_canon(v[r * CPL + j]);
                         if (pairs) { // gate and up of a pair are neighbouring lanes
                             const float other = __shfl_xor_sync(0xFFFFFFFFu, x, 1);
-                            if (!(lane & 1) && row < g.m && c + 1 < g.n) g.c[(size_t)row * (g.n / 2) + c / 2] = epilogue_pair_apply(x, other, g.epi.bias, g.epi.act, c / 2);
-                        } else if (row < g.m && c < g.n) {
+                            if (alive && !(lane & 1) && row < g.m && c + 1 < g.n) g.c[(size_t)row * (g.n / 2) + c / 2] = epilogue_pair_apply(x, other, g.epi.bias, g.epi.act, c / 2);
+                        } else if (alive && row < g.m && c < g.n) {
                             out[(size_t)row * g.n + c] = on ? epilogue_apply(x, g.epi.bias, g.epi.act, c) : x;
                         }
                     }
@@ -295,42 +284,57 @@ __global__ void __launch_bounds__(32 * NW, 1) gemm_stream_kernel(const __grid_co
     }
 }
 
-inline bool sm_make_map(CUtensorMap *map, const void *base, long long rows, long long k, int wkind, int box_rows) {
+inline bool sm_make_map(CUtensorMap *map, const GemmArgs &g) {
     T8EncodeFn fn = t8_encode_fn();
     if (!fn) return false;
-    const int es = wkind == W_F32 ? 4 : (wkind == W_BF16 ? 2 : 1);
-    const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)k * es};
-    const cuuint32_t box[2] = {(cuuint32_t)(SM_SEG / es), (cuuint32_t)box_rows}, estr[2] = {1u, 1u};
-    const CUtensorMapDataType type = wkind == W_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : (wkind == W_BF16 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8);
-    return fn(map, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    const int es = g.wkind == W_F32 ? 4 : 2;
+    const cuuint64_t dims[2] = {(cuuint64_t)g.k, (cuuint64_t)g.n}, strides[1] = {(cuuint64_t)g.k * es};
+    const cuuint32_t box[2] = {(cuuint32_t)(SM_SEG / es), (cuuint32_t)SM_CB}, estr[2] = {1u, 1u};
+    return fn(map, g.wkind == W_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(g.b), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int WK, int MT, int RG, int CPL, int NW>
-inline bool launch_stream_cfg(const GemmArgs &g, int sms, cudaStream_t st) {
-    constexpr int CB = 32 / RG * CPL;
-    if (g.group_leaves > SM_MAX_RUN || g.groups > sms) return false;
-    alignas(64) CUtensorMap map;
-    if (!sm_make_map(&map, g.b, g.n, g.k, WK, CB)) return false;
+inline int stream_mt(long long m) { return m <= 8 ? 8 : 16; }
+// leaves in groups of at most SM_MAX_RUN (the lanes' fold stacks), at most two groups of which a CTA meets (groups <= SMs); the
+// column units and items are counted in 32 bits
+inline bool stream_plan_fits(long long m, long long n, long long k, int op, int wkind, int group_leaves, int sms) {
+    const long long leaves = leaf_count(k), run = std::min<long long>(group_leaves, leaves);
+    return m <= SM_MAX_ROWS && n <= (1ll << 26) && skinny_plan_fits(m, n, k, op) && leaf_size(k) <= SM_LEAF && (wkind == W_F32 || wkind == W_BF16) &&
+           run <= SM_MAX_RUN && (leaves + run - 1) / run <= sms;
+}
+
+template <int WK, int MT, int RG, int CPL>
+inline void launch_stream_cfg(const CUtensorMap &map, const GemmArgs &g, int sms, cudaStream_t st) {
     StreamPlan p;
-    p.units = (g.n + CB - 1) / CB;
+    p.units = (g.n + SM_CB - 1) / SM_CB;
     p.items = p.units * g.groups;
-    p.key_off = std::min(g.groups, SM_SLABS) * g.group_leaves * SM_LEAF * MT * 4;
+    p.key_off = std::min(g.groups, SM_SLABS) * g.group_leaves * SM_LEAF * MT * 4; // at most 64 KB
     p.bar_off = (p.key_off + SM_SLABS * g.group_leaves * 4 + 15) / 16 * 16;
-    p.stages = 8;
-    auto ring = [&](int s) { return (p.bar_off + NW * s * 8 + 1023) / 1024 * 1024; };
-    while (p.stages > 1 && ring(p.stages) + NW * p.stages * CB * SM_SEG > SM_SMEM_LIMIT) p.stages--;
+    p.stages = 3; // two where the activations leave no room for three; a stage is 64 KB over the warps
+    auto ring = [&](int s) { return (p.bar_off + SM_WARPS * s * 8 + 1023) / 1024 * 1024; };
+    while (ring(p.stages) + SM_WARPS * p.stages * SM_CB * SM_SEG > SM_SMEM_LIMIT) p.stages--;
     p.ring_off = ring(p.stages);
-    const int smem = p.ring_off + NW * p.stages * CB * SM_SEG;
-    if (smem > SM_SMEM_LIMIT) return false;
     static std::atomic<bool> configured[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaFuncSetAttribute(gemm_stream_kernel<WK, MT, RG, CPL, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_SMEM_LIMIT);
+        cudaFuncSetAttribute(gemm_stream_kernel<WK, MT, RG, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_SMEM_LIMIT);
         configured[dev] = true;
     }
-    gemm_stream_kernel<WK, MT, RG, CPL, NW><<<std::min(p.items, sms), 32 * NW, smem, st>>>(map, g, p);
+    gemm_stream_kernel<WK, MT, RG, CPL><<<std::min(p.items, sms), 32 * SM_WARPS, p.ring_off + SM_WARPS * p.stages * SM_CB * SM_SEG, st>>>(map, g, p);
+}
+
+// false where no tensor map can be made
+inline bool launch_stream(const GemmArgs &g, int sms, cudaStream_t st) {
+    alignas(64) CUtensorMap map;
+    if (!sm_make_map(&map, g)) return false;
+    if (g.wkind == W_F32) {
+        if (stream_mt(g.m) == 8) launch_stream_cfg<W_F32, 8, 1, 2>(map, g, sms, st);
+        else launch_stream_cfg<W_F32, 16, 2, 4>(map, g, sms, st);
+    } else {
+        if (stream_mt(g.m) == 8) launch_stream_cfg<W_BF16, 8, 1, 2>(map, g, sms, st);
+        else launch_stream_cfg<W_BF16, 16, 2, 4>(map, g, sms, st);
+    }
     return true;
 }
 
