@@ -43,5 +43,24 @@ def build(force=False, verbose=False, sabotage=False):
     return lib
 
 
+#: the native host side of a product call (host_call.cpp), a Python extension over torch's C++ library
+HOST_LIB = os.path.join(os.path.dirname(HERE), "_host_call.so")
+
+
+def build_host(force=False):
+    source = os.path.join(HERE, "host_call.cpp")
+    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= os.path.getmtime(source):
+        return HOST_LIB
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+           "-I" + os.path.join(root, "include"), "-I/usr/local/cuda/include", "-I" + sysconfig.get_paths()["include"], source, "-L" + os.path.join(root, "lib"),
+           "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_python", "-o", HOST_LIB]
+    subprocess.run(cmd, check=True)
+    return HOST_LIB
+
+
 if __name__ == "__main__":
+    build_host("--force" in sys.argv)
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv, sabotage="--sabotage" in sys.argv))

@@ -19,6 +19,11 @@ import functools
 import torch
 
 from . import _native
+
+try:
+    from . import _host_call  # csrc/host_call.cpp; without it the same calls go through ctypes
+except ImportError:
+    _host_call = None
 from .linalg import OP_NN, OP_NT, OP_TN, W_BF16, W_F32, W_INT8_EXP, W_INT8_SCALE, leaf_count
 
 PLAN_AUTO, PLAN_FLAT, PLAN_T128, PLAN_T64, PLAN_DECODE, PLAN_T32, PLAN_T128X64, PLAN_SKINNY, PLAN_PACKED, PLAN_TALL, PLAN_ROWS, PLAN_BAND, PLAN_STREAM = -1, 0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11
@@ -82,11 +87,28 @@ ACT_NONE, ACT_GELU_ERF, ACT_GELU_TANH, ACT_SILU = 0, 1, 2, 3
 ACT_PAIR_SWIGLU, ACT_PAIR_GEGLU_ERF, ACT_PAIR_GEGLU_TANH = 4, 5, 6  # over interleaved (gate, up) weight rows: output [m, n / 2]
 
 
+def _bind_plain_product(*args):
+    global _plain_product
+    lib = _native.lib()
+    _host_call.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.b200i_gemm_w_plan, lib.b200i_product_workspace_bytes, lib.b200i_plan_workspace_bytes)),
+                    _native.NativeError)
+    _plain_product = _host_call.product
+    return _plain_product(*args)
+
+
+#: a product of plain device tensors in native code, or None where a call is anything else ([11008, 4096] int8 row: see host_call.cpp)
+_plain_product = _bind_plain_product if _host_call is not None else None
+
+
 def product(a, b, bscale=None, wkind=W_F32, op=OP_NN, out=None, plan=PLAN_AUTO, group_leaves=0, bias=None, act=ACT_NONE):
     """C = op(a) . op(b) with b in weight storage `wkind`. `plan` forces an
     execution plan (tests); every plan gives the same bits. `bias` (one float32 per
     output column) and `act` are applied where the product stores its output: the
     words of the product followed by the separate bias and activation seams."""
+    if out is None and bias is None and act == ACT_NONE and _plain_product is not None:
+        done = _plain_product(a, b, bscale, wkind, op, plan, group_leaves)
+        if done is not None:
+            return done
     _check(a, "a", torch.float32)
     wdtype = _W_DTYPES[wkind]
     if wkind == W_BF16 and b.dtype in (torch.int16, torch.bfloat16):
