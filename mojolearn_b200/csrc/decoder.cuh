@@ -1053,7 +1053,7 @@ __global__ void __launch_bounds__(32 * CTX_WARPS) attn_context_kernel(float *__r
 // batch) gets up to CTX_ST_MAX stages instead: what bounds it is the bytes one CTA keeps in flight.
 constexpr int CTX_NB = 32, CTX_ST = 3, CTX_ST_MAX = 12;
 // Threads: up to four warps of chains; with 256, where there are too few rows to fill the device, four or more others share
-// what is not a chain.
+// the exponentials and divisions and issue the copies.
 inline size_t attn_context_row_smem(int s_grid, int hd, int stages = CTX_ST) {
     return ((size_t)((s_grid + 3) & ~3) + (size_t)stages * CTX_NB * hd) * sizeof(float) + (size_t)(s_grid + CTX_NB) / CTX_NB;
 }
@@ -1098,23 +1098,27 @@ __global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(fl
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    auto issue = [&](int k) { // stage k: keys jlo + 32k ..., into slot k % stages
-        if (bulk) {
-            if (tid == 0 && k < nstages) {
-                const int first = jlo + k * CTX_NB, keys = min(CTX_NB, jhi - first + 1);
-                const unsigned bytes = (unsigned)(keys * hd) * 4u;
-                mbar_expect_tx(&full[k % stages], bytes);
-                bulk_copy_g2s(ring + (size_t)(k % stages) * CTX_NB * hd, vbase + (long long)first * hd, bytes, &full[k % stages]);
-            }
-        } else { // always one commit, so that the groups count stages
-            if (k < nstages) {
-                const int first = jlo + k * CTX_NB, keys = min(CTX_NB, jhi - first + 1);
-                cp_async_floats(ring + (size_t)(k % stages) * CTX_NB * hd, vbase + (long long)first * hd, keys * hd, false, tid, CTX_T);
-            }
-            cp_async_commit();
-        }
+    auto copy_bulk = [&](int k, int to) { // stage k: keys jlo + 32k ..., into slot `to`, by the calling thread alone
+        const int first = jlo + k * CTX_NB, keys = min(CTX_NB, jhi - first + 1);
+        const unsigned bytes = (unsigned)(keys * hd) * 4u;
+        mbar_expect_tx(&full[to], bytes);
+        bulk_copy_g2s(ring + (size_t)to * CTX_NB * hd, vbase + (long long)first * hd, bytes, &full[to]);
     };
-    for (int k = 0; k < stages; k++) issue(k);
+    auto copy_words = [&](int k, int to) { // the same by every thread; always one commit, so that the groups count stages
+        if (k < nstages) {
+            const int first = jlo + k * CTX_NB, keys = min(CTX_NB, jhi - first + 1);
+            cp_async_floats(ring + (size_t)to * CTX_NB * hd, vbase + (long long)first * hd, keys * hd, false, tid, CTX_T);
+        }
+        cp_async_commit();
+    };
+    // The first stages go out from as many lanes of the last warp, which has no chain where there are warps to spare: one thread
+    // issuing twelve copies one after the other took 4500 cycles, and the first barrier waits for it.
+    const int issuer = CTX_T - 32;
+    if (!bulk) {
+        for (int k = 0; k < stages; k++) copy_words(k, k);
+    } else if (tid >= issuer && lane < min(stages, nstages)) {
+        copy_bulk(lane, lane);
+    }
     // wrow[i] belongs to key jlo + i, so a tile of 32 keys is one warp's 32 words and starts on a 16-byte boundary
     const int keys = jhi - jlo + 1;
     unsigned best = 0u;
@@ -1153,28 +1157,32 @@ __global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(fl
     }
     __syncthreads();
     // Values: thread d of the first warps walks feature d. The 32 words of a tile go to registers while the chain of the tile
-    // before runs, so a chain step costs its own latency. When all weights and values of a tile pass the product's admission
-    // test and every earlier step of the chain was admitted too, the bare fma is the contract's step (no result can be
-    // subnormal), else the flushed step. The values' keys are taken 16 bytes at a time by the warps that have no feature (by all when every one has), and
-    // the barrier that frees the tile's slot carries the verdict.
-    const int chains = (hd + 31) / 32, helpers = CTX_T / 32 - chains; // warps; head_dim <= 128
+    // before runs, so a chain step costs its own latency. When a tile's weights and this thread's words of it pass the product's
+    // admission test and every earlier step of its chain was admitted too, the bare fma is the contract's step (no result can be
+    // subnormal), else the flushed step. The bare chain runs while the words' keys are taken beside it, and is walked again where
+    // they fail: a thread's verdict is its own, so the warps meet only where a slot is filled again (keys by other warps and a
+    // vote per tile: 1080 cycles a tile, 500 of them the keys).
+    const int chains = (hd + 31) / 32; // warps; head_dim <= 128
     float acc = 0.f;
-    bool clean = true, admitted = false;
+    bool clean = true;
     const int d = tid < hd ? tid : 0;
     float cur[CTX_NB];
     auto walk = [&](int k, const float (&v)[CTX_NB]) { // tile k, whole
         const float *w = wrow + k * CTX_NB;
-        clean = clean && admitted;
-        if (clean) {
+        const float before = acc;
+        unsigned key = wok[k] && clean ? 0xFFFFFFFFu : 0u;
 #pragma unroll
-            for (int u = 0; u < CTX_NB; u += 4) {
-                const float4 w4 = *reinterpret_cast<const float4 *>(w + u);
-                acc = step_bare(w4.x, v[u], acc);
-                acc = step_bare(w4.y, v[u + 1], acc);
-                acc = step_bare(w4.z, v[u + 2], acc);
-                acc = step_bare(w4.w, v[u + 3], acc);
-            }
-        } else {
+        for (int u = 0; u < CTX_NB; u += 4) {
+            const float4 w4 = *reinterpret_cast<const float4 *>(w + u);
+            acc = step_bare(w4.x, v[u], acc);
+            acc = step_bare(w4.y, v[u + 1], acc);
+            acc = step_bare(w4.z, v[u + 2], acc);
+            acc = step_bare(w4.w, v[u + 3], acc);
+            key = min(min(key, admit_key(v[u])), min(admit_key(v[u + 1]), min(admit_key(v[u + 2]), admit_key(v[u + 3]))));
+        }
+        if (key < ADMIT_MIN) {
+            clean = false;
+            acc = before;
 #pragma unroll
             for (int u = 0; u < CTX_NB; u++) acc = step_flush(w[u], ftz_bits(v[u]), acc);
         }
@@ -1189,10 +1197,9 @@ __global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(fl
             cp_async_wait<CTX_ST - 1>(); // this thread's copies of stage k have landed
             __syncthreads();             // and everyone's
         }
-        const float *tile = ring + (size_t)slot * CTX_NB * hd, *vs = tile + d;
+        const float *vs = ring + (size_t)slot * CTX_NB * hd + d;
         const int count = min(CTX_NB, keys - k * CTX_NB);
         float next[CTX_NB];
-        unsigned key = wok[k] ? 0xFFFFFFFFu : 0u;
         if (warp < chains) {
             if (count == CTX_NB) {
 #pragma unroll
@@ -1200,11 +1207,8 @@ __global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(fl
             }
             if (k > 0) walk(k - 1, cur);
         }
-        if (count == CTX_NB && (helpers == 0 || warp >= chains)) {
-            const int first = helpers == 0 ? tid : tid - chains * 32, step = helpers == 0 ? CTX_T : 32 * helpers;
-            for (int i = first * 4; i < CTX_NB * hd; i += 4 * step) key = min(key, key_of4(*reinterpret_cast<const float4 *>(tile + i)));
-        }
-        admitted = __syncthreads_and(key >= ADMIT_MIN); // every thread holds its words of the tile: the slot is free
+        const bool refill = !bulk || k + stages < nstages;
+        if (refill) __syncthreads(); // every thread holds its words of the tile: the slot is free
         if (warp >= chains) {
             // nothing to walk
         } else if (count < CTX_NB) { // the last tile, ragged
@@ -1214,7 +1218,8 @@ __global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(fl
             for (int u = 0; u < CTX_NB; u++) cur[u] = next[u];
             if (k == nstages - 1) walk(k, cur);
         }
-        if (k + stages < nstages || !bulk) issue(k + stages);
+        if (!bulk) copy_words(k + stages, slot); // the slot just read
+        else if (refill && tid == issuer) copy_bulk(k + stages, slot);
         if (++slot == stages) { slot = 0; parity ^= 1u; }
     }
     if (tid < hd) ctx[((long long)bb * l + qi) * ((long long)nh * hd) + (long long)h * hd + tid] = acc;
