@@ -16,15 +16,16 @@
 //     twelve warps and twice the cells per lane measured the same or slower.
 //
 // Measured (graph replay, several weights in turn, fold included), the plan before -> this: float32 at eight rows [11008, 4096]
-// 57 -> 45 us, [50304, 768] 54 -> 43, [10512, 2256] 48 -> 29; at sixteen [16384, 2048] 62 -> 50, [39296, 6416] 393 -> 270; bf16 at
-// eight [11008, 4096] 43.7 -> 38.6, at sixteen 67.9 -> 62.8. Bound: float32 at eight rows HBM (63 % of the measured copy rate at
-// [11008, 4096], 75 % at [39296, 6416]); otherwise the warps' own instructions. Int8 weights measured no faster than the rows and
+// 56 -> 43 us, [10512, 2256] 47 -> 27, at five [50304, 768] 54 -> 41, at sixteen [39296, 6416] 393 -> 248; bf16 [11008, 4096] at
+// eight 42.6 -> 35.4, at sixteen 67.4 -> 58.6. Bound: float32 at eight rows HBM (64 % of the measured copy rate at [11008, 4096]);
+// otherwise the warps' own instructions and the items' uneven number per warp. Int8 weights measured no faster than the rows and
 // register skinny kernels (36 against 34 us at eight rows, 87 against 86 at 32), nor did float32 ones at 32 rows (79 to 114
 // against 85 to 108), so those keep theirs.
 //
 // Admission is per leaf and lane: the activations' keys are taken while they are staged, the weights' while they are widened
 // (bf16: two words an instruction, a zero passing as 0xFFFF after the subtraction); a lane whose leaf fails runs the defining
-// flushed chain again from global memory. Every wait is bounded (status 10).
+// flushed chain again from global memory. Every wait is bounded and decided by the whole warp: where one runs out the warp sets the
+// status (10), asks for no further copy, waits for those in flight (stream_ring.cuh) and leaves its items unwritten.
 #pragma once
 #include <cuda.h>
 
@@ -32,6 +33,7 @@
 
 #include "gemm_int8_tma.cuh"
 #include "gemm_skinny.cuh"
+#include "stream_ring.cuh"
 
 namespace b200i {
 
@@ -63,6 +65,16 @@ struct StreamKind {
 template <int MT>
 __host__ __device__ constexpr int sm_turn(int k) { return (k / (32 / MT)) & (MT / 4 - 1); }
 
+struct StreamWait { // by a whole warp, with one answer
+    unsigned long long *full;
+    __device__ __forceinline__ bool operator()(int slot, unsigned phase) const { return __all_sync(0xFFFFFFFFu, mbar_wait(&full[slot], phase)) != 0; }
+};
+// A warp's wait ran out. (Not inlined: its loop would cost the product's loop registers.)
+__device__ __noinline__ void sm_lost(unsigned long long *full, StreamRing flow) {
+    if ((threadIdx.x & 31) == 0) atomicExch(&g_decode_status, 10);
+    flow.drain(StreamWait{full});
+}
+
 template <int WK, int MT, int RG, int CPL>
 __global__ void __launch_bounds__(32 * SM_WARPS, 1) gemm_stream_kernel(const __grid_constant__ CUtensorMap wmap, const GemmArgs g, const StreamPlan p) {
     static_assert(WK == W_F32 || WK == W_BF16, "int8 weights keep their kernels");
@@ -73,7 +85,8 @@ __global__ void __launch_bounds__(32 * SM_WARPS, 1) gemm_stream_kernel(const __g
     extern __shared__ __align__(1024) unsigned char sm_smem[];
     float *act = reinterpret_cast<float *>(sm_smem);
     unsigned *lkey = reinterpret_cast<unsigned *>(sm_smem + p.key_off);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, stages = p.stages;
+    const int tid = threadIdx.x, lane = tid & 31, stages = p.stages;
+    const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0); // one value a warp: what follows from it lies in uniform registers
     unsigned long long *full = reinterpret_cast<unsigned long long *>(sm_smem + p.bar_off) + warp * stages;
     unsigned char *ring = sm_smem + p.ring_off + (size_t)warp * stages * STAGE;
 
@@ -87,7 +100,7 @@ __global__ void __launch_bounds__(32 * SM_WARPS, 1) gemm_stream_kernel(const __g
     __syncwarp();
 
     // ---- the copy stream of this warp: (item, chunk of its leaves) ----
-    int p_item = lo + warp, p_k = 0, p_slot = 0, p_row = 0, p_end = 0;
+    int p_item = lo + warp, p_k = 0, p_row = 0, p_end = 0;
     auto p_enter = [&]() {
         if (p_item < hi) {
             const int slab = p_item / p.units;
@@ -96,21 +109,22 @@ __global__ void __launch_bounds__(32 * SM_WARPS, 1) gemm_stream_kernel(const __g
             p_end = min(p_k + gl * SM_LEAF, g.k);
         }
     };
-    auto issue = [&]() {
-        if (p_item >= hi) return;
+    auto fill = [&](int slot) { // false where the warp's items have no more
+        if (p_item >= hi) return false;
         if (lane == 0) {
-            mbar_expect_tx(&full[p_slot], STAGE);
-            t8_tma_load(ring + (size_t)p_slot * STAGE, &wmap, &full[p_slot], p_k, p_row);
+            mbar_expect_tx(&full[slot], STAGE);
+            t8_tma_load(ring + (size_t)slot * STAGE, &wmap, &full[slot], p_k, p_row);
         }
-        if (++p_slot == stages) p_slot = 0;
         p_k += K::KC;
         if (p_k >= p_end) {
             p_item += NW;
             p_enter();
         }
+        return true;
     };
+    StreamRing flow{stages};
     p_enter();
-    for (int s = 0; s < stages; s++) issue();
+    flow.start(fill);
 
     // ---- activations of the CTA's leaf groups, rows past m zero; one key per leaf ----
     const int k_first = slab0 * gl * SM_LEAF, k_last = min(min((hi - 1) / p.units + 1, g.groups) * gl * SM_LEAF, g.k), klen = k_last - k_first;
@@ -138,9 +152,6 @@ __global__ void __launch_bounds__(32 * SM_WARPS, 1) gemm_stream_kernel(const __g
     const int wswz = (lc >> 1) & 3; // the copy's swizzle: 16-byte pieces of row r lie at piece ^ (r / 2 % 4)
     unsigned long long acc[PAIRS][CPL];
     float stack[SM_LEVELS][CELLS];
-    int slot = 0;
-    unsigned phase = 0;
-    bool alive = true;
 
     for (int item = lo + warp; item < hi; item += NW) {
         const int slab = item / p.units, col0 = (item - slab * p.units) * CB;
@@ -154,11 +165,11 @@ __global__ void __launch_bounds__(32 * SM_WARPS, 1) gemm_stream_kernel(const __g
 #pragma unroll
                 for (int j = 0; j < CPL; j++) acc[i][j] = 0ull;
             for (int koff = 0; koff < leaf_len; koff += K::KC) {
-                if (alive && !mbar_wait(&full[slot], phase)) {
-                    if (lane == 0) atomicExch(&g_decode_status, 10);
-                    alive = false;
+                if (!StreamWait{full}(flow.slot, flow.phase)) { // (no barrier of the block follows)
+                    sm_lost(full, flow);
+                    return;
                 }
-                const unsigned char *st = ring + (size_t)slot * STAGE + lc * SM_SEG;
+                const unsigned char *st = ring + (size_t)flow.slot * STAGE + lc * SM_SEG;
                 const int len = min(K::KC, leaf_len - koff);
 #pragma unroll 1
                 for (int s = 0; s * UN < len; s++) { // len is a multiple of sixteen
@@ -204,8 +215,7 @@ __global__ void __launch_bounds__(32 * SM_WARPS, 1) gemm_stream_kernel(const __g
                     }
                 }
                 __syncwarp(); // every lane has read the slot
-                issue();
-                if (++slot == stages) { slot = 0; phase ^= 1u; }
+                flow.release(fill);
             }
             // ---- the leaf's nodes ----
             float v[CELLS];
@@ -273,8 +283,8 @@ __global__ void __launch_bounds__(32 * SM_WARPS, 1) gemm_stream_kernel(const __g
                         const float x = nan_canon(v[r * CPL + j]);
                         if (pairs) { // gate and up of a pair are neighbouring lanes
                             const float other = __shfl_xor_sync(0xFFFFFFFFu, x, 1);
-                            if (alive && !(lane & 1) && row < g.m && c + 1 < g.n) g.c[(size_t)row * (g.n / 2) + c / 2] = epilogue_pair_apply(x, other, g.epi.bias, g.epi.act, c / 2);
-                        } else if (alive && row < g.m && c < g.n) {
+                            if (!(lane & 1) && row < g.m && c + 1 < g.n) g.c[(size_t)row * (g.n / 2) + c / 2] = epilogue_pair_apply(x, other, g.epi.bias, g.epi.act, c / 2);
+                        } else if (row < g.m && c < g.n) {
                             out[(size_t)row * g.n + c] = on ? epilogue_apply(x, g.epi.bias, g.epi.act, c) : x;
                         }
                     }
