@@ -44,6 +44,10 @@ constexpr int SM_STEPS = 8; // k-steps of an unrolled body
 constexpr int SM_LEAF = 128;
 constexpr int SM_MAX_ROWS = 16;
 constexpr int SM_SMEM_LIMIT = 225 * 1024;
+// The swizzled stages start on multiples of 512 bytes, inside an array that asks for no more than its siblings do: the strictest
+// alignment of a library's dynamic shared memory is what the static arrays of all its kernels are rounded up to, and the decode
+// attention shares out an SM to the last kilobyte (1024 here took its fourth CTA from an SM).
+constexpr int SM_ALIGN = 128, SM_RING_ALIGN = 512;
 constexpr int SM_SLABS = 2; // leaf groups whose activations a CTA holds
 constexpr int SM_LEVELS = 2, SM_MAX_RUN = 1 << SM_LEVELS; // levels of a lane's fold stack, and the leaves of a group that they hold
 
@@ -81,14 +85,16 @@ __global__ void __launch_bounds__(32 * SM_WARPS, 1) gemm_stream_kernel(const __g
     using K = StreamKind<WK>;
     constexpr int LC = 32 / RG, CB = LC * CPL, RL = MT / RG, PAIRS = RL / 2, QUADS = RL / 4, CELLS = RL * CPL, NW = SM_WARPS, UN = SM_STEPS;
     constexpr int STAGE = CB * SM_SEG;
+    static_assert(STAGE % SM_RING_ALIGN == 0, "every stage starts on one");
     static_assert(CB == SM_CB && sm_turn<MT>(UN) == 0, "the quads' places inside a body are constants");
-    extern __shared__ __align__(1024) unsigned char sm_smem[];
+    extern __shared__ __align__(SM_ALIGN) unsigned char sm_smem[];
     float *act = reinterpret_cast<float *>(sm_smem);
     unsigned *lkey = reinterpret_cast<unsigned *>(sm_smem + p.key_off);
     const int tid = threadIdx.x, lane = tid & 31, stages = p.stages;
     const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0); // one value a warp: what follows from it lies in uniform registers
     unsigned long long *full = reinterpret_cast<unsigned long long *>(sm_smem + p.bar_off) + warp * stages;
-    unsigned char *ring = sm_smem + p.ring_off + (size_t)warp * stages * STAGE;
+    const unsigned off = smem_u32(sm_smem) + (unsigned)p.ring_off;
+    unsigned char *ring = sm_smem + p.ring_off + ((0u - off) & (SM_RING_ALIGN - 1)) + (size_t)warp * stages * STAGE;
 
     const int lo = (int)((long long)p.items * blockIdx.x / gridDim.x), hi = (int)((long long)p.items * (blockIdx.x + 1) / gridDim.x);
     const int slab0 = lo / p.units, gl = g.group_leaves;
@@ -321,8 +327,9 @@ inline void launch_stream_cfg(const CUtensorMap &map, const GemmArgs &g, int sms
     p.key_off = std::min(g.groups, SM_SLABS) * g.group_leaves * SM_LEAF * MT * 4; // at most 64 KB
     p.bar_off = (p.key_off + SM_SLABS * g.group_leaves * 4 + 15) / 16 * 16;
     p.stages = 3; // two where the activations leave no room for three; a stage is 64 KB over the warps
-    auto ring = [&](int s) { return (p.bar_off + SM_WARPS * s * 8 + 1023) / 1024 * 1024; };
-    while (ring(p.stages) + SM_WARPS * p.stages * SM_CB * SM_SEG > SM_SMEM_LIMIT) p.stages--;
+    auto ring = [&](int s) { return (p.bar_off + SM_WARPS * s * 8 + SM_ALIGN - 1) / SM_ALIGN * SM_ALIGN; };
+    auto total = [&](int s) { return ring(s) + SM_RING_ALIGN - SM_ALIGN + SM_WARPS * s * SM_CB * SM_SEG; };
+    while (total(p.stages) > SM_SMEM_LIMIT) p.stages--;
     p.ring_off = ring(p.stages);
     static std::atomic<bool> configured[64];
     int dev = 0;
@@ -331,7 +338,7 @@ inline void launch_stream_cfg(const CUtensorMap &map, const GemmArgs &g, int sms
         cudaFuncSetAttribute(gemm_stream_kernel<WK, MT, RG, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_SMEM_LIMIT);
         configured[dev] = true;
     }
-    gemm_stream_kernel<WK, MT, RG, CPL><<<std::min(p.items, sms), 32 * SM_WARPS, p.ring_off + SM_WARPS * p.stages * SM_CB * SM_SEG, st>>>(map, g, p);
+    gemm_stream_kernel<WK, MT, RG, CPL><<<std::min(p.items, sms), 32 * SM_WARPS, total(p.stages), st>>>(map, g, p);
 }
 
 // false where no tensor map can be made
