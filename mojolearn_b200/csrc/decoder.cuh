@@ -1047,8 +1047,9 @@ __global__ void __launch_bounds__(32 * CTX_WARPS) attn_context_kernel(float *__r
 // softmax phases, so a CTA keeps up to 32 KB outstanding to HBM while the chain runs.
 // A head_dim that is not a multiple of 4 leaves rows off the 16-byte grid the bulk
 // copy needs; those caches go through per-thread cp.async instead.
-// Every wait on an mbarrier is bounded; one that runs out sets the status word read by
-// b200i_decode_status (value 3) and the kernel carries on to its end.
+// Every wait on an mbarrier is bounded, by each thread on its own; one that runs out sets the status word read by
+// b200i_decode_status (value 3) and ends its thread, which stores nothing (a barrier counts the threads that are left). The
+// thread that fills the slots does so only after its own wait came back true, and drains what is in flight before it ends.
 // Three stages and a 4K-key weight row fit four CTAs on an SM. A call with few CTAs (a head-sharded rank, a small
 // batch) gets up to CTX_ST_MAX stages instead: what bounds it is the bytes one CTA keeps in flight.
 constexpr int CTX_NB = 32, CTX_ST = 3, CTX_ST_MAX = 12;
@@ -1069,6 +1070,13 @@ inline long long att_cta_bytes(long long ctas, int sms, long long most) { // eno
 inline int attn_context_row_stages(long long rows, int s_grid, int hd, int sms) {
     const long long ring = att_cta_bytes(rows, sms, 4) - (long long)attn_context_row_smem(s_grid, hd, 0);
     return (int)std::min<long long>(std::max<long long>(ring / (CTX_NB * hd * (long long)sizeof(float)), CTX_ST), CTX_ST_MAX);
+}
+// The wait for stage k of a value ring ran out; the thread that fills the slots waits once more for each copy in flight. (Not
+// inlined, and its thread returns afterwards: a flag that the loop asks cost 3 % of a row.)
+__device__ __noinline__ void value_ring_lost(unsigned long long *full, bool fills, int k, int stages, int nstages) {
+    atomicExch(&g_decode_status, 3);
+    if (!fills) return;
+    for (const int end = min(k + stages, nstages); k < end; k++) mbar_wait(&full[k % stages], (unsigned)(k / stages) & 1u);
 }
 template <int CTX_T>
 __global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(float *__restrict__ ctx, float *__restrict__ scores,
@@ -1192,7 +1200,10 @@ __global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(fl
 #pragma unroll 2
     for (int k = 0; k < nstages; k++) {
         if (bulk) {
-            if (!mbar_wait(&full[slot], parity) && lane == 0) atomicExch(&g_decode_status, 3);
+            if (!mbar_wait(&full[slot], parity)) {
+                value_ring_lost(full, tid == issuer, k, stages, nstages);
+                return;
+            }
         } else {
             cp_async_wait<CTX_ST - 1>(); // this thread's copies of stage k have landed
             __syncthreads();             // and everyone's
@@ -1432,12 +1443,11 @@ __global__ void __launch_bounds__(ATD_THREADS) attn_decode_kernel(float *__restr
         rhi[i] = i < l ? min(own0 + i, s - 1) : -1;
         rlo[i] = (window > 0) ? max(own0 + i - window + 1, 0) : 0;
     }
-    bool alive = true;
     for (int k = 0; k < nstages; k++) {
         issue(k + stages - 1); // refills the slot the previous turn finished with
-        if (alive && !mbar_wait(&full[k % stages], (unsigned)(k / stages) & 1u)) {
-            if (lane == 0) atomicExch(&g_decode_status, 3);
-            alive = false;
+        if (!mbar_wait(&full[k % stages], (unsigned)(k / stages) & 1u)) {
+            value_ring_lost(full, tid == 0, k, stages, nstages);
+            return;
         }
         __syncthreads();
         if (tid < hd) {

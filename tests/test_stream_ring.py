@@ -74,3 +74,13 @@ def test_the_streaming_kernel_waits_as_a_warp():
         code = re.sub(r"//[^\n]*", "", f.read())
     assert code.count("mbar_wait(") == code.count("__all_sync(0xFFFFFFFFu, mbar_wait(") == 1
     assert code.count("t8_tma_load(") == 1 and "flow.start(fill)" in code and "flow.drain(StreamWait{full})" in code and "flow.release(fill)" in code
+
+
+def test_the_value_rings_of_decode_attention_fill_nothing_after_a_lost_wait():
+    """Whichever thread's wait runs out reports it and ends there; the thread that fills the slots drains its copies first."""
+    with open(os.path.join(CSRC, "decoder.cuh")) as f:
+        code = re.sub(r"\s+", " ", re.sub(r"//[^\n]*", "", f.read()))
+    fillers = re.findall(r"if \(!mbar_wait\([^{};]*\)\) \{ value_ring_lost\(full, tid == (\w+), k, stages, nstages\); return; \}", code)
+    assert fillers == ["issuer", "0"]
+    assert code.count("mbar_wait(") == 3  # those two, and the drain's own
+    assert "else if (refill && tid == issuer) copy_bulk(" in code and "if (tid == 0 && k < nstages) {" in code
