@@ -1167,9 +1167,10 @@ __global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(fl
     // Values: thread d of the first warps walks feature d. The 32 words of a tile go to registers while the chain of the tile
     // before runs, so a chain step costs its own latency. When a tile's weights and this thread's words of it pass the product's
     // admission test and every earlier step of its chain was admitted too, the bare fma is the contract's step (no result can be
-    // subnormal), else the flushed step. The bare chain runs while the words' keys are taken beside it, and is walked again where
-    // they fail: a thread's verdict is its own, so the warps meet only where a slot is filled again (keys by other warps and a
-    // vote per tile: 1080 cycles a tile, 500 of them the keys).
+    // subnormal), else the flushed step. Where the weights and the chain so far allow it, the bare chain runs while the words' keys
+    // are taken beside it, and is walked again if they fail: a thread's verdict is its own, so the warps meet only where a slot is
+    // filled again (keys by other warps and a vote per tile: 1080 cycles a tile, 500 of them the keys). Where they do not (a row
+    // whose softmax has weights under 2^-40), only the flushed chain runs.
     const int chains = (hd + 31) / 32; // warps; head_dim <= 128
     float acc = 0.f;
     bool clean = true;
@@ -1178,18 +1179,21 @@ __global__ void __launch_bounds__(CTX_T, 512 / CTX_T) attn_context_row_kernel(fl
     auto walk = [&](int k, const float (&v)[CTX_NB]) { // tile k, whole
         const float *w = wrow + k * CTX_NB;
         const float before = acc;
-        unsigned key = wok[k] && clean ? 0xFFFFFFFFu : 0u;
+        clean = clean && wok[k];
+        if (clean) {
+            unsigned key = 0xFFFFFFFFu;
 #pragma unroll
-        for (int u = 0; u < CTX_NB; u += 4) {
-            const float4 w4 = *reinterpret_cast<const float4 *>(w + u);
-            acc = step_bare(w4.x, v[u], acc);
-            acc = step_bare(w4.y, v[u + 1], acc);
-            acc = step_bare(w4.z, v[u + 2], acc);
-            acc = step_bare(w4.w, v[u + 3], acc);
-            key = min(min(key, admit_key(v[u])), min(admit_key(v[u + 1]), min(admit_key(v[u + 2]), admit_key(v[u + 3]))));
+            for (int u = 0; u < CTX_NB; u += 4) {
+                const float4 w4 = *reinterpret_cast<const float4 *>(w + u);
+                acc = step_bare(w4.x, v[u], acc);
+                acc = step_bare(w4.y, v[u + 1], acc);
+                acc = step_bare(w4.z, v[u + 2], acc);
+                acc = step_bare(w4.w, v[u + 3], acc);
+                key = min(min(key, admit_key(v[u])), min(admit_key(v[u + 1]), min(admit_key(v[u + 2]), admit_key(v[u + 3]))));
+            }
+            clean = key >= ADMIT_MIN;
         }
-        if (key < ADMIT_MIN) {
-            clean = false;
+        if (!clean) {
             acc = before;
 #pragma unroll
             for (int u = 0; u < CTX_NB; u++) acc = step_flush(w[u], ftz_bits(v[u]), acc);

@@ -110,6 +110,38 @@ def test_decode_step_attention_admission_fails_in_a_late_tile(l):
             assert got.tobytes() == want.tobytes(), (l, variant, at)
 
 
+def value_chain_cases():
+    """One decode row's chains with one feature zero but for a tile of words so small that each weighted one is flushed, the other
+    features ordinary: the first, a middle and the last whole tile, with few rows (256 threads a row) and many (128)."""
+    for hd in (64, 128):
+        for b, nh in ((1, 2), (10, 32)):
+            rng = np.random.default_rng(hd + b)
+            used, d = 672, hd - 5
+            q, kc, vc = _operands(rng, b, 1, nh, 1, hd, used, 0.01)
+            for tile in (0, 10, 20):
+                v2 = vc.copy()
+                v2[:, :, :, d] = 0.0
+                v2[:, :, 32 * tile:32 * tile + 32, d] = np.float32(2.0 ** -118)
+                yield "head_dim %d, %d rows, tile %d" % (hd, b * nh, tile), d, q, kc, v2, used
+
+
+def value_chain_right():
+    """name -> whether all words are right, over the cases above; the walked feature's and the others' apart."""
+    out = {}
+    for name, d, q, kc, vc, used in value_chain_cases():
+        want = oracle.attention(q, kc, vc, 1, used)
+        hd = vc.shape[3]
+        assert not want.reshape(-1, hd)[:, d].any(), name  # every weighted word is below 2^-126
+        for at in (False, True):
+            same = (_run(q, kc, vc, 1, used, 0, at).view(np.int32) == want.view(np.int32)).reshape(-1, hd)
+            out["%s, at %d" % (name, at)] = (bool(same[:, d].all()), bool(np.delete(same, d, axis=1).all()))
+    return out
+
+
+def test_a_value_chain_takes_the_flushed_step_by_its_own_words():
+    assert set(value_chain_right().values()) == {(True, True)}
+
+
 def test_prefill_attention_against_the_oracle_at_head_dim_128_and_64():
     """A prompt-sized call (l > 8 takes the tiled kernels): 200 and 77 positions on an empty and on a part-filled cache."""
     rng = np.random.default_rng(5)

@@ -108,3 +108,21 @@ def test_admit_always_build_fails_every_forcing_case_of_the_split_paths():
     right = json.loads(line[len("RESULT "):])
     whole = {name: ok for name, ok in right.items() if "ragged" not in name}
     assert len(whole) > 100 and not any(whole.values()), [name for name, ok in whole.items() if ok]
+
+
+VALUE_CHILD = r"""
+import json, sys
+sys.path[:0] = [%(root)r, %(root)r + "/tests"]
+import test_gpu_attention as t
+print("RESULT " + json.dumps(t.value_chain_right()))
+"""
+
+
+def test_admit_always_build_fails_every_value_chain_case():
+    """The feature of small words goes wrong in every case; the ordinary features, whose words are admitted anyway, stay right."""
+    from mojolearn_b200.csrc import build as cuda_build
+    run = subprocess.run([sys.executable, "-c", VALUE_CHILD % {"root": ROOT}], env=dict(os.environ, MOJOLEARN_B200_LIB=cuda_build.build(sabotage=True)),
+                         capture_output=True, text=True, timeout=600)
+    assert run.returncode == 0, run.stderr[-3000:]
+    right = json.loads([ln for ln in run.stdout.splitlines() if ln.startswith("RESULT ")][-1][len("RESULT "):])
+    assert len(right) == 24 and all(v == [False, True] for v in right.values()), right
