@@ -83,8 +83,8 @@ int64_t b200i_gemm_w(int64_t device, void *stream, float *c, const float *a, con
  * rows plan (op NT, up to 16 activation rows, leaf groups of at most 32, at 9 to 16 rows 16, and a weight for which
  * b200i_rows_plan_stages is not 0: a CTA holds the int8 factors of its n * groups / SMs columns), 10 = the band plan (op NT,
  * float32 weights, up to 32 rows), 11 = the stream plan (op NT, float32 or bf16 weights, up to 16 rows, leaf groups of at most
- * four; a call of 5 to 16 rows over a large weight takes it in the place of the plan that b200i_auto_plan names, where its
- * workspace holds the nodes); `group_leaves` = leaves per group (a power of two, 0 = no split). Every plan returns the same bits; the tests
+ * four; what a call of 5 to 16 rows over a large weight takes, where tensor maps can be made and its workspace holds the nodes);
+ * `group_leaves` = leaves per group (a power of two, 0 = no split). Every plan returns the same bits; the tests
  * hold them to that (the reference's launch-invariance gate,
  * gemm/checks/gemm_device_check.mojo:1016). */
 int64_t b200i_gemm_w_plan(int64_t device, void *stream, float *c, const float *a, const void *b, const void *bscale,
@@ -130,8 +130,8 @@ int64_t b200i_kernel_timing_read(double *total_ms, int64_t *launches);
 int64_t b200i_plan_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t plan, int64_t group_leaves);
 
 /* The plan (and the leaves per group) that the automatic choice takes on a device of `sms` SMs for 16-byte aligned
- * operands, a plain store and `ws_bytes` of workspace (-1 = all it asks for; a plan that the workspace does not hold is passed
- * over for the one before it); -1 for a bad extent. No CUDA call is made. */
+ * operands, a plain store, a driver that makes tensor maps and `ws_bytes` of workspace (-1 = all it asks for; a plan that the
+ * workspace does not hold is passed over for the one before it); -1 for a bad extent. No CUDA call is made. */
 int64_t b200i_auto_plan(int64_t m, int64_t n, int64_t k, int64_t op, int64_t wkind, int64_t sms, int64_t ws_bytes, int64_t *group_leaves);
 
 /* Stages of the rows plan's shared-memory ring on a device of `sms` SMs (2 or 3), 0 where the plan refuses the shape;

@@ -353,28 +353,64 @@ inline bool band_preferred(const Plan &skinny, const Plan &band, long long m, lo
     return m > 16 || band_us(m, n, k, band.group_leaves, sms) < 0.97 * before_rows_us(skinny, m, n, k, W_F32, sms);
 }
 
-// 5 to 16 rows over large weights: the streaming kernel (gemm_stream.cuh) in the place of what choose_auto comes to. Lines from
-// 57 sizes of 768 to 50304 columns by 768 to 8192 steps at 5, 8, 11 and 16 rows, the plan before -> this one, in microseconds:
-// float32 from nine million words (8 rows [4935, 1840] 21.4 -> 16.8, 16 rows 32.7 -> 22.2; below, [1376, 5824] 17.4 -> 16.6 but
-// [3776, 1600] 12.5 -> 15.9); bf16 from 30 million at 5 to 8 rows ([7632, 4192] 35.6 -> 30.7; below, [2800, 7472] 23.8 -> 25.3)
-// and from 42 million at 9 to 16 ([11008, 4096] 67.9 -> 62.8; below, [18880, 2064] 58.1 -> 62.2).
-inline bool stream_preferred(long long m, long long n, long long k, int wkind) {
-    const double words = (double)n * (double)k;
-    if (m < 5) return false;
-    return wkind == W_F32 ? words >= 9.0e6 : (wkind == W_BF16 && words >= (m <= 8 ? 30.0e6 : 42.0e6));
+// 5 to 16 rows over large weights: modelled microseconds of the streaming kernel, its fold included. A CTA's warps take its items
+// in turn; a turn of sixteen runs at the warps' common rate, the last one at its own number of warps or, with few, at the pace of
+// one. Fitted to 1800 launches of 1024 to 50304 columns by 768 to 12208 steps in groups of one, two and four leaves (nine in ten
+// within 6 % for bf16, 9 for float32).
+double stream_us(long long m, long long n, long long k, int wkind, int group_leaves, int sms) {
+    static const double fit[2][2][5] = { // [float32, bf16][8 rows, 16]: start, a leaf of one warp among many, alone, fold, a turn's start
+        {{5.5, 0.85, 3.6, 2.4, 1.0}, {8.8, 1.06, 4.5, 3.3, 1.6}}, {{8.2, 0.566, 3.65, 3.2, 0.74}, {10.3, 0.959, 4.2, 3.9, 2.1}}};
+    const double *f = fit[wkind == W_F32 ? 0 : 1][m <= 8 ? 0 : 1];
+    const long long leaves = leaf_count(k), run = std::min<long long>(group_leaves, leaves), groups = (leaves + run - 1) / run;
+    const long long items = (n + SM_CB - 1) / SM_CB * groups, ctas = std::min<long long>(items, sms), own = (items + ctas - 1) / ctas;
+    const long long turns = own / SM_WARPS, rest = own % SM_WARPS;
+    const double walk = groups > 1 ? (double)run : k / 128.0; // leaves of an item
+    double t = f[0] + (double)turns * (SM_WARPS * f[1] * walk + f[4]);
+    if (rest) t += std::max(f[2], (double)rest * f[1]) * walk + f[4];
+    if (groups > 1) t += f[3] + (double)groups * m * n * 8.0 / 7.5e6;
+    return t;
 }
-// Leaves per group: single ones while every warp has an item or two, more where the items are many, so that fewer nodes pass
-// through L2 (float32, 8 rows, groups of one / two / four leaves: [5536, 2208] 20.2 / 23 / 31 us, [10512, 2256] 32.6 / 28.9 / 36,
-// [11008, 4096] 49.9 / 53.7 / 45.1). Groups of four want eight leaves at least.
-Plan choose_stream(long long n, long long k) {
+// Leaves per group, by the weight's words: single ones while every warp has an item or two, more where the items are many, so that
+// fewer nodes pass through L2 (float32, 8 rows, groups of one / two / four leaves: [5536, 2208] 20.2 / 23 / 31 us, [10512, 2256]
+// 32.6 / 28.9 / 36, [11008, 4096] 45.6 / 49.2 / 42.7). Groups of four want eight leaves at least. For bf16 another split is taken
+// where the model has it 4 or 5 % faster: at the words' lines a CTA's items just pass sixteen, and a second turn of one or two warps
+// costs as much as a whole one (8 rows, groups of two / four [9600, 4096] 40.2 / 35.9, of four / two / one [33236, 2064] 61 / 49 / 51).
+Plan choose_stream(long long m, long long n, long long k, int wkind, int sms) {
     const int leaves = (int)leaf_count(k) > 0 ? (int)leaf_count(k) : 1;
     const double words = (double)n * (double)k;
+    auto groups = [&](int run) { return (leaves + run - 1) / run; };
     int run = words < 16.0e6 ? 1 : (words < 42.0e6 || leaves < 8 ? 2 : 4);
-    while (run < SM_MAX_RUN && (leaves + run - 1) / run > MAX_GROUPS) run *= 2;
-    return Plan{PLAN_STREAM, run, (leaves + run - 1) / run};
+    while (run < SM_MAX_RUN && groups(run) > MAX_GROUPS) run *= 2;
+    if (wkind == W_BF16) {
+        double least = (m <= 8 ? 0.96 : 0.95) * stream_us(m, n, k, wkind, run, sms);
+        for (int r = 1; r <= SM_MAX_RUN; r *= 2)
+            if (groups(r) <= MAX_GROUPS && stream_us(m, n, k, wkind, r, sms) < least) {
+                least = stream_us(m, n, k, wkind, r, sms);
+                run = r;
+            }
+    }
+    return Plan{PLAN_STREAM, run, groups(run)};
 }
-inline bool stream_takes(const Plan &p, long long m, long long n, long long k, int op, int wkind, int sms) {
-    return stream_preferred(m, n, k, wkind) && stream_plan_fits(m, n, k, op, wkind, p.group_leaves, sms) && p.groups <= MAX_GROUPS;
+// Lines from 57 sizes of 768 to 50304 columns by 768 to 8192 steps at 5, 8, 11 and 16 rows, the plan before -> this one, in
+// microseconds: float32 from nine million words (8 rows [4935, 1840] 21.4 -> 16.8, 16 rows 32.7 -> 22.2; below, [1376, 5824]
+// 17.4 -> 16.6 but [3776, 1600] 12.5 -> 15.9); bf16 from 30 million at 5 to 8 rows ([7632, 4192] 35.6 -> 30.7; below, [2800, 7472]
+// 23.8 -> 25.3) and from 42 million at 9 to 16 ([11008, 4096] 67.4 -> 58.0; below, [18880, 2064] 58.1 -> 62.2). Above the lines the
+// modelled times decide: a rows plan whose strips come out even keeps the call (float32, 8 rows: [4736, 1920] 12.9 against 15.7,
+// [3072, 3072] 15.5 against 16.1, but [4800, 2000] 23.3 against 16.9), and so does the register skinny kernel where the leaves or
+// columns do not divide well (bf16, 9 rows: [44000, 1040] 60.9 against 66.3, [25254, 2064] 67.6 against 72.5).
+inline bool stream_preferred(const Plan &before, const Plan &stream, long long m, long long n, long long k, int wkind, int sms) {
+    const double words = (double)n * (double)k;
+    if (m < 5 || words < (wkind == W_F32 ? 9.0e6 : (m <= 8 ? 30.0e6 : 42.0e6))) return false;
+    const double us = stream_us(m, n, k, wkind, stream.group_leaves, sms);
+    if (before.kind == PLAN_ROWS && m <= 8) {
+        RowsLaunch r;
+        return !rows_layout(m, n, k, wkind, before.group_leaves, sms, r) || us < 0.94 * rows_us(r, m, n, wkind);
+    }
+    if (wkind == W_F32 || before.kind != PLAN_SKINNY) return true;
+    if (m <= 8) return us < 0.94 * before_rows_us(before, m, n, k, wkind, sms);
+    const long long ctas = (n + 255) / 256 * before.groups - sms / 20; // the same for 9 to 16 rows, fitted to 150 sizes (nine in ten within 9 %)
+    const double walk = (double)std::max<long long>((ctas + sms - 1) / sms, 1) * std::min<long long>(before.group_leaves, leaf_count(k));
+    return us < 0.94 * (8.7 + 1.21 * walk + 0.958 * words / 1e6 + 0.51 * (double)(m - 8));
 }
 
 // A^T B of few cells over many rows: every leaf of every 32 x 32 tile as a warp of its own (gemm_tall.cuh).
@@ -511,7 +547,7 @@ size_t plan_need(const Plan &p, long long m, long long n, long long k) { // work
 struct AutoCall {
     long long m, n, k;
     int op, wkind, sms;
-    bool al16, pairs, nodes;
+    bool al16, pairs, nodes, maps; // maps: tensor maps can be made
 };
 template <class Fits>
 Plan choose_auto(const AutoCall &x, Fits fits) {
@@ -534,6 +570,12 @@ Plan choose_auto(const AutoCall &x, Fits fits) {
         if (band_preferred(plan, band, m, n, k, x.sms)) take(band);
     } else if (rows_plan_fits(m, n, k, x.op) && x.al16 && rows_preferred(plan, m, n, k, x.wkind, x.sms)) {
         take(choose_rows(k));
+    }
+    if (skinny && x.maps && (x.wkind == W_F32 || x.wkind == W_BF16) && m <= SM_MAX_ROWS) {
+        const Plan stream = choose_stream(m, n, k, x.wkind, x.sms);
+        if (stream.groups <= MAX_GROUPS && stream_plan_fits(m, n, k, x.op, x.wkind, stream.group_leaves, x.sms) &&
+            stream_preferred(plan, stream, m, n, k, x.wkind, x.sms))
+            take(stream);
     }
     if (tall_fits(m, n, k, x.op, x.wkind) && tall_candidate(m, n, k) && !x.nodes && !x.pairs) take(Plan{PLAN_TALL, 1, (int)leaf_count(k)});
     return plan;
@@ -572,14 +614,13 @@ int64_t launch_product(int dev, cudaStream_t st, float *c, const float *a, const
     if (plan_kind == PLAN_AUTO) {
         const bool pairs = epilogue_pairs(g.epi);
         const bool al16 = aligned(b, 16) && aligned(a, 16);
+        const bool maps = m <= SM_MAX_ROWS && op == OP_NT && t8_encode_fn() != nullptr; // (asked for where it can matter)
         auto fits = [&](const Plan &p) {
             const size_t need = plan_need(p, m, n, k);
             if (need && (!ws || ws_bytes < (int64_t)need || !aligned(ws, p.kind == PLAN_PACKED ? 256 : 4))) return false;
             return !pairs || p.groups <= 1 || (aligned(ws, 16) && aligned(c, 8)); // the fold of a gated store
         };
-        plan = choose_auto(AutoCall{m, n, k, op, wkind, sm_count(dev), al16, pairs, leave_nodes != nullptr}, fits);
-        const Plan stream = choose_stream(n, k);
-        if (al16 && stream_takes(stream, m, n, k, op, wkind, sm_count(dev)) && fits(stream) && t8_encode_fn() != nullptr) plan = stream;
+        plan = choose_auto(AutoCall{m, n, k, op, wkind, sm_count(dev), al16, pairs, leave_nodes != nullptr, maps}, fits);
     } else {
         plan.kind = plan_kind;
         int s = group_leaves > 0 ? (int)group_leaves : g.leaves;
@@ -784,9 +825,10 @@ int64_t b200i_workspace_bytes(int64_t m, int64_t n, int64_t k) {
         }
         if (rows_plan_fits(m, n, k, OP_NT)) groups = std::max(groups, choose_rows(k).groups);
         groups = std::max(groups, choose_band(m, n, k, sm_count(dev)).groups);
-        const Plan stream = choose_stream(n, k);
-        for (const int wkind : {W_F32, W_BF16})
-            if (stream_takes(stream, m, n, k, OP_NT, wkind, sm_count(dev))) groups = std::max(groups, stream.groups);
+        for (const int wkind : {W_F32, W_BF16}) {
+            const Plan q = choose_auto(AutoCall{m, n, k, OP_NT, wkind, sm_count(dev), true, false, false, true}, [](const Plan &) { return true; });
+            if (q.kind == PLAN_STREAM) groups = std::max(groups, q.groups);
+        }
     }
     return groups > 1 ? (int64_t)groups * m * n * 4 : 0;
 }
@@ -795,14 +837,13 @@ int64_t b200i_product_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t o
     if (m <= 0 || n <= 0 || k <= 0) return 0;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); dev = -1; }
-    size_t most = 0; // of what the choice comes to over operand alignments and stores, and of what it falls back to
+    size_t most = 0; // of what the choice comes to over operand alignments, stores and tensor maps, and of what it falls back to
     for (const bool al16 : {true, false})
         for (const bool pairs : {false, true})
             for (const bool all : {true, false})
-                most = std::max(most, plan_need(choose_auto(AutoCall{m, n, k, (int)op, (int)wkind, sm_count(dev), al16, pairs, false},
-                                                            [&](const Plan &p) { return all || p.kind == PLAN_PACKED; }), m, n, k));
-    const Plan stream = choose_stream(n, k);
-    if (stream_takes(stream, m, n, k, (int)op, (int)wkind, sm_count(dev))) most = std::max(most, plan_need(stream, m, n, k));
+                for (const bool maps : {true, false})
+                    most = std::max(most, plan_need(choose_auto(AutoCall{m, n, k, (int)op, (int)wkind, sm_count(dev), al16, pairs, false, maps},
+                                                                [&](const Plan &p) { return all || p.kind == PLAN_PACKED; }), m, n, k));
     return (int64_t)most;
 }
 
@@ -845,7 +886,7 @@ int64_t b200i_plan_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t plan
 
 int64_t b200i_auto_plan(int64_t m, int64_t n, int64_t k, int64_t op, int64_t wkind, int64_t sms, int64_t ws_bytes, int64_t *group_leaves) {
     if (m <= 0 || n <= 0 || k <= 0 || sms <= 0) return -1;
-    const Plan p = choose_auto(AutoCall{m, n, k, (int)op, (int)wkind, (int)sms, true, false, false},
+    const Plan p = choose_auto(AutoCall{m, n, k, (int)op, (int)wkind, (int)sms, true, false, false, true},
                                [&](const Plan &q) { return ws_bytes < 0 || (int64_t)plan_need(q, m, n, k) <= ws_bytes; });
     if (group_leaves) *group_leaves = p.group_leaves;
     return p.kind;

@@ -199,8 +199,9 @@ def test_tall_plan_store_epilogues(m, n, k):
 
 @pytest.mark.parametrize("m", [9, 16, 17, 32])
 def test_band_plan_by_the_rule(m):
-    """Float32 weights of a size that the rule gives to the band plan, ragged columns: the automatic split and its workspace."""
-    n, k = (8201, 2048) if m <= 16 else (4901, 2048)
+    """Float32 weights of a size that the rule gives to the band plan, ragged columns: the automatic split and its workspace (at 9
+    to 16 rows a depth whose leaves the stream plan has no groups for)."""
+    n, k = (301, 33808) if m <= 16 else (4901, 2048)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert _native.lib().b200i_auto_plan(m, n, k, linalg.OP_NT, linalg.W_F32, sms, -1, None) == torch_ops.PLAN_BAND
     rng = np.random.default_rng(m)

@@ -11,7 +11,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 import oracle  # noqa: E402
-from mojolearn_b200 import linalg, torch_ops  # noqa: E402
+from mojolearn_b200 import _native, linalg, torch_ops  # noqa: E402
 
 
 def _bits(t):
@@ -54,9 +54,11 @@ def test_stream_plan_store_epilogues(m, n, k, gl, act):
     assert np.array_equal(_bits(got), _bits(want))
 
 
-@pytest.mark.parametrize("m,n,k,kind", [(5, 4500, 2000, linalg.W_F32), (16, 8467, 2048, linalg.W_F32), (9, 60001, 784, linalg.W_F32), (8, 11008, 4096, linalg.W_BF16),
+@pytest.mark.parametrize("m,n,k,kind", [(5, 4801, 2000, linalg.W_F32), (16, 8467, 2048, linalg.W_F32), (9, 60001, 784, linalg.W_F32), (8, 11008, 4096, linalg.W_BF16),
                                         (12, 11008, 4096, linalg.W_BF16)])
 def test_automatic_choice_at_the_sizes_that_stream(m, n, k, kind):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert _native.lib().b200i_auto_plan(m, n, k, linalg.OP_NT, kind, sms, -1, None) == torch_ops.PLAN_STREAM
     rng = np.random.default_rng(n)
     a, w = rng.standard_normal((m, k)).astype(np.float32), (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
     got = _run(a, w, kind)

@@ -6,7 +6,7 @@ import pytest
 
 from mojolearn_b200 import _native
 from mojolearn_b200.linalg import OP_NN, OP_NT, OP_TN, W_BF16, W_F32, W_INT8_EXP, W_INT8_SCALE, leaf_count
-from mojolearn_b200.torch_ops import PLAN_BAND, PLAN_ROWS, PLAN_SKINNY
+from mojolearn_b200.torch_ops import PLAN_BAND, PLAN_DECODE, PLAN_ROWS, PLAN_SKINNY, PLAN_STREAM
 
 SMEM_LIMIT = 225 * 1024  # of a CTA of the rows plan; the device's own limit is 227 KB
 KINDS = [W_F32, W_BF16, W_INT8_EXP, W_INT8_SCALE]
@@ -53,7 +53,7 @@ def test_the_rows_plan_always_has_two_stages(kind, sms):
     assert taken > 50
 
 
-@pytest.mark.parametrize("m,n,k,plan", [(8, 220000, 4096, PLAN_ROWS), (4, 400000, 4096, PLAN_ROWS), (14, 178374, 12208, PLAN_BAND), (31, 165405, 1536, PLAN_BAND)])
+@pytest.mark.parametrize("m,n,k,plan", [(4, 220000, 4096, PLAN_ROWS), (4, 400000, 4096, PLAN_ROWS), (31, 178374, 12208, PLAN_BAND), (31, 165405, 1536, PLAN_BAND)])
 def test_a_workspace_that_holds_the_skinny_plan_only_gets_the_skinny_plan(m, n, k, plan):
     """These sizes are unsplit in the skinny plan, which needs no workspace, and split in the plan that the rule prefers."""
     got, leaves = auto_plan(m, n, k)
@@ -63,6 +63,16 @@ def test_a_workspace_that_holds_the_skinny_plan_only_gets_the_skinny_plan(m, n, 
     for ws in (0, need - 1):
         got, leaves = auto_plan(m, n, k, ws=ws)
         assert got != plan and leaves >= leaf_count(k)
+
+
+@pytest.mark.parametrize("m,n,k,before", [(8, 220000, 4096, PLAN_ROWS), (14, 178374, 12208, PLAN_BAND)])
+def test_a_workspace_that_does_not_hold_the_stream_plan_gets_the_plan_before_it(m, n, k, before):
+    got, leaves = auto_plan(m, n, k)
+    need = -(-leaf_count(k) // leaves) * m * n * 4
+    assert got == PLAN_STREAM and auto_plan(m, n, k, ws=need) == (got, leaves)
+    got, leaves = auto_plan(m, n, k, ws=need - 1)
+    assert got == before and -(-leaf_count(k) // leaves) * m * n * 4 < need
+    assert auto_plan(m, n, k, ws=0) == (PLAN_SKINNY, leaf_count(k))
 
 
 def test_workspace_by_op_and_storage():
@@ -83,10 +93,16 @@ def test_workspace_by_op_and_storage():
 
 
 @pytest.mark.parametrize("m,n,k,kind,plan", [
-    (8, 2304, 768, W_F32, PLAN_ROWS), (8, 11008, 4096, W_F32, PLAN_ROWS), (4, 11008, 4096, W_F32, PLAN_ROWS), (8, 2304, 768, W_INT8_EXP, PLAN_ROWS),
-    (8, 11008, 4096, W_INT8_EXP, PLAN_ROWS), (12, 2304, 768, W_F32, PLAN_ROWS), (8, 1536, 6160, W_F32, PLAN_SKINNY), (8, 32000, 1792, W_F32, PLAN_SKINNY),
-    (8, 1536, 6160, W_BF16, PLAN_SKINNY), (8, 1536, 6160, W_INT8_EXP, PLAN_SKINNY), (16, 1536, 6160, W_F32, PLAN_SKINNY), (16, 5120, 4096, W_F32, PLAN_SKINNY),
-    (16, 8192, 1792, W_F32, PLAN_BAND), (16, 16384, 2048, W_F32, PLAN_BAND), (32, 16384, 2048, W_F32, PLAN_BAND)])
+    (8, 2304, 768, W_F32, PLAN_ROWS), (8, 11008, 4096, W_F32, PLAN_STREAM), (4, 11008, 4096, W_F32, PLAN_ROWS), (8, 2304, 768, W_INT8_EXP, PLAN_ROWS),
+    (8, 11008, 4096, W_INT8_EXP, PLAN_ROWS), (12, 2304, 768, W_F32, PLAN_ROWS), (8, 1536, 6160, W_F32, PLAN_STREAM), (8, 32000, 1792, W_F32, PLAN_STREAM),
+    (8, 1536, 6160, W_BF16, PLAN_SKINNY), (8, 1536, 6160, W_INT8_EXP, PLAN_SKINNY), (16, 1536, 6160, W_F32, PLAN_STREAM), (16, 5120, 4096, W_F32, PLAN_STREAM),
+    (16, 8192, 1792, W_F32, PLAN_STREAM), (16, 16384, 2048, W_F32, PLAN_STREAM), (32, 16384, 2048, W_F32, PLAN_BAND),
+    (4, 11008, 4096, W_BF16, PLAN_DECODE), (5, 11008, 4096, W_BF16, PLAN_STREAM), (16, 11008, 4096, W_BF16, PLAN_STREAM), (17, 11008, 4096, W_BF16, PLAN_SKINNY),
+    (17, 11008, 4096, W_F32, PLAN_BAND), (5, 4800, 1872, W_F32, PLAN_ROWS), (5, 4800, 1888, W_F32, PLAN_STREAM), (16, 4800, 1888, W_F32, PLAN_STREAM),
+    (16, 4800, 1872, W_F32, PLAN_SKINNY), (8, 7300, 4096, W_BF16, PLAN_SKINNY), (8, 7340, 4096, W_BF16, PLAN_STREAM), (9, 10240, 4096, W_BF16, PLAN_SKINNY),
+    (9, 10288, 4096, W_BF16, PLAN_STREAM), (8, 4736, 1920, W_F32, PLAN_ROWS), (8, 9216, 1024, W_F32, PLAN_ROWS), (9, 44000, 1040, W_BF16, PLAN_SKINNY),
+    (8, 220000, 4112 * 16, W_F32, PLAN_ROWS)])
 def test_small_batches_take_the_plan_that_measured_faster(m, n, k, kind, plan):
-    """Both sides of the rules' lines: depths whose last group or strip is nearly empty keep the skinny plan."""
+    """Both sides of the rules' lines: depths whose last group or strip is nearly empty keep the skinny plan; from nine million
+    words (bf16 30 and 42) the stream plan, but where a rows plan comes out even or the columns and leaves divide badly."""
     assert auto_plan(m, n, k, wkind=kind)[0] == plan
