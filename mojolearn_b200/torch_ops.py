@@ -89,7 +89,10 @@ ACT_PAIR_SWIGLU, ACT_PAIR_GEGLU_ERF, ACT_PAIR_GEGLU_TANH = 4, 5, 6  # over inter
 
 def _bind_plain_product(*args):
     global _plain_product
-    lib = _native.lib()
+    try:
+        lib = _native.lib()
+    except _native.NativeError:
+        return None  # the Python path's checks of the operands come first, then its own refusal
     _host_call.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.b200i_gemm_w_plan, lib.b200i_product_workspace_bytes, lib.b200i_plan_workspace_bytes)),
                     _native.NativeError)
     _plain_product = _host_call.product
