@@ -47,20 +47,41 @@ def build(force=False, verbose=False, sabotage=False):
 HOST_LIB = os.path.join(os.path.dirname(HERE), "_host_call.so")
 
 
+def host_tag():
+    """What a built host extension belongs to: torch's C++ classes and Python's objects have no stable layout."""
+    import torch
+    return "torch %s, python %d.%d" % ((torch.__version__,) + sys.version_info[:2])
+
+
+def host_stale(lib=None):
+    lib = lib or HOST_LIB
+    if not os.path.exists(lib) or any(os.path.getmtime(d) > os.path.getmtime(lib) for d in (os.path.join(HERE, "host_call.cpp"), os.path.abspath(__file__))):
+        return True
+    with open(lib, "rb") as f:
+        return host_tag().encode() + b"\0" not in f.read()  # BUILT_FOR, as host_call.cpp keeps it
+
+
 def build_host(force=False):
-    source = os.path.join(HERE, "host_call.cpp")
-    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= os.path.getmtime(source):
+    if not force and not host_stale():
         return HOST_LIB
     import sysconfig
     import torch
     root = os.path.dirname(torch.__file__)
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
-           "-I" + os.path.join(root, "include"), "-I/usr/local/cuda/include", "-I" + sysconfig.get_paths()["include"], source, "-L" + os.path.join(root, "lib"),
-           "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_python", "-o", HOST_LIB]
+           '-DBUILT_FOR="%s"' % host_tag(), "-I" + os.path.join(root, "include"), "-I/usr/local/cuda/include", "-I" + sysconfig.get_paths()["include"],
+           os.path.join(HERE, "host_call.cpp"), "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_python", "-o", HOST_LIB]
     subprocess.run(cmd, check=True)
     return HOST_LIB
 
 
+def main(argv):
+    """The CUDA library needs nvcc alone; the host extension is built where torch and a host compiler are there too."""
+    print(build(force="--force" in argv, verbose="--verbose" in argv, sabotage="--sabotage" in argv))
+    try:
+        print(build_host("--force" in argv))
+    except (ImportError, OSError, subprocess.CalledProcessError) as x:
+        print("no native host side for torch products (%s); they go through ctypes" % x, file=sys.stderr)
+
+
 if __name__ == "__main__":
-    build_host("--force" in sys.argv)
-    print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv, sabotage="--sabotage" in sys.argv))
+    main(sys.argv[1:])

@@ -126,4 +126,10 @@ PyModuleDef MODULE = {PyModuleDef_HEAD_INIT, "_host_call", "native host side of 
 
 } // namespace
 
-PyMODINIT_FUNC PyInit__host_call() { return PyModule_Create(&MODULE); }
+// BUILT_FOR, of the compiler's command line: the versions of torch and Python whose headers this was compiled with. The package
+// does not use a module of others.
+PyMODINIT_FUNC PyInit__host_call() {
+    PyObject *m = PyModule_Create(&MODULE);
+    if (m && PyModule_AddStringConstant(m, "BUILT_FOR", BUILT_FOR) < 0) Py_CLEAR(m);
+    return m;
+}

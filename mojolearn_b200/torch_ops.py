@@ -15,16 +15,32 @@ the product can sit inside a torch program (fake-tensor shapes included).
 import contextlib
 import ctypes
 import functools
+import os
+import warnings
 
 import torch
 
 from . import _native
-
-try:
-    from . import _host_call  # csrc/host_call.cpp; without it the same calls go through ctypes
-except ImportError:
-    _host_call = None
+from .csrc import build as _build
 from .linalg import OP_NN, OP_NT, OP_TN, W_BF16, W_F32, W_INT8_EXP, W_INT8_SCALE, leaf_count
+
+
+def _load_host_call():
+    """csrc/host_call.cpp, or None: the same calls then go through ctypes. A module that is there and cannot be used is not passed
+    over in silence: the calls are slower without it."""
+    try:
+        from . import _host_call as module
+        problem = None if module.BUILT_FOR == _build.host_tag() else "it was built for %s" % module.BUILT_FOR
+    except (ImportError, AttributeError) as x:
+        problem = str(x) if os.path.exists(_build.HOST_LIB) else ""
+    if problem is None:
+        return module
+    if problem:
+        warnings.warn("mojolearn_b200: %s is not used (%s); build it again with `python -m mojolearn_b200.csrc.build`" % (_build.HOST_LIB, problem), RuntimeWarning, stacklevel=3)
+    return None
+
+
+_host_call = _load_host_call()
 
 PLAN_AUTO, PLAN_FLAT, PLAN_T128, PLAN_T64, PLAN_DECODE, PLAN_T32, PLAN_T128X64, PLAN_SKINNY, PLAN_PACKED, PLAN_TALL, PLAN_ROWS, PLAN_BAND, PLAN_STREAM = -1, 0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11
 
