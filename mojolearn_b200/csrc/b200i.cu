@@ -302,6 +302,8 @@ double before_rows_us(const Plan &before, long long m, long long n, long long k,
 // columns, at 5 to 8 rows also where they are deep; bf16 ones to 3072 columns; low-bit ones at 9 to 16 rows while small enough to
 // be bound by latency. Inside these lines the modelled times decide: float32 [2304, 768] at eight rows 6.5 against 14 us,
 // [11008, 4096] 57 against 80, but [32000, 1792] 138 against 96 and [1536, 6160] 28 against 21 (a strip of 64 columns for ten).
+// (At 5 to 8 float32 rows from nine million words the answer stands where strips come out even, stream_preferred, where the depth
+// is past 32768 steps, and where a call's workspace is too small for the stream plan.)
 inline bool rows_preferred(const Plan &before, long long m, long long n, long long k, int wkind, int sms) {
     RowsLaunch r;
     if (m < 4 || !rows_layout(m, n, k, wkind, choose_rows(k).group_leaves, sms, r)) return false;
@@ -347,7 +349,8 @@ Plan choose_band(long long m, long long n, long long k, int sms) {
     return p;
 }
 // Float32 weights from ten million words up (the sizes on both sides of the line stand in gemm_band.cuh); up to sixteen rows also
-// by the modelled times ([8192, 1792] 35 against 41 us, but [5120, 4096] 55 against 51).
+// by the modelled times ([8192, 1792] 35 against 41 us, but [5120, 4096] 55 against 51), which matters past 32768 steps and where a
+// call's workspace is too small for the stream plan: that takes the others.
 inline bool band_size(long long n, long long k, int wkind) { return wkind == W_F32 && (double)n * (double)k >= 1.0e7; }
 inline bool band_preferred(const Plan &skinny, const Plan &band, long long m, long long n, long long k, int sms) {
     return m > 16 || band_us(m, n, k, band.group_leaves, sms) < 0.97 * before_rows_us(skinny, m, n, k, W_F32, sms);

@@ -13,7 +13,7 @@
 //   barrier one per window; it publishes the window and its admission verdict.
 // Leaves of a CTA's group are folded by a per-thread counter stack, groups by fold_groups as in the other plans.
 // Measured (graph replay, fold included) against the skinny kernel: [16384, 2048] 88 against 108 us at 32 rows, 62 against
-// 82 at 16; [50304, 2048] 242 against 297; [11008, 4096] 120 against 130; [2304, 768] 23 against 18, hence the rule's size.
+// 82 at 16 (45 in the streaming kernel, which takes such calls up to sixteen rows); [50304, 2048] 242 against 297; [11008, 4096] 120 against 130; [2304, 768] 23 against 18, hence the rule's size.
 // The same kernel with low-bit weights widened on the way lost to the register kernel (int8 [11008, 4096] 111 against 95).
 #pragma once
 #include "gemm_skinny.cuh"

@@ -17,8 +17,9 @@
 //     subtrees), so no node crosses L2 and there is no second launch up to sixteen leaves; beyond that the leaves are cut
 //     into groups (the activations of more would leave too short a ring) and fold_groups finishes as for the other plans.
 // Measured at eight rows, float32 (graph replay): [768, 768] 13.1 -> 5.6 us, [2304, 768] 14.1 -> 6.5, [768, 3072] 13.9 -> 8.6,
-// [50304, 768] 66 -> 54. Bound: latency below ten million weights (a leaf is 128 dependent steps), above by the warps' own
-// instructions (about six per step and column of 32 lanes) and by HBM.
+// [50304, 768] 66 -> 54 (41 in the streaming kernel, which takes most large weights at 5 rows and more). Bound: latency below ten
+// million weights (a leaf is 128 dependent steps), above by the warps' own instructions (about six per step and column of 32 lanes)
+// and by HBM.
 //
 // Admission is per leaf: the activations' keys are taken while they are staged, the weights' while they are used; a lane
 // whose leaf fails runs the defining flushed chain again from global memory.

@@ -13,14 +13,15 @@
 //     No other warp is waited for, and an SM has up to 192 KB in flight. Edges of the weight and the k tail are zero-filled;
 //   - a lane owns eight rows (MT rows over RG row groups) by CPL columns, the rows in pairs: one 16-byte read of the activations
 //     serves 2 * CPL packed fmas, one 16-byte read of a column serves 4 or 8 k-steps. Bodies of 4, 8 and 16 k-steps, eight and
-//     twelve warps and twice the cells per lane measured the same or slower.
+//     twelve warps and twice the cells per lane measured the same or slower, with the items dealt out as below.
 //
 // Measured (graph replay, several weights in turn, fold included), the plan before -> this: float32 at eight rows [11008, 4096]
 // 56 -> 43 us, [10512, 2256] 47 -> 27, at five [50304, 768] 54 -> 41, at sixteen [39296, 6416] 393 -> 248; bf16 [11008, 4096] at
 // eight 42.6 -> 35.4, at sixteen 67.4 -> 58.6. Bound: float32 at eight rows HBM (64 % of the measured copy rate at [11008, 4096]);
-// otherwise the warps' own instructions and the items' uneven number per warp. Int8 weights measured no faster than the rows and
-// register skinny kernels (36 against 34 us at eight rows, 87 against 86 at 32), nor did float32 ones at 32 rows (79 to 114
-// against 85 to 108), so those keep theirs.
+// otherwise too few warps with work: a CTA's items rarely divide by sixteen ([11008, 4096] in groups of four: 9.3 of them, so 9.2
+// warps are active, issue slots 45 % and fma pipe 36 % busy at eight bf16 rows). Under that split int8 weights measured no faster
+// than the rows and register skinny kernels (36 against 34 us at eight rows, 87 against 86 at 32), nor did float32 ones at 32 rows
+// (79 to 114 against 85 to 108), so those keep theirs; an even split was not tried.
 //
 // Admission is per leaf and lane: the activations' keys are taken while they are staged, the weights' while they are widened
 // (bf16: two words an instruction, a zero passing as 0xFFFF after the subtraction); a lane whose leaf fails runs the defining

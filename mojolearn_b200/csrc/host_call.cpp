@@ -1,12 +1,13 @@
 // The host side of a product call on device tensors, in native code: torch_ops.product without bias, activation or `out`.
 //
-// A one-token product is a 14 us kernel ([11008, 4096] int8), and the same checks, allocations and argument conversions
-// spelled in Python and ctypes took about 18 us a call, so a loop of such calls ran at the host's pace. This module makes
-// the checks on the tensors themselves, takes output and workspace from torch's allocator and calls the C ABI directly.
+// The checks, allocations and argument conversions of a one-row product take 15.5 us of host time a call in Python and ctypes and
+// 6.5 here, on the tensors themselves, with output and workspace from torch's allocator and the C ABI called directly. A loop of
+// int8 [768, 768] rows went from 15.3 to 6.4 us a call. One of [11008, 4096] rows takes 16.4 either way, also when it is queued
+// behind other work: a 14.5 us kernel (graph replay) and what the device leaves between two plain launches.
 //
 // It takes the plain case only: exact torch tensors (no subclass, no functorch or python-dispatch wrapper) of the storage
-// types, contiguous, on the current device, extents that agree, no torch mode active. For anything else it returns None and the caller's Python
-// path decides, so refusals keep their exceptions and messages.
+// types, contiguous, on the current device, extents that agree, no torch mode active. For anything else it returns None and the
+// caller's Python path decides, so refusals keep their exceptions and messages.
 #include <Python.h>
 
 #include <ATen/ATen.h>

@@ -115,7 +115,7 @@ def _bind_plain_product(*args):
     return _plain_product(*args)
 
 
-#: a product of plain device tensors in native code, or None where a call is anything else ([11008, 4096] int8 row: see host_call.cpp)
+#: a product of plain device tensors in native code, or None where a call is anything else (figures in csrc/host_call.cpp)
 _plain_product = _bind_plain_product if _host_call is not None else None
 
 
